@@ -22,7 +22,7 @@ LIB = os.path.join(HERE, "libpyspectral_b200.so")
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 FLAGS = ARCH + ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr",
-                "-Xcompiler", "-Wno-deprecated-declarations"]
+                "-Xcompiler", "-Wno-deprecated-declarations", "-split-compile=4"]
 
 
 def nvcc() -> str:

@@ -128,6 +128,26 @@ struct Batch {
     epi = reinterpret_cast<Epi*>(take(sizeof(Epi) * R * 5));
   }
 
+  // Fields of pass p's register form (x-inverse: Pre, y-inverse: YPre, y-forward: a copy).
+  template <class P>
+  static constexpr bool has_fields() {
+    return pre_has_fields<P>::value;
+  }
+  static constexpr bool reg_pass(int pass) {
+    return pass == 0 ? has_fields<Pre>() : (pass == 1 ? has_fields<YPre>() : pass == 3);
+  }
+  // Column tile and plan in the argument blocks of axis pass `pass`: the pass's own shape, or,
+  // where the pass runs as a register pass (which takes neither), the default of the
+  // runtime-schedule bodies that the persistent ensemble runs on the same blocks.
+  void generic_shape(int pass, int& tile, FFTPlan& plan) const {
+    tile = b->tile[pass];
+    plan = b->plan[pass];
+    if (!reg_pass(pass) || !is_reg_axis(plan)) return;
+    const int F = pass == 0 ? Fi : (pass == 1 ? YPre::F_DST : 1);
+    const int no = pass == 0 ? d.N2 : (pass == 1 ? YP::groups * d.M1 : Fo * d.M1);
+    default_axis_shape<T>(c, plan.L, d.Kz, F, no, false, tile, plan);
+  }
+
   // Argument blocks of every run (host copy, then one upload).
   int build(const Pre& pre0, Phys (*mkphys)(psb_ctx*, const psb_params&),
             Epi (*mkepi)(psb_ctx*, StepIO<T>, const psb_params&)) {
@@ -141,7 +161,7 @@ struct Batch {
       const Cx<T>* Q = reinterpret_cast<const Cx<T>*>(b->state[r]);
       Cx<T>*A = run_buf(r, 0), *B = run_buf(r, 1), *C = run_buf(r, 2), *D = run_buf(r, 3);
       AxisArgs<T> a{};
-      a.plan = b->plan[0];
+      generic_shape(0, a.col_tile, a.plan);
       a.tw = twiddles<T>(c);
       a.scale = (T)1;
       a.in = Q;
@@ -154,7 +174,6 @@ struct Batch {
       a.out_rstride = (long long)d.N2 * d.Kz;
       a.nouter = d.N2;
       a.ncols = d.Kz;
-      a.col_tile = b->tile[0];
       a.in_rows = d.N1;
       a.out_rows = d.M1;
       a.in_map = map_pad32(d.N1);
@@ -164,7 +183,7 @@ struct Batch {
       a.k_col = c->kz;
       ax[r] = a;
       AxisArgs<T> y{};
-      y.plan = b->plan[1];
+      generic_shape(1, y.col_tile, y.plan);
       y.tw = twiddles<T>(c);
       y.scale = (T)1;
       y.in = A;
@@ -178,7 +197,6 @@ struct Batch {
       y.out_fstride = (long long)YP::out_fields * d.M1 * d.M2 * d.Kz;
       y.k_row = c->ky;
       y.ncols = d.Kz;
-      y.col_tile = b->tile[1];
       y.in_rows = d.N2;
       y.out_rows = d.M2;
       y.in_map = map_pad32(d.N2);
@@ -199,7 +217,7 @@ struct Batch {
       z.tw = twiddles<T>(c);
       az[r] = z;
       AxisArgs<T> yf{};
-      yf.plan = b->plan[3];
+      generic_shape(3, yf.col_tile, yf.plan);
       yf.tw = twiddles<T>(c);
       yf.scale = (T)1;
       yf.in = C;
@@ -210,7 +228,6 @@ struct Batch {
       yf.out_rstride = d.Kz;
       yf.nouter = Fo * d.M1;
       yf.ncols = d.Kz;
-      yf.col_tile = b->tile[3];
       yf.in_rows = d.M2;
       yf.out_rows = d.N2;
       yf.in_map = map_id(d.M2);
@@ -314,18 +331,20 @@ struct Batch {
     const size_t esz = sizeof(Cx<T>);
     switch (pass) {
       case 0: {
+        const double by = (double)R * esz * d.N2 * d.Kz * (3.0 * d.N1 + (double)Fi * d.M1);
+        if constexpr (has_fields<Pre>())
+          if (is_reg_axis(b->plan[0]))
+            return reg_axis_batch<T>(c, ax, Pre{}.fields(), d.M1, d.Kz, d.N2, R, true, "batch x-inverse", by);
         const int ct = b->tile[0];
         dim3 g((d.Kz + ct - 1) / ct, d.N2, R);
         const size_t sm = smem_axis(d.M1, Fi, ct);
         auto go = [&](auto k) {
           set_smem(k, sm);
-          LaunchScope s(c, "batch x-inverse", (double)R * esz * d.N2 * d.Kz * (3.0 * d.N1 + (double)Fi * d.M1));
+          LaunchScope s(c, "batch x-inverse", by);
           launch_pdl(k, g, 256, sm, c->stream, (const AxisArgs<T>*)ax, (const Pre*)pre);
           return launch_ok(c, "batch x-inverse");
         };
-        return by_plan(
-            0, [&](auto id) { return go(axis_pass_batch<T, true, Pre, false, decltype(id)::value>); },
-            [&] { return go(axis_pass_batch<T, true, Pre, W>); });
+        return go(axis_pass_batch<T, true, Pre, W>);
       }
       case 1:
       case 3: {
@@ -333,9 +352,16 @@ struct Batch {
         const int ct = b->tile[pass];
         // y-inverse: YP::groups outer groups of YPre::F_DST lines per column
         const int G = inv ? YP::groups : Fo, F = inv ? Fb : Fo;
+        const double by = (double)R * esz * F * d.M1 * d.Kz * (double)(d.N2 + d.M2);
+        if (is_reg_axis(b->plan[pass])) {
+          if (!inv)
+            return reg_axis_batch<T>(c, ayf, PreCopy<T>{}.fields(), d.M2, d.Kz, G * d.M1, R, false, "batch y-forward",
+                                     by);
+          if constexpr (has_fields<YPre>())
+            return reg_axis_batch<T>(c, ay, YPre{}.fields(), d.M2, d.Kz, G * d.M1, R, true, "batch y-inverse", by);
+        }
         dim3 g((d.Kz + ct - 1) / ct, G * d.M1, R);
         const size_t sm = smem_axis(d.M2, inv ? YPre::F_DST : 1, ct);
-        const double by = (double)R * esz * F * d.M1 * d.Kz * (double)(d.N2 + d.M2);
         if (inv) {
           auto go = [&](auto k) {
             set_smem(k, sm);
@@ -343,9 +369,7 @@ struct Batch {
             launch_pdl(k, g, 256, sm, c->stream, (const AxisArgs<T>*)ay, (const YPre*)ypre);
             return launch_ok(c, "batch y-inverse");
           };
-          return by_plan(
-              1, [&](auto id) { return go(axis_pass_batch<T, true, YPre, false, decltype(id)::value>); },
-              [&] { return go(axis_pass_batch<T, true, YPre, W>); });
+          return go(axis_pass_batch<T, true, YPre, W>);
         }
         auto go = [&](auto k) {
           set_smem(k, sm);
@@ -353,9 +377,7 @@ struct Batch {
           launch_pdl(k, g, 256, sm, c->stream, (const AxisArgs<T>*)ayf, (const PreCopy<T>*)cpy);
           return launch_ok(c, "batch y-forward");
         };
-        return by_plan(
-            3, [&](auto id) { return go(axis_pass_batch<T, false, PreCopy<T>, false, decltype(id)::value>); },
-            [&] { return go(axis_pass_batch<T, false, PreCopy<T>, W>); });
+        return go(axis_pass_batch<T, false, PreCopy<T>, W>);
       }
       case 2: {
         const int P = b->tile[2];
@@ -452,6 +474,8 @@ struct Batch {
     // full RHS first so that every intermediate buffer holds real data.
     for (int pass = 0; pass < 5; ++pass) PSB_TRY(launch(pass, 4));
     for (int pass = 0; pass < 5; ++pass) {
+      // a register pass has one shape (the runtime-schedule shapes of its length are slower throughout)
+      if (pass != 2 && reg_pass(pass) && is_reg_axis(b->plan[pass])) continue;
       std::vector<int> tiles;
       if (pass == 2) {
         for (int P : {1, 2, 4, 8})
@@ -530,14 +554,17 @@ EpiNS<T, SMAG> mk_epi(psb_ctx* c, StepIO<T> io, const psb_params& p) {
 
 // Default launch shapes: the single-run rules of the library.
 // Fz: z-pass inputs (with the fields it derives itself); Fy / Gy: lines per
-// column and outer groups of the y-inverse pass
-void default_shapes(psb_batch* b, int Fi, int Fb, int Fz, int Fo, int Fy, int Gy, size_t esz, int ppc,
+// column and outer groups of the y-inverse pass; reg: which passes have a
+// register form
+template <typename T>
+void default_shapes(psb_batch* b, int Fi, int Fb, int Fz, int Fo, int Fy, int Gy, bool (*reg)(int), int ppc,
                     size_t zextra) {
   psb_ctx* c = b->c;
+  const size_t esz = sizeof(Cx<T>);
   const Dims d = dims(c, Fi, Fb, Fo);
-  b->tile[0] = pick_ct(d.Kz, Fi, d.M1, esz, d.N2);
-  b->tile[1] = pick_ct(d.Kz, Fy, d.M2, esz, Gy * d.M1);
-  b->tile[3] = pick_ct(d.Kz, 1, d.M2, esz, Fo * d.M1);
+  default_axis_shape<T>(c, d.M1, d.Kz, Fi, d.N2, reg(0), b->tile[0], b->plan[0]);
+  default_axis_shape<T>(c, d.M2, d.Kz, Fy, Gy * d.M1, reg(1), b->tile[1], b->plan[1]);
+  default_axis_shape<T>(c, d.M2, d.Kz, 1, Fo * d.M1, reg(3), b->tile[3], b->plan[3]);
   b->tile[4] = pick_ct(d.Kz, Fo, d.M1, esz, d.N2);
   const int FMAX = std::max(Fz, Fo);
   int P = ppc;
@@ -547,10 +574,7 @@ void default_shapes(psb_batch* b, int Fi, int Fb, int Fz, int Fo, int Fy, int Gy
   const long long np = (long long)d.M1 * d.M2;
   while (P > 1 && (np + P - 1) / P * b->nruns < 2 * 148) P /= 2;
   b->tile[2] = P;
-  b->plan[0] = *plan_for(c, d.M1);
-  b->plan[1] = *plan_for(c, d.M2);
   b->plan[2] = *plan_for(c, d.M3);
-  b->plan[3] = *plan_for(c, d.M2);
   b->plan[4] = *plan_for(c, d.M1);
 }
 
@@ -573,7 +597,7 @@ int run_batch(psb_batch* b, int nsteps, bool tune, Pre pre0, Phys (*mkphys)(psb_
     b->arena_bytes = need;
   }
   if (b->plan[0].L == 0) {
-    default_shapes(b, BT::Fi, BT::Fb, Phys::F_IN, BT::Fo, BT::YPre::F_DST, BT::YP::groups, sizeof(Cx<T>),
+    default_shapes<T>(b, BT::Fi, BT::Fb, Phys::F_IN, BT::Fo, BT::YPre::F_DST, BT::YP::groups, &BT::reg_pass,
                    phys_default_ppc<Phys>::value, (size_t)phys_is_block<Phys>::extra);
     // the register-direct z pass's schedule where it exists (as for single runs)
     if constexpr (phys_fixed_fft<Phys>::value && sizeof(T) == 4)
@@ -730,7 +754,12 @@ size_t ens_group(psb_batch* b, int kind, EnsGroup& g) {
   g.cpy = x.cpy;
   g.phys = x.phys;
   g.epi = x.epi;
-  const int* t = b->tile.data();
+  // the tiles in the argument blocks (the runtime-schedule bodies run here)
+  std::array<int, 5> t = b->tile;
+  for (int k : {0, 1, 3}) {
+    FFTPlan plan;
+    x.generic_shape(k, t[k], plan);
+  }
   g.nx[0] = (d.Kz + t[0] - 1) / t[0];
   g.ny[0] = d.N2;
   g.nx[1] = (d.Kz + t[1] - 1) / t[1];

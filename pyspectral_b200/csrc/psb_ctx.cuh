@@ -14,6 +14,7 @@
 
 #include "../../include/pyspectral_b200.h"
 #include "psb_physics.cuh"
+#include "psb_reg.cuh"
 
 // Launch shape of one pass picked by the autotuner: tile (columns per CTA, or
 // pencils per CTA for the z pass), its transform's radix order, and whether
@@ -305,6 +306,51 @@ inline bool plan_is_wide_h(const psb::FFTPlan& p) {
   return false;
 }
 
+// ---- register passes (psb_reg.cuh; launched by psb_axis_f32.cu / psb_axis_f64.cu) ----
+// The register axis pass's radices of a length; false when it has none.
+inline bool reg_axis_plan(int L, FFTPlan& p) {
+  switch (L) {
+#define PSB_CASE(LEN, A, B) \
+  case LEN:                 \
+    p.radix[0] = A;         \
+    p.radix[1] = B;         \
+    break;
+    PSB_REG_AXIS(PSB_CASE)
+#undef PSB_CASE
+    default:
+      return false;
+  }
+  p.npass = 2;
+  for (int s = 2; s < psb::kMaxPasses; ++s) p.radix[s] = 0;
+  return true;
+}
+inline bool has_reg_axis(int L) {
+  FFTPlan p{};
+  return reg_axis_plan(L, p);
+}
+inline bool is_reg_axis(const FFTPlan& p) {
+  FFTPlan q{};
+  return reg_axis_plan(p.L, q) && p.npass == 2 && p.radix[0] == q.radix[0] && p.radix[1] == q.radix[1];
+}
+// a: one launch's arguments (plan.L and plan.tw_off name the length and its
+// twiddles); the batched form reads run r's arguments from args[r] on the device
+template <typename T>
+int reg_axis(psb_ctx* c, const psb::AxisArgs<T>& a, const psb::FieldTab<T>& ft, bool inv, const char* what,
+             double bytes);
+template <typename T>
+int reg_axis_batch(psb_ctx* c, const psb::AxisArgs<T>* args, const psb::FieldTab<T>& ft, int L, int ncols, int nouter,
+                   int runs, bool inv, const char* what, double bytes);
+
+// Launch shape (tile and radices) of an axis pass that no tuner has touched.
+template <typename T>
+inline void default_axis_shape(psb_ctx* c, int L, int ncols, int F, int nouter, bool reg, int& tile, FFTPlan& plan) {
+  plan = *plan_for(c, L);
+  if (reg && reg_axis_plan(L, plan))
+    tile = psb::reg_cols<T>();
+  else
+    tile = pick_ct(ncols, F, L, sizeof(Cx<T>), nouter);
+}
+
 // sh: an autotuned shape (TUNABLE launch sites only) or null for the default
 template <typename T, bool INV, class Pre, bool TUNABLE = false>
 int launch_axis(psb_ctx* c, psb::AxisArgs<T> a, Pre pre, const char* what, const psb_pass_shape* sh = nullptr) {
@@ -315,39 +361,21 @@ int launch_axis(psb_ctx* c, psb::AxisArgs<T> a, Pre pre, const char* what, const
     a.col_tile = sh->tile;
     a.plan = sh->plan;
   }
-  const size_t smem = (size_t)(L + 2 * L * Pre::F_DST * a.col_tile) * esz;
-  dim3 grid((a.ncols + a.col_tile - 1) / a.col_tile, a.nouter);
   const double bytes = (double)esz * a.nouter * a.ncols *
                        ((double)Pre::F_SRC * count_mapped(a.in_map, a.in_rows) + (double)Pre::F_DST * a.out_rows);
+  // the register pass of this length (psb_reg.cuh), where there is one; a tuned shape's tile and
+  // radices apply to the runtime-schedule kernels of the other lengths
+  if constexpr (psb::pre_has_fields<Pre>::value) {
+    if (has_reg_axis(L)) return reg_axis<T>(c, a, pre.fields(), INV, what, bytes);
+  }
+  const size_t smem = (size_t)(L + 2 * L * Pre::F_DST * a.col_tile) * esz;
+  dim3 grid((a.ncols + a.col_tile - 1) / a.col_tile, a.nouter);
   auto go = [&](auto k) {
     set_smem(k, smem);
     LaunchScope scope(c, what, bytes);
     launch_pdl(k, grid, 256, smem, c->stream, a, pre);
     return launch_ok(c, what);
   };
-  // A compiled two-pass schedule on a tunable pass whose Pre forms each field
-  // on load: registers straight from and to global memory around a single
-  // shared-memory exchange (psb::axis_rr_body).
-  if constexpr (TUNABLE && psb::pre_fieldwise<Pre>::value) {
-    const size_t rsmem = (size_t)(L + (size_t)L * Pre::F_DST * a.col_tile) * esz;
-    auto gor = [&](auto k) {
-      set_smem(k, rsmem);
-      LaunchScope scope(c, what, bytes);
-      launch_pdl(k, grid, 256, rsmem, c->stream, a, pre);
-      return launch_ok(c, what);
-    };
-    switch (psb::fixed_plan_id(a.plan)) {
-#define PSB_FIXED_CASE(ID, ...)                                                                       \
-  case ID:                                                                                            \
-    if constexpr (psb::fixed_plan_compiled<T, ID>::value && psb::FixedPlan<ID>::Radices::NP == 2) \
-      return gor(psb::axis_pass_rr_kernel<T, INV, Pre, ID>);                                          \
-    break;
-      PSB_FIXED_PLANS(PSB_FIXED_CASE)
-#undef PSB_FIXED_CASE
-      default:
-        break;
-    }
-  }
   // Rows read unchanged (a plain copy, every row at its own position): the
   // tile is staged by bulk tensor copies when the view meets TMA's rules.
   if constexpr (std::is_same<Pre, psb::PreCopy<T>>::value) {
@@ -369,31 +397,11 @@ int launch_axis(psb_ctx* c, psb::AxisArgs<T> a, Pre pre, const char* what, const
           launch_pdl(k, grid, 256, tsmem, c->stream, a, map, nbox, c->dstatus);
           return launch_ok(c, what);
         };
-        switch (psb::fixed_plan_id(a.plan)) {
-#define PSB_FIXED_CASE(ID, ...) \
-  case ID:                      \
-    if constexpr (psb::fixed_plan_compiled<T, ID>::value) return got(psb::axis_pass_tma_kernel<T, INV, ID>); \
-    break;
-          PSB_FIXED_PLANS(PSB_FIXED_CASE)
-#undef PSB_FIXED_CASE
-          default:
-            break;
-        }
-        if (!plan_is_wide_h(a.plan)) return got(psb::axis_pass_tma_kernel<T, INV, 0>);
+        if (!plan_is_wide_h(a.plan)) return got(psb::axis_pass_tma_kernel<T, INV>);
       }
     }
   }
   if constexpr (TUNABLE) {
-    switch (psb::fixed_plan_id(a.plan)) {
-#define PSB_FIXED_CASE(ID, ...) \
-  case ID:                      \
-    if constexpr (psb::fixed_plan_compiled<T, ID>::value) return go(psb::axis_pass_kernel<T, INV, Pre, false, ID>); \
-    break;
-      PSB_FIXED_PLANS(PSB_FIXED_CASE)
-#undef PSB_FIXED_CASE
-      default:
-        break;
-    }
     if (sh && sh->wide) return go(psb::axis_pass_kernel<T, INV, Pre, true>);
   }
   return go(psb::axis_pass_kernel<T, INV, Pre>);

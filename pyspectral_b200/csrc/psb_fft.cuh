@@ -117,36 +117,50 @@ __device__ __forceinline__ void dft8(Cx<T>* v) {
   }
 }
 
-// cos and sin of 2 pi q / 48 from a quarter-wave table (steps of 7.5 degrees)
-struct Trig48 {
-  static constexpr double c[13] = {1.0,
-                                   0.99144486137381041114455,
-                                   0.96592582628906828674974,
-                                   0.92387953251128675612818,
-                                   0.86602540378443864676372,
-                                   0.79335334029123516457751,
-                                   0.70710678118654752440084,
-                                   0.60876142900872063941609,
-                                   0.5,
-                                   0.38268343236508977172846,
-                                   0.25881904510252076234890,
-                                   0.13052619222005159154840,
-                                   0.0};
-  static constexpr double cosq(int q) {
-    q = ((q % 48) + 48) % 48;
-    return q <= 12 ? c[q] : (q <= 24 ? -c[24 - q] : (q <= 36 ? -c[q - 24] : c[48 - q]));
+// cos and sin of 2 pi q / R at compile time: the angle is folded into [0, pi/4]
+// in integer units of 2 pi / (8 R), where the Taylor series to x^18 is exact to
+// the last bit or two of a double.
+struct Trig {
+  static constexpr double ser_cos(double x) {
+    const double y = x * x;
+    double s = 1.0;
+    for (int n = 18; n >= 2; n -= 2) s = 1.0 - y / (n * (n - 1.0)) * s;
+    return s;
   }
-  static constexpr double sinq(int q) { return cosq(12 - q); }
+  static constexpr double ser_sin(double x) {
+    const double y = x * x;
+    double s = 1.0;
+    for (int n = 19; n >= 3; n -= 2) s = 1.0 - y / (n * (n - 1.0)) * s;
+    return x * s;
+  }
+  static constexpr double cosq(int q, int R) {
+    int a = 8 * (((q % R) + R) % R);
+    bool neg = false;
+    if (a > 4 * R) a = 8 * R - a;
+    if (a > 2 * R) {
+      a = 4 * R - a;
+      neg = true;
+    }
+    const double u = 0.78539816339744830961566084581988 / R;  // pi / (4 R)
+    const double c = a > R ? ser_sin((2 * R - a) * u) : ser_cos(a * u);
+    return neg ? -c : c;
+  }
+  // sin(2 pi q / R) = cos(2 pi (R - 4 q) / (4 R))
+  static constexpr double sinq(int q, int R) { return cosq(R - 4 * (((q % R) + R) % R), 4 * R); }
 };
 
-// x * W_R^M, W_R = exp(-2 pi i / R) (conjugate for INV); 48 % R == 0
+// x * W_R^M, W_R = exp(-2 pi i / R) (conjugate for INV)
 template <typename T, bool INV, int M, int R>
 __device__ __forceinline__ Cx<T> twc(Cx<T> x) {
-  constexpr int q = (M * (48 / R)) % 48;
+  constexpr int q = M % R;
   if constexpr (q == 0) {
     return x;
+  } else if constexpr (4 * q == R) {
+    return INV ? mul_i(x) : mul_mi(x);
+  } else if constexpr (2 * q == R) {
+    return mk<T>(-x.x, -x.y);
   } else {
-    constexpr T c = (T)Trig48::cosq(q), s = (T)Trig48::sinq(q);
+    constexpr T c = (T)Trig::cosq(q, R), s = (T)Trig::sinq(q, R);
     return INV ? mk<T>(c * x.x - s * x.y, c * x.y + s * x.x) : mk<T>(c * x.x + s * x.y, c * x.y - s * x.x);
   }
 }
@@ -206,9 +220,19 @@ __device__ __forceinline__ void small_dft(Cx<T>* v) {
     DftCT<T, 2, 3, INV>::run(v);
   } else if constexpr (R == 12) {
     DftCT<T, 4, 3, INV>::run(v);
-  } else {
-    static_assert(R == 16, "radix 2, 3, 4, 6, 8, 12 or 16");
+  } else if constexpr (R == 9) {
+    DftCT<T, 3, 3, INV>::run(v);
+  } else if constexpr (R == 16) {
     DftCT<T, 4, 4, INV>::run(v);
+  } else if constexpr (R == 18) {
+    DftCT<T, 6, 3, INV>::run(v);
+  } else if constexpr (R == 24) {
+    DftCT<T, 8, 3, INV>::run(v);
+  } else if constexpr (R == 27) {
+    DftCT<T, 9, 3, INV>::run(v);
+  } else {
+    static_assert(R == 32, "radix 2, 3, 4, 6, 8, 9, 12, 16, 18, 24, 27 or 32");
+    DftCT<T, 8, 4, INV>::run(v);
   }
 }
 

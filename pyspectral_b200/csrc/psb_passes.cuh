@@ -25,6 +25,8 @@
 // index N/2 of x and y and the k3=N/2 plane; pad_2x/unpad_2x keep the -N/2
 // mode).
 #pragma once
+#include <utility>
+
 #include "psb_fft.cuh"
 #include "psb_tma.cuh"
 
@@ -136,26 +138,40 @@ struct AxisArgs {
   const double* k_col;
 };
 
+// For the register passes (psb_reg.cuh): which stored field each destination
+// field of a pass comes from, and its factor.  Pre functors that have such a
+// table provide `fields()`.
+enum FieldKind : unsigned char {
+  kCopy = 0,   // s[a]
+  kIkRow = 1,  // i k_row s[a]
+};
 template <typename T>
-struct PreCopy {
-  static constexpr int F_SRC = 1, F_DST = 1;
-  static constexpr bool FIELDWISE = true;
-  __device__ void operator()(int, int, int, const AxisArgs<T>&, const Cx<T>* s, Cx<T>* d) const { d[0] = s[0]; }
-  __device__ __forceinline__ Cx<T> field(int, int i, int, int col, const AxisArgs<T>& a, const Cx<T>* in) const {
-    return in[i * a.in_rstride + col];
-  }
+struct FieldTab {
+  int nf = 0;
+  unsigned char kind[12] = {}, sa[12] = {};
+  // optional separable factors (m1[row] m2[outer] m3[col]), applied in this order
+  const double *m1 = nullptr, *m2 = nullptr, *m3 = nullptr;
+  const double *f1 = nullptr, *f2 = nullptr, *f3 = nullptr;
 };
 
-// Pre functors that can form any one destination field at a row straight
-// from the inputs (`field(g, i, o, col, a, in)`), so a pass can load its
-// first transform pass's elements from global memory into registers.
 template <class P, class = void>
-struct pre_fieldwise {
+struct pre_has_fields {
   static constexpr bool value = false;
 };
 template <class P>
-struct pre_fieldwise<P, decltype((void)P::FIELDWISE, void())> {
-  static constexpr bool value = P::FIELDWISE;
+struct pre_has_fields<P, decltype((void)sizeof(decltype(std::declval<const P&>().fields())), void())> {
+  static constexpr bool value = true;
+};
+
+template <typename T>
+struct PreCopy {
+  static constexpr int F_SRC = 1, F_DST = 1;
+  __device__ void operator()(int, int, int, const AxisArgs<T>&, const Cx<T>* s, Cx<T>* d) const { d[0] = s[0]; }
+  __host__ FieldTab<T> fields() const {
+    FieldTab<T> t;
+    t.nf = 1;
+    return t;
+  }
 };
 
 // Row of a row map's position p (the inverse of RowMap), or -1.
@@ -178,7 +194,7 @@ __device__ __forceinline__ Cx<T>* axfft(Cx<T>* a, Cx<T>* b, const FFTPlan& p, co
 
 // Transform of a staged tile (F fields x ct columns, position-major in bufA)
 // and the store of its output rows.  Must be called by all threads.
-template <typename T, bool INV, int F, bool WIDE, int FP>
+template <typename T, bool INV, int F, bool WIDE>
 __device__ __forceinline__ void axis_transform_store(const AxisArgs<T>& a, Cx<T>* bufA, Cx<T>* bufB,
                                                      const Cx<T>* tw, int o, int c0) {
   const int ct = a.col_tile;
@@ -188,7 +204,7 @@ __device__ __forceinline__ void axis_transform_store(const AxisArgs<T>& a, Cx<T>
   const int c = threadIdx.x % ct, r0 = threadIdx.x / ct, dr = nt / ct;
   const int col = c0 + c;
   const bool colok = col < a.ncols;
-  Cx<T>* res = axfft<T, INV, WIDE, FP>(bufA, bufB, a.plan, tw, lines);
+  Cx<T>* res = block_fft<T, INV, WIDE>(bufA, bufB, a.plan, tw, lines, 1, lines, true);
   Cx<T>* outb = a.out + (long long)o * a.out_ostride;
   if (!colok || threadIdx.x >= dr * ct) return;
   const int nrow = a.out_rows * F;
@@ -236,7 +252,7 @@ __device__ __forceinline__ bool tma_issue(const CUtensorMap* map, Cx<T>* dst, si
   return true;
 }
 
-template <typename T, bool INV, class Pre, bool WIDE = false, int FP = 0>
+template <typename T, bool INV, class Pre, bool WIDE = false>
 __device__ __forceinline__ void axis_pass_body(const AxisArgs<T>& a, const Pre& pre, int bx, int by) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   Cx<T>* tw = reinterpret_cast<Cx<T>*>(smem_raw);
@@ -298,7 +314,7 @@ __device__ __forceinline__ void axis_pass_body(const AxisArgs<T>& a, const Pre& 
     }
   }
   __syncthreads();
-  axis_transform_store<T, INV, Pre::F_DST, WIDE, FP>(a, bufA, bufB, tw, o, c0);
+  axis_transform_store<T, INV, Pre::F_DST, WIDE>(a, bufA, bufB, tw, o, c0);
 }
 
 // TMA-staged axis pass for passes that read their rows unchanged (PreCopy,
@@ -308,7 +324,7 @@ __device__ __forceinline__ void axis_pass_body(const AxisArgs<T>& a, const Pre& 
 // A copy that does not complete within the poll limit raises *status and the
 // CTA writes NaN in place of its tile (after waiting again, bounded, for the
 // copy to land).
-template <typename T, bool INV, int FP = 0>
+template <typename T, bool INV>
 __global__ void __launch_bounds__(256) axis_pass_tma_kernel(AxisArgs<T> a, const __grid_constant__ CUtensorMap map,
                                                             int nbox, int* status) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -347,99 +363,20 @@ __global__ void __launch_bounds__(256) axis_pass_tma_kernel(AxisArgs<T> a, const
     for (int l = threadIdx.x; l < L * ct; l += blockDim.x) bufA[l] = mk<T>(nan_of<T>(), nan_of<T>());
     __syncthreads();
   }
-  axis_transform_store<T, INV, 1, false, FP>(a, bufA, bufB, tw, o, c0);
-}
-
-// ---------------------------------------------------------------------------
-// Two-pass axis transform with global memory on both sides.  For a compiled
-// schedule of exactly two radices (L = R1 R2) the first Stockham pass loads
-// its R1 elements of a line straight from the input rows (the Pre functor
-// forms the line's field on load: `field`), and the second stores its R2
-// results straight to the output rows; the only shared-memory traffic is the
-// exchange between the passes (one store and one load per element instead of
-// the staged tile's six) and the only barrier is the one between them.
-// Items walk the lines fast (line = field * ct + column), so consecutive
-// threads touch consecutive columns in global memory and consecutive lines
-// in the exchange buffer.  smem = L twiddles + L * F * ct elements.
-template <typename T, bool INV, class Pre, int FP>
-__device__ __forceinline__ void axis_rr_body(const AxisArgs<T>& a, const Pre& pre, int bx, int by) {
-  using FPl = FixedPlan<FP>;
-  constexpr int L = FPl::L, R1 = FPl::Radices::A, R2 = FPl::Radices::B;
-  static_assert(FPl::Radices::NP == 2 && R1 * R2 == L, "two-pass schedules only");
-  constexpr int F = Pre::F_DST, NB1 = L / R1, NB2 = L / R2;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  Cx<T>* tw = reinterpret_cast<Cx<T>*>(smem_raw);
-  const int ct = a.col_tile, lines = F * ct;
-  Cx<T>* X = tw + L;
-  const int o = by, c0 = bx * ct;
-  const Cx<T> zero = mk<T>(0, 0);
-  pdl_trigger();
-  stage_twiddles(tw, a.tw, a.plan);
-  pdl_wait();
-  const Cx<T>* inb = a.in + (long long)o * a.in_ostride;
-  for (Walk2 w(lines); w.s < NB1; w.next()) {
-    const int line = w.f, j1 = w.s;
-    const int g = line / ct, col = c0 + (line - g * ct);
-    Cx<T> v[R1];
-#pragma unroll
-    for (int r = 0; r < R1; ++r) {
-      const int i = row_of(a.in_map, j1 + r * NB1, a.in_rows);
-      v[r] = (i >= 0 && col < a.ncols) ? pre.field(g, i, o, col, a, inb) : zero;
-    }
-    small_dft<T, R1, INV>(v);
-#pragma unroll
-    for (int r = 0; r < R1; ++r) X[(size_t)(j1 * R1 + r) * lines + line] = v[r];
-  }
-  __syncthreads();
-  Cx<T>* outb = a.out + (long long)o * a.out_ostride;
-  for (Walk2 w(lines); w.s < NB2; w.next()) {
-    const int line = w.f, j2 = w.s;
-    const int g = line / ct, col = c0 + (line - g * ct);
-    const int k = j2 % R1;
-    Cx<T> v[R2];
-#pragma unroll
-    for (int r = 0; r < R2; ++r) v[r] = X[(size_t)(j2 + r * NB2) * lines + line];
-    // twiddles W_L^{r k} (sub-transform length R1: the table's stride L / (R1 R2) is 1)
-#pragma unroll
-    for (int r = 1; r < R2; ++r) {
-      Cx<T> t = tw[r * k];
-      if (INV) t.y = -t.y;
-      v[r] = cmul(v[r], t);
-    }
-    small_dft<T, R2, INV>(v);
-    if (col < a.ncols) {
-#pragma unroll
-      for (int r = 0; r < R2; ++r) {
-        const int i = row_of(a.out_map, (j2 - k) * R2 + k + r * R1, a.out_rows);
-        if (i >= 0) outb[g * a.out_fstride + i * a.out_rstride + col] = a.scale * v[r];
-      }
-    }
-  }
-  // output rows the map leaves without a position are zero
-  const int zlo = a.out_map.lo, zhi = min(a.out_map.hi, a.out_rows);
-  for (int t = threadIdx.x; zlo < zhi && t < (zhi - zlo) * lines; t += blockDim.x) {
-    const int line = t % lines, i = zlo + t / lines;
-    const int g = line / ct, col = c0 + (line - g * ct);
-    if (col < a.ncols) outb[g * a.out_fstride + i * a.out_rstride + col] = zero;
-  }
-}
-
-template <typename T, bool INV, class Pre, int FP>
-__global__ void __launch_bounds__(256) axis_pass_rr_kernel(AxisArgs<T> a, Pre pre) {
-  axis_rr_body<T, INV, Pre, FP>(a, pre, blockIdx.x, blockIdx.y);
+  axis_transform_store<T, INV, 1, false>(a, bufA, bufB, tw, o, c0);
 }
 
 // grid = (ceil(ncols/col_tile), nouter)
-template <typename T, bool INV, class Pre, bool WIDE = false, int FP = 0>
+template <typename T, bool INV, class Pre, bool WIDE = false>
 __global__ void __launch_bounds__(256) axis_pass_kernel(AxisArgs<T> a, Pre pre) {
-  axis_pass_body<T, INV, Pre, WIDE, FP>(a, pre, blockIdx.x, blockIdx.y);
+  axis_pass_body<T, INV, Pre, WIDE>(a, pre, blockIdx.x, blockIdx.y);
 }
 
 // Batched: grid = (ceil(ncols/col_tile), nouter, runs); run blockIdx.z takes
 // its arguments from A[z] and pre[z] (same tile shape for every run).
-template <typename T, bool INV, class Pre, bool WIDE, int FP = 0>
+template <typename T, bool INV, class Pre, bool WIDE>
 __global__ void __launch_bounds__(256) axis_pass_batch(const AxisArgs<T>* __restrict__ A, const Pre* __restrict__ pre) {
-  axis_pass_body<T, INV, Pre, WIDE, FP>(A[blockIdx.z], pre[blockIdx.z], blockIdx.x, blockIdx.y);
+  axis_pass_body<T, INV, Pre, WIDE>(A[blockIdx.z], pre[blockIdx.z], blockIdx.x, blockIdx.y);
 }
 
 // ---------------------------------------------------------------------------

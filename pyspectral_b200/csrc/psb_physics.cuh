@@ -83,19 +83,28 @@ struct StepIO {
   }
 };
 
+// field table of a pass that copies fields 0..nf-1, each times m1[row] m2[outer] m3[col] when given
+template <typename T>
+__host__ inline FieldTab<T> copy_fields(int nf, const double* m1 = nullptr, const double* m2 = nullptr,
+                                        const double* m3 = nullptr) {
+  FieldTab<T> t;
+  t.nf = nf;
+  for (int f = 0; f < nf; ++f) t.sa[f] = (unsigned char)f;
+  t.m1 = m1;
+  t.m2 = m2;
+  t.m3 = m3;
+  return t;
+}
+
 // ---- 3/2-padded Navier-Stokes: DNS and Smagorinsky --------------------------
 template <typename T, int F>
 struct PreCopyN {
   static constexpr int F_SRC = F, F_DST = F;
-  static constexpr bool FIELDWISE = true;
   __device__ void operator()(int, int, int, const AxisArgs<T>&, const Cx<T>* s, Cx<T>* d) const {
 #pragma unroll
     for (int f = 0; f < F; ++f) d[f] = s[f];
   }
-  // field g of row i, column col, read from the row's inputs (in: the outer index's base)
-  __device__ __forceinline__ Cx<T> field(int g, int i, int, int col, const AxisArgs<T>& a, const Cx<T>* in) const {
-    return in[g * a.in_fstride + i * a.in_rstride + col];
-  }
+  __host__ FieldTab<T> fields() const { return copy_fields<T>(F); }
 };
 
 // (u,v,w) -> (u,v,w,S11,S22,S33,S12,S13,S23), S_ij = (i/2)(k_j u_i + k_i u_j)
@@ -103,15 +112,6 @@ struct PreCopyN {
 template <typename T>
 struct PreStrain {
   static constexpr int F_SRC = 3, F_DST = 9;
-  static constexpr bool FIELDWISE = true;
-  __device__ __forceinline__ Cx<T> field(int g, int i, int o, int col, const AxisArgs<T>& a, const Cx<T>* in) const {
-    auto src = [&](int f) { return in[f * a.in_fstride + i * a.in_rstride + col]; };
-    const T k[3] = {(T)a.k_row[i], (T)a.k_outer[o], (T)a.k_col[col]};
-    if (g < 3) return src(g);
-    if (g < 6) return pik(k[g - 3], src(g - 3));
-    const int p = g == 6 ? 0 : (g == 7 ? 0 : 1), q = g == 6 ? 1 : 2;  // S_pq
-    return (T)0.5 * (pik(k[q], src(p)) + pik(k[p], src(q)));
-  }
   __device__ void operator()(int i, int o, int c, const AxisArgs<T>& a, const Cx<T>* s, Cx<T>* d) const {
     const T k1 = (T)a.k_row[i], k2 = (T)a.k_outer[o], k3 = (T)a.k_col[c];
     d[0] = s[0];
@@ -251,6 +251,7 @@ struct PreMask6 {
 #pragma unroll
     for (int f = 0; f < 6; ++f) d[f] = m * s[f];
   }
+  __host__ FieldTab<T> fields() const { return copy_fields<T>(6, m1, m2, m3); }
 };
 
 // (u_i u_j - B_i B_j) and u x B (:117-134; the momentum and pressure terms are
@@ -686,10 +687,12 @@ struct PreGrad {
 template <typename T>
 struct PreYGrad {
   static constexpr int F_SRC = 2, F_DST = 3, GROUPS = 3, IN_FIELDS = 3, OUT_FIELDS = 3;
-  static constexpr bool FIELDWISE = true;
-  __device__ __forceinline__ Cx<T> field(int g, int i, int, int col, const AxisArgs<T>& a, const Cx<T>* in) const {
-    const Cx<T> v = in[(g == 1 ? a.in_fstride : 0) + i * a.in_rstride + col];
-    return g == 2 ? pik((T)a.k_row[i], v) : v;
+  __host__ FieldTab<T> fields() const {
+    FieldTab<T> t;
+    t.nf = 3;
+    t.sa[1] = 1;
+    t.kind[2] = kIkRow;
+    return t;
   }
   __device__ void operator()(int i, int, int, const AxisArgs<T>& a, const Cx<T>* s, Cx<T>* d) const {
     d[0] = s[0];
@@ -706,10 +709,14 @@ struct PreYGrad {
 template <typename T>
 struct PreGradXY {
   static constexpr int F_SRC = 3, F_DST = 6, F_B = 9, Z_DERIVED = 3;
-  static constexpr bool FIELDWISE = true;
-  __device__ __forceinline__ Cx<T> field(int g, int i, int, int col, const AxisArgs<T>& a, const Cx<T>* in) const {
-    const Cx<T> v = in[(g < 3 ? g : g - 3) * a.in_fstride + i * a.in_rstride + col];
-    return g < 3 ? v : pik((T)a.k_row[i], v);
+  __host__ FieldTab<T> fields() const {
+    FieldTab<T> t;
+    t.nf = 6;
+    for (int g = 0; g < 6; ++g) {
+      t.sa[g] = (unsigned char)(g % 3);
+      t.kind[g] = g < 3 ? kCopy : kIkRow;
+    }
+    return t;
   }
   using YPass = PreYGrad<T>;
   __device__ void operator()(int i, int, int, const AxisArgs<T>& a, const Cx<T>* s, Cx<T>* d) const {

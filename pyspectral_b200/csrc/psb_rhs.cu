@@ -165,6 +165,7 @@ struct PreMask3 {
     d[1] = g * s[1];
     d[2] = g * s[2];
   }
+  __host__ FieldTab<T> fields() const { return copy_fields<T>(3, g1, g2, g3); }
 };
 
 template <typename T>
@@ -1550,6 +1551,13 @@ struct PreMask3x2 {
 #pragma unroll
     for (int q = 0; q < 3; ++q) d[q] = f * (m * s[q]);
   }
+  __host__ FieldTab<T> fields() const {
+    FieldTab<T> t = copy_fields<T>(3, m1, m2, m3);
+    t.f1 = f1;
+    t.f2 = f2;
+    t.f3 = f3;
+    return t;
+  }
 };
 
 template <typename T>
@@ -1933,6 +1941,7 @@ bool plan_is_wide(const FFTPlan& p) {
 // Fy / Gy: lines per column and outer groups of the y-inverse pass
 struct TuneDims {
   int Fi, Fb, Fz, Fo, maxppc, defppc, Fy = 1, Gy;
+  bool regx = true, regy = true;  // the x- / y-inverse pass has a register form
   size_t zextra = 0;
   int Ls[5], Fs[5];
 };
@@ -1946,6 +1955,7 @@ TuneDims tune_dims(psb_ctx* c, int closure) {
     t.defppc = phys_default_ppc<PhysProducts<T>>::value;
   } else if (closure == PSB_SMAG) {
     t.Fi = t.Fb = t.Gy = 9, t.Fo = 12, t.maxppc = phys_max_ppc<PhysSmag<T>>::value;
+    t.regx = psb::pre_has_fields<PreStrain<T>>::value;
     t.Fz = PhysSmag<T>::F_IN;
     t.defppc = phys_default_ppc<PhysSmag<T>>::value;
   } else {
@@ -1974,12 +1984,20 @@ size_t pass_smem(const TuneDims& t, int k, int tile) {
   return (size_t)(t.Ls[k] + 2 * (size_t)t.Ls[k] * t.Fs[k] * tile) * sizeof(Cx<T>);
 }
 
+// Untuned shape of axis pass k (x-inverse, y-inverse, y-forward, x-forward).
+template <typename T>
+void default_pass_shape(psb_ctx* c, const TuneDims& t, int k, psb_pass_shape& sh) {
+  const int nouter = k == 0 || k == 4 ? c->N2 : (k == 1 ? t.Gy * t.Ls[0] : t.Fo * t.Ls[0]);
+  const bool reg = k == 0 ? t.regx : (k == 1 ? t.regy : k == 3);
+  default_axis_shape<T>(c, t.Ls[k], c->N3 / 2, t.Fs[k], nouter, reg, sh.tile, sh.plan);
+}
+
 template <typename T>
 int tune_rhs(psb_ctx* c, int closure, const void* state, const psb_params* p) {
   const int N1 = c->N1, N2 = c->N2, N3 = c->N3, N3h = c->N3h;
   const int M1 = 3 * N1 / 2, M2 = 3 * N2 / 2, M3 = 3 * N3 / 2, Kz = N3 / 2;
   const TuneDims td = tune_dims<T>(c, closure);
-  const int Fi = td.Fi, Fz = td.Fz, Fo = td.Fo, maxppc = td.maxppc, defppc = td.defppc, Fy = td.Fy, Gy = td.Gy;
+  const int Fz = td.Fz, Fo = td.Fo, maxppc = td.maxppc, defppc = td.defppc;
   const size_t zextra = td.zextra;
   const size_t esz = sizeof(Cx<T>);
   const size_t n = (size_t)3 * N1 * N2 * N3h;
@@ -2000,12 +2018,9 @@ int tune_rhs(psb_ctx* c, int closure, const void* state, const psb_params* p) {
   psb_tuned t;
   const int* Ls = td.Ls;
   const int* Fs = td.Fs;
-  t.pass[0].tile = pick_ct(Kz, Fi, M1, esz, N2);
-  t.pass[1].tile = pick_ct(Kz, Fy, M2, esz, Gy * M1);
+  for (int k : {0, 1, 3, 4}) default_pass_shape<T>(c, td, k, t.pass[k]);
   t.pass[2].tile = P;
-  t.pass[3].tile = pick_ct(Kz, 1, M2, esz, Fo * M1);
-  t.pass[4].tile = pick_ct(Kz, Fo, M1, esz, N2);
-  for (int k = 0; k < 5; ++k) t.pass[k].plan = *plan_for(c, Ls[k]);
+  t.pass[2].plan = *plan_for(c, M3);
   c->tuned[closure] = t;
   static const char* names[5] = {"x-inverse", "y-inverse", "z-fused", "y-forward", "x-forward+epilogue"};
   const int timing_was = c->timing;
@@ -2033,6 +2048,8 @@ int tune_rhs(psb_ctx* c, int closure, const void* state, const psb_params* p) {
   for (int k = 0; k < 5 && status == PSB_OK; ++k) {
     psb_pass_shape& cur = c->tuned[closure].pass[k];
     const psb_pass_shape inc = cur;
+    // a register pass has one shape (the runtime-schedule shapes of its length are slower throughout)
+    if (k != 2 && is_reg_axis(inc.plan)) continue;
     float base = 0.f;
     if ((status = time_pass(k, 6, &base)) != PSB_OK) break;
     std::vector<int> tiles;
@@ -2089,8 +2106,17 @@ int set_shape(psb_ctx* c, int closure, int k, int tile, const int* radices, int 
   bool wide = false;
   FFTPlan q = *plan_for(c, L);
   q.npass = nrad;
+  // the register pass's own radices name it (its tile is fixed)
+  FFTPlan rp = q;
+  const bool reg_shape = (k == 0 ? td.regx : (k == 1 ? td.regy : k == 3)) && nrad == 2 && reg_axis_plan(L, rp) &&
+                         radices[0] == rp.radix[0] && radices[1] == rp.radix[1];
   for (int s = 0; s < nrad; ++s) {
     const int r = radices[s];
+    if (reg_shape) {
+      q.radix[s] = r;
+      prod *= r;
+      continue;
+    }
     if (r != 2 && r != 3 && r != 4 && r != 6 && r != 8 && r != 12 && r != 16)
       return fail(c, PSB_ERR_ARG, "psb_set_tuned_shape: radices must be 2, 3, 4, 6, 8, 12 or 16");
     wide = wide || r > 8 || r == 6;
@@ -2104,23 +2130,18 @@ int set_shape(psb_ctx* c, int closure, int k, int tile, const int* radices, int 
   const int tmax = k == 2 ? td.maxppc : 32;
   if (tile < 1 || tile > tmax || (tile & (tile - 1)))
     return fail(c, PSB_ERR_ARG, "psb_set_tuned_shape: tile must be a power of two <= " + std::to_string(tmax));
-  if (pass_smem<T>(td, k, tile) > kSmemBudget)
+  if (!reg_shape && pass_smem<T>(td, k, tile) > kSmemBudget)
     return fail(c, PSB_ERR_SHAPE, "psb_set_tuned_shape: tile needs more shared memory than the budget");
   auto it = c->tuned.find(closure);
   if (it == c->tuned.end()) {
     // start from the default shapes of every pass
-    const int Kz = c->N3 / 2;
-    const size_t esz = sizeof(Cx<T>);
     psb_tuned t;
     int P = td.defppc;
     while (P > 1 && pass_smem<T>(td, 2, P) > kSmemBudget) P /= 2;
     while (P > 1 && ((long long)td.Ls[0] * td.Ls[1] + P - 1) / P < 2 * 148) P /= 2;
-    t.pass[0].tile = pick_ct(Kz, td.Fi, td.Ls[0], esz, c->N2);
-    t.pass[1].tile = pick_ct(Kz, td.Fy, td.Ls[1], esz, td.Gy * td.Ls[0]);
+    for (int j : {0, 1, 3, 4}) default_pass_shape<T>(c, td, j, t.pass[j]);
     t.pass[2].tile = P;
-    t.pass[3].tile = pick_ct(Kz, 1, td.Ls[3], esz, td.Fo * td.Ls[0]);
-    t.pass[4].tile = pick_ct(Kz, td.Fo, td.Ls[4], esz, c->N2);
-    for (int j = 0; j < 5; ++j) t.pass[j].plan = *plan_for(c, td.Ls[j]);
+    t.pass[2].plan = *plan_for(c, td.Ls[2]);
     it = c->tuned.emplace(closure, t).first;
   }
   psb_pass_shape& sh = it->second.pass[k];
