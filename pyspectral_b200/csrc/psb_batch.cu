@@ -136,6 +136,28 @@ struct Batch {
   static constexpr bool reg_pass(int pass) {
     return pass == 0 ? has_fields<Pre>() : (pass == 1 ? has_fields<YPre>() : pass == 3);
   }
+  // The z pass runs as a register pass (its plan is the register pass's {A, B, 2}).
+  bool reg_z_pass() const {
+    FFTPlan q{};
+    if constexpr (z_registered<Phys>::value) {
+      if (!has_reg_z<T, Phys>(d.M3)) return false;
+      reg_z_shape<T, Phys>(d.M3, (long long)d.M1 * d.M2 * R, q);
+      return b->plan[2].npass == q.npass && std::equal(q.radix, q.radix + q.npass, b->plan[2].radix);
+    }
+    return false;
+  }
+  // Pencils per CTA and plan of the staged z pass: the pass's own shape, or the default
+  // where the register pass runs (the persistent ensemble runs the staged one).
+  void generic_z(int& P, FFTPlan& plan) const {
+    P = b->tile[2];
+    plan = b->plan[2];
+    if (!reg_z_pass()) return;
+    plan = *plan_for(c, d.M3);
+    P = phys_default_ppc<Phys>::value;
+    while (P > 1 && smem_z(P) > kSmemBudget) P /= 2;
+    const long long np = (long long)d.M1 * d.M2;
+    while (P > 1 && (np + P - 1) / P * R < 2 * 148) P /= 2;
+  }
   // Column tile and plan in the argument blocks of axis pass `pass`: the pass's own shape, or,
   // where the pass runs as a register pass (which takes neither), the default of the
   // runtime-schedule bodies that the persistent ensemble runs on the same blocks.
@@ -211,9 +233,8 @@ struct Batch {
       }
       z.out_kz = d.Kz;
       z.npencils = (long long)d.M1 * d.M2;
-      z.ppc = b->tile[2];
+      generic_z(z.ppc, z.plan);
       z.fac = (T)(s32 / ((double)d.M1 * d.M2 * d.M3));
-      z.plan = b->plan[2];
       z.tw = twiddles<T>(c);
       az[r] = z;
       AxisArgs<T> yf{};
@@ -382,6 +403,10 @@ struct Batch {
       case 2: {
         const int P = b->tile[2];
         const long long np = (long long)d.M1 * d.M2;
+        if constexpr (z_registered<Phys>::value)
+          if (reg_z_pass())
+            return reg_z_batch<T, Phys>(c, az, phys, d.M3, np, R, "batch z-fused",
+                                        (double)R * esz * np * d.Kz * (Fb + Fo));
         const long long items = (np + P - 1) / P * R;
         const size_t sm = smem_z(P);
         // persistent over (run, tile): at most the resident CTAs of the device
@@ -392,25 +417,6 @@ struct Batch {
           launch_pdl(k, dim3((unsigned)g), 256, sm, c->stream, (const ZArgs<T>*)az, (const Phys*)phys, R);
           return launch_ok(c, "batch z-fused");
         };
-        // a compiled two-pass (R1, 16) schedule with pencils paired: register-direct
-        if constexpr (phys_fixed_fft<Phys>::value && sizeof(T) == 4) {
-          if ((P & 1) == 0 && c->use_zrr) {
-            switch (fixed_plan_id(b->plan[2])) {
-#define PSB_FIXED_CASE(ID, ...)                                                   \
-  case ID:                                                                        \
-    if constexpr (zrr_plan<ID>::value && zrr_plan<ID>::R2 == 16) return go(zpass_rr_batch<T, Phys, ID>); \
-    break;
-              PSB_FIXED_PLANS(PSB_FIXED_CASE)
-#undef PSB_FIXED_CASE
-              default:
-                break;
-            }
-          }
-        }
-        if constexpr (phys_fixed_fft<Phys>::value)
-          return by_plan(
-              2, [&](auto id) { return go(zpass_batch<T, Phys, false, decltype(id)::value>); },
-              [&] { return go(zpass_batch<T, Phys, W>); });
         return go(zpass_batch<T, Phys, W>);
       }
       default: {
@@ -475,7 +481,7 @@ struct Batch {
     for (int pass = 0; pass < 5; ++pass) PSB_TRY(launch(pass, 4));
     for (int pass = 0; pass < 5; ++pass) {
       // a register pass has one shape (the runtime-schedule shapes of its length are slower throughout)
-      if (pass != 2 && reg_pass(pass) && is_reg_axis(b->plan[pass])) continue;
+      if (pass == 2 ? reg_z_pass() : reg_pass(pass) && is_reg_axis(b->plan[pass])) continue;
       std::vector<int> tiles;
       if (pass == 2) {
         for (int P : {1, 2, 4, 8})
@@ -599,9 +605,9 @@ int run_batch(psb_batch* b, int nsteps, bool tune, Pre pre0, Phys (*mkphys)(psb_
   if (b->plan[0].L == 0) {
     default_shapes<T>(b, BT::Fi, BT::Fb, Phys::F_IN, BT::Fo, BT::YPre::F_DST, BT::YP::groups, &BT::reg_pass,
                    phys_default_ppc<Phys>::value, (size_t)phys_is_block<Phys>::extra);
-    // the register-direct z pass's schedule where it exists (as for single runs)
-    if constexpr (phys_fixed_fft<Phys>::value && sizeof(T) == 4)
-      if ((b->tile[2] & 1) == 0 && c->use_zrr) zrr_default_plan(b->plan[2]);
+    if constexpr (z_registered<Phys>::value)
+      if (c->use_zrr && has_reg_z<T, Phys>(x.d.M3))
+        b->tile[2] = reg_z_shape<T, Phys>(x.d.M3, (long long)x.d.M1 * x.d.M2 * x.R, b->plan[2]);
   }
   if (b->dirty) {
     PSB_TRY(x.build(pre0, mkphys, mkepi));
@@ -759,6 +765,10 @@ size_t ens_group(psb_batch* b, int kind, EnsGroup& g) {
   for (int k : {0, 1, 3}) {
     FFTPlan plan;
     x.generic_shape(k, t[k], plan);
+  }
+  {
+    FFTPlan plan;
+    x.generic_z(t[2], plan);
   }
   g.nx[0] = (d.Kz + t[0] - 1) / t[0];
   g.ny[0] = d.N2;

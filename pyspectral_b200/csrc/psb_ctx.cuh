@@ -15,6 +15,7 @@
 #include "../../include/pyspectral_b200.h"
 #include "psb_physics.cuh"
 #include "psb_reg.cuh"
+#include "psb_zreg.cuh"
 
 // Launch shape of one pass picked by the autotuner: tile (columns per CTA, or
 // pencils per CTA for the z pass), its transform's radix order, and whether
@@ -23,6 +24,7 @@ struct psb_pass_shape {
   int tile = 0;
   psb::FFTPlan plan{};
   bool wide = false;
+  bool reg = false;  // the register pass's own shape: the runtime-schedule kernels ignore it
 };
 // Shapes of the five passes (x-inverse, y-inverse, z, y-forward, x-forward) of
 // a 3/2-padded closure's RHS.
@@ -65,7 +67,7 @@ struct psb_ctx {
   unsigned long long launches = 0;
   int timing = 0;
   int use_tma = 1;          // stage eligible pass inputs with bulk tensor copies
-  int use_zrr = 1;          // register-direct z-pass for two-pass (R1, 16) schedules
+  int use_zrr = 1;          // register z pass where the length has one (0: the staged one)
   int* dstatus = nullptr;   // device status word (a bounded wait gave up), owned
   struct Rec {
     std::string name;
@@ -241,31 +243,34 @@ inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, int block, si
 // the largest shared-memory carveout first: under 48 KB per CTA the default
 // carveout would otherwise leave room for fewer CTAs than the registers and
 // shared memory allow (one per SM was seen).  Results are cached per
-// (kernel, device, shared memory) in a fixed table.
+// (kernel, device, shared memory) in a fixed table under a mutex (host threads
+// of several contexts launch).
 struct OccCache {
   const void* fn[256];
   int dev[256];
   size_t smem[256];
   int per[256], nsm[256];
   int n = 0;
+  std::mutex mu;
 };
 inline OccCache& occ_cache() {
   static OccCache c;
   return c;
 }
 template <typename K>
-inline long long persistent_grid(K kernel, size_t smem, long long ntiles) {
+inline long long persistent_grid(K kernel, size_t smem, long long ntiles, int block = 256) {
   int dev = 0;
   cudaGetDevice(&dev);
   OccCache& oc = occ_cache();
   const void* f = reinterpret_cast<const void*>(kernel);
+  std::lock_guard<std::mutex> lk(oc.mu);
   for (int i = 0; i < oc.n; ++i)
     if (oc.fn[i] == f && oc.dev[i] == dev && oc.smem[i] == smem)
       return std::min<long long>(ntiles, (long long)oc.per[i] * oc.nsm[i]);
   int nsm = 0, per = 0;
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, 256, smem) != cudaSuccess || per < 1 || nsm < 1) {
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, block, smem) != cudaSuccess || per < 1 || nsm < 1) {
     (void)cudaGetLastError();
     return ntiles;
   }
@@ -341,6 +346,61 @@ template <typename T>
 int reg_axis_batch(psb_ctx* c, const psb::AxisArgs<T>* args, const psb::FieldTab<T>& ft, int L, int ncols, int nouter,
                    int runs, bool inv, const char* what, double bytes);
 
+// ---- register z pass (psb_zreg.cuh; launched by the psb_z_*.cu files) ----
+// Whether physics Phys has a register z pass of H = M/2 complex points: the 3/2-padded
+// closures (Smagorinsky, learned) run multiples of three only.
+template <class Phys>
+struct z_pad32_only {
+  static constexpr bool value = false;
+};
+template <typename T>
+struct z_pad32_only<psb::PhysSmag<T>> {
+  static constexpr bool value = true;
+};
+template <typename T, int ACT, int HID>
+struct z_pad32_only<psb::PhysLearned<T, ACT, HID>> {
+  static constexpr bool value = true;
+};
+template <class Phys>
+constexpr bool z_plan_of(int H) {
+  return !z_pad32_only<Phys>::value || H % 3 == 0;
+}
+// physics with instantiated register z passes (the GELU network keeps the staged one)
+template <class Phys>
+struct z_registered {
+  static constexpr bool value = psb::Mid<Phys>::value;
+};
+template <typename T, int HID>
+struct z_registered<psb::PhysLearned<T, psb::kActGelu, HID>> {
+  static constexpr bool value = false;
+};
+template <typename T, class Phys>
+inline bool has_reg_z(int M) {
+  if constexpr (z_registered<Phys>::value) {
+    switch (M) {
+#define PSB_CASE(H, A, B) \
+  case 2 * H:             \
+    return z_plan_of<Phys>(H);
+      PSB_REG_Z_F64(PSB_CASE)
+      case 432:
+      case 512:
+        return sizeof(T) == 4 && z_plan_of<Phys>(M / 2);
+      default:
+        return false;
+#undef PSB_CASE
+    }
+  }
+  return false;
+}
+template <typename T, class Phys>
+int reg_z(psb_ctx* c, const psb::ZArgs<T>& z, const Phys& phys, const char* what, double bytes);
+template <typename T, class Phys>
+int reg_z_batch(psb_ctx* c, const psb::ZArgs<T>* args, const Phys* phys, int M, long long npencils, int runs,
+                const char* what, double bytes);
+// pencils per CTA and radices {A, B, 2} of the register z pass of M points (0: none)
+template <typename T, class Phys>
+int reg_z_shape(int M, long long npencils, FFTPlan& plan);
+
 // Launch shape (tile and radices) of an axis pass that no tuner has touched.
 template <typename T>
 inline void default_axis_shape(psb_ctx* c, int L, int ncols, int F, int nouter, bool reg, int& tile, FFTPlan& plan) {
@@ -357,7 +417,7 @@ int launch_axis(psb_ctx* c, psb::AxisArgs<T> a, Pre pre, const char* what, const
   const size_t esz = sizeof(Cx<T>);
   const int L = a.plan.L;
   a.col_tile = pick_ct(a.ncols, Pre::F_DST, L, esz, a.nouter);
-  if (sh && sh->tile) {
+  if (sh && sh->tile && !sh->reg) {
     a.col_tile = sh->tile;
     a.plan = sh->plan;
   }
@@ -416,23 +476,24 @@ int launch_z(psb_ctx* c, psb::ZArgs<T> z, Phys phys, const char* what, double ex
   constexpr size_t extra = (size_t)psb::phys_is_block<Phys>::extra;
   (void)esz;
   auto smem_for = [&](int P) { return psb::zpass_smem_bytes<T>(FMAX, P, M, extra); };
-  int P = psb::phys_default_ppc<Phys>::value;
-  while (P > 1 && smem_for(P) > kSmemBudget) P /= 2;
-  while (P > 1 && (z.npencils + P - 1) / P < 2 * 148) P /= 2;
-  if (sh && sh->tile) {
-    P = sh->tile;
-    z.plan = sh->plan;
-  } else if constexpr (psb::phys_fixed_fft<Phys>::value && sizeof(T) == 4) {
-    // default shape: the register-direct z pass where its schedule exists
-    if ((P & 1) == 0 && c->use_zrr) psb::zrr_default_plan(z.plan);
-  }
-  z.ppc = P;
-  const size_t smem = smem_for(P);
-  const long long grid = (z.npencils + P - 1) / P;
   double bytes = extra_bytes + (double)esz * z.npencils * Phys::F_OUT * z.out_kz;
   // a field formed as d/dz of another input re-reads that input's line: no new bytes
   for (int f = 0; f < Phys::F_IN; ++f)
     if (!z.dz[f]) bytes += (double)esz * z.npencils * z.in_kz[f];
+  // the register z pass of this length (psb_zreg.cuh), where there is one; a tuned shape applies to
+  // the staged one
+  if constexpr (z_registered<Phys>::value)
+    if (c->use_zrr && has_reg_z<T, Phys>(M)) return reg_z<T, Phys>(c, z, phys, what, bytes);
+  int P = psb::phys_default_ppc<Phys>::value;
+  while (P > 1 && smem_for(P) > kSmemBudget) P /= 2;
+  while (P > 1 && (z.npencils + P - 1) / P < 2 * 148) P /= 2;
+  if (sh && sh->tile && !sh->reg) {
+    P = sh->tile;
+    z.plan = sh->plan;
+  }
+  z.ppc = P;
+  const size_t smem = smem_for(P);
+  const long long grid = (z.npencils + P - 1) / P;
   auto go = [&](auto k) {
     set_smem(k, smem);
     const long long g = persistent_grid(k, smem, grid);
@@ -440,36 +501,6 @@ int launch_z(psb_ctx* c, psb::ZArgs<T> z, Phys phys, const char* what, double ex
     launch_pdl(k, dim3((unsigned)g), 256, smem, c->stream, z, phys);
     return launch_ok(c, what);
   };
-  // A compiled two-pass schedule (R1, 16) with pencils paired per packed line
-  // (P even): the register-direct z-pass, whose transforms read the packed
-  // spectra from and write them to global memory (psb::zpass_rr_tile).
-  if constexpr (psb::phys_fixed_fft<Phys>::value && sizeof(T) == 4) {
-    if ((P & 1) == 0 && c->use_zrr) {
-      switch (psb::fixed_plan_id(z.plan)) {
-#define PSB_FIXED_CASE(ID, ...)                                                                   \
-  case ID:                                                                                        \
-    if constexpr (psb::zrr_plan<ID>::value && psb::zrr_plan<ID>::R2 == 16)                      \
-      return go(psb::zpass_rr_kernel<T, Phys, ID>);                                               \
-    break;
-        PSB_FIXED_PLANS(PSB_FIXED_CASE)
-#undef PSB_FIXED_CASE
-        default:
-          break;
-      }
-    }
-  }
-  if constexpr (psb::phys_fixed_fft<Phys>::value) {
-    switch (psb::fixed_plan_id(z.plan)) {
-#define PSB_FIXED_CASE(ID, ...) \
-  case ID:                      \
-    if constexpr (psb::fixed_plan_compiled<T, ID>::value) return go(psb::zpass_kernel<T, Phys, false, ID>); \
-    break;
-      PSB_FIXED_PLANS(PSB_FIXED_CASE)
-#undef PSB_FIXED_CASE
-      default:
-        break;
-    }
-  }
   if constexpr (TUNABLE) {
     if (sh && sh->wide) return go(psb::zpass_kernel<T, Phys, true>);
   }
@@ -482,7 +513,7 @@ int launch_epi(psb_ctx* c, psb::XEpiArgs<T> e, Epi epi, const char* what, const 
   const size_t esz = sizeof(Cx<T>);
   const int L = e.plan.L;
   e.col_tile = pick_ct(e.kz, Epi::F_IN, L, esz, e.n2);
-  if (sh && sh->tile) {
+  if (sh && sh->tile && !sh->reg) {
     e.col_tile = sh->tile;
     e.plan = sh->plan;
   }

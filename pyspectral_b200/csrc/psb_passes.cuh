@@ -450,14 +450,10 @@ __host__ inline size_t zpass_smem_bytes(int fmax, int P, int M, size_t extra) {
   return (size_t)(M + 2 * (size_t)((fmax * P + 1) / 2) * zline(M)) * sizeof(Cx<T>) + extra;
 }
 
-// Transform of the z-pass's contiguous lines: the plan's schedule (FP = 0) or
-// the compiled-in schedule FP (which must equal the plan's).
-template <typename T, bool INV, bool WIDE, int FP>
+// Transform of the z-pass's contiguous lines.
+template <typename T, bool INV, bool WIDE>
 __device__ __forceinline__ Cx<T>* zfft(Cx<T>* a, Cx<T>* b, const FFTPlan& p, const Cx<T>* tw, int nlines) {
-  if constexpr (FP == 0)
-    return block_fft<T, INV, WIDE>(a, b, p, tw, nlines, zline(p.L), 1, nlines >= 8);
-  else
-    return FixedPlan<FP>::template run<T, INV>(a, b, tw, nlines, zline(p.L));
+  return block_fft<T, INV, WIDE>(a, b, p, tw, nlines, zline(p.L), 1, nlines >= 8);
 }
 
 // Per-CTA staging of the z-pass: the twiddle table and the Phys extra (the
@@ -523,7 +519,7 @@ __device__ __forceinline__ void zpass_physics(const ZArgs<T>& a, const Phys& phy
 // One tile of the z-pass: pencils bx*ppc ..; smem = zpass_smem_bytes, staged
 // by zpass_setup.  Ends with the results stored; the caller synchronises
 // before the CTA's next tile reuses the buffers.
-template <typename T, class Phys, bool WIDE = false, int FP = 0>
+template <typename T, class Phys, bool WIDE = false>
 __device__ __forceinline__ void zpass_tile(const ZArgs<T>& a, const Phys& phys, int bx) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   Cx<T>* tw = reinterpret_cast<Cx<T>*>(smem_raw);
@@ -637,14 +633,14 @@ __device__ __forceinline__ void zpass_tile(const ZArgs<T>& a, const Phys& phys, 
       }
     }
     __syncthreads();
-    R = zfft<T, true, WIDE, FP>(X, Y, a.plan, tw, nin);
+    R = zfft<T, true, WIDE>(X, Y, a.plan, tw, nin);
   }
   Cx<T>* W = (R == X) ? Y : X;
   const int nout = (FO * P + 1) / 2;
   zpass_physics<T, Phys>(a, phys, R, W, P, M, LS, p0, extra);
   if constexpr (FO > 0) {
     __syncthreads();
-    Cx<T>* R2 = zfft<T, false, WIDE, FP>(W, R, a.plan, tw, nout);
+    Cx<T>* R2 = zfft<T, false, WIDE>(W, R, a.plan, tw, nout);
     // unpack: A_k = (Z_k + conj(Z_{M-k}))/2, B_k = (Z_k - conj(Z_{M-k}))/(2i)
     const int kzo = a.out_kz;
     if ((P & 1) == 0) {
@@ -685,189 +681,25 @@ __device__ __forceinline__ void zpass_tile(const ZArgs<T>& a, const Phys& phys, 
 }
 
 // One CTA, one tile (the batched kernel's unit).
-template <typename T, class Phys, bool WIDE = false, int FP = 0>
+template <typename T, class Phys, bool WIDE = false>
 __device__ __forceinline__ void zpass_body(const ZArgs<T>& a, const Phys& phys, int bx) {
   pdl_trigger();
   zpass_setup<T, Phys>(a, phys);
   pdl_wait();
-  zpass_tile<T, Phys, WIDE, FP>(a, phys, bx);
+  zpass_tile<T, Phys, WIDE>(a, phys, bx);
 }
 
 // Tiles bx = blockIdx.x, + gridDim.x, ... < ceil(npencils/ppc): any grid
 // size covers every tile; a grid of (resident CTAs per SM) x SMs stages the
 // twiddles and the Phys extra once per CTA instead of once per tile.
-// FP: compiled-in transform schedule (FixedPlan id) equal to a.plan, or 0.
-template <typename T, class Phys, bool WIDE = false, int FP = 0>
+template <typename T, class Phys, bool WIDE = false>
 __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 1) zpass_kernel(ZArgs<T> a, Phys phys) {
   pdl_trigger();
   zpass_setup<T, Phys>(a, phys);
   pdl_wait();
   const long long ntiles = (a.npencils + a.ppc - 1) / a.ppc;
   for (long long bx = blockIdx.x; bx < ntiles; bx += gridDim.x) {
-    zpass_tile<T, Phys, WIDE, FP>(a, phys, (int)bx);
-    __syncthreads();
-  }
-}
-
-// ---------------------------------------------------------------------------
-// z-pass with global memory on both sides of its transforms.  For a compiled
-// two-pass schedule (R1, R2) with R2 = 16 or 8 the inverse runs (R1, R2) and
-// the forward (R2, R1), so that both transforms' global-facing passes have R2
-// items per packed line, one per lane of an aligned R2-lane group:
-//  * inverse pass 1 loads its R1 elements of a packed line, positions
-//    j + R2 r, straight from the two pencils' stored spectra (Hermitian
-//    packing Z = A + iB, z derivatives i k3 u formed on load): the lanes of a
-//    group read R2 consecutive k3 of each pencil;
-//  * forward pass 2 hands its R1 results, positions j + R2 r, straight to the
-//    unpack A_q = (Z_q + conj Z_{M-q})/2, B_q = (Z_q - conj Z_{M-q})/(2i).
-//    For q = j + R2 r (j > 0), M - q = (R2 - j) + R2 (R1 - 1 - r): register
-//    R1 - 1 - r of lane R2 - j of the same group, fetched with a warp shuffle
-//    (lane 0 pairs with itself: M - R2 r is its register (R1 - r) mod R1).
-// A packed line's shared-memory traffic is the exchange inside each transform
-// and the physics' reads and writes; the packed spectra never pass through
-// shared memory.  P must be even (packed lines pair pencils p, p+1 of one
-// field).  smem and staging as zpass_kernel (zpass_smem_bytes, zpass_setup).
-template <int FP>
-struct zrr_plan {
-  using Pl = FixedPlan<FP>;
-  static constexpr int R1 = Pl::Radices::A, R2 = Pl::Radices::B, REV = fixed_plan_reversed(FP);
-  static constexpr bool value = Pl::Radices::NP == 2 && REV != 0 && (R2 == 16 || R2 == 8);
-};
-
-// The default schedule of a register-direct z pass of length p.L: the
-// compiled two-pass order (p.L / 16, 16) when there is one (48, 96, 192).
-__host__ inline bool zrr_default_plan(FFTPlan& p) {
-  for (const FixedDesc& d : kFixedDescs)
-    if (d.L == p.L && d.n == 2 && d.r[1] == 16 && fixed_plan_reversed(d.id) != 0) {
-      p.npass = 2;
-      p.radix[0] = d.r[0];
-      p.radix[1] = d.r[1];
-      for (int s = 2; s < kMaxPasses; ++s) p.radix[s] = 0;
-      return true;
-    }
-  return false;
-}
-
-template <typename T, class Phys, int FP>
-__device__ __forceinline__ void zpass_rr_tile(const ZArgs<T>& a, const Phys& phys, int bx) {
-  static_assert(zrr_plan<FP>::value, "two-pass schedule (R1, 16 or 8) with its reverse compiled in");
-  constexpr int M = FixedPlan<FP>::L, R1 = zrr_plan<FP>::R1, R2 = zrr_plan<FP>::R2;
-  constexpr int FI = Phys::F_IN, FO = Phys::F_OUT;
-  static_assert(FI > 0 && FO > 0, "a z-pass with inputs and outputs");
-  constexpr int FMAX = FI > FO ? FI : FO;
-  constexpr int half = M / 2, LS = zline(M);
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  Cx<T>* tw = reinterpret_cast<Cx<T>*>(smem_raw);
-  const int P = a.ppc, hp = P >> 1;
-  const int nl = FMAX * hp;
-  Cx<T>* X = tw + M;
-  Cx<T>* Y = X + (size_t)nl * LS;
-  unsigned char* extra = reinterpret_cast<unsigned char*>(Y + (size_t)nl * LS);
-  const long long p0 = (long long)bx * P;
-  const Cx<T> zero = mk<T>(0, 0);
-  const int nin = FI * hp, nout = FO * hp;
-  const int gpc = blockDim.x / R2;  // line groups per CTA
-  const int j = threadIdx.x % R2, grp = threadIdx.x / R2;
-  // ---- inverse pass 1: packed spectra -> registers -> radix R1 -> X
-  for (int c = grp; c < nin; c += gpc) {
-    const int f = c / hp, p = 2 * (c - f * hp);
-    const long long pa = p0 + p;
-    const bool oka = pa < a.npencils, okb = pa + 1 < a.npencils;
-    const long long ps = a.in_pstride[f];
-    const Cx<T>* src = a.in[f] + (oka ? pa * ps : 0);
-    const int kz = min(a.in_kz[f], half + 1);
-    Cx<T> va[R1], vb[R1];
-#pragma unroll
-    for (int r = 0; r < R1; ++r) {
-      const int n = j + R2 * r;
-      const int m = n <= half ? n : M - n;
-      va[r] = (m < kz && oka) ? src[m] : zero;
-      vb[r] = (m < kz && okb) ? src[ps + m] : zero;
-    }
-    const bool dz = a.dz[f] != 0;
-    Cx<T> v[R1];
-#pragma unroll
-    for (int r = 0; r < R1; ++r) {
-      const int n = j + R2 * r;
-      const bool lo = n <= half;
-      const int m = lo ? n : M - n;
-      Cx<T> A = va[r], B = vb[r];
-      if (dz) {
-        const T kk = m < kz ? (T)a.k3[m] : (T)0;
-        A = mk<T>(-kk * A.y, kk * A.x);
-        B = mk<T>(-kk * B.y, kk * B.x);
-      }
-      if (lo)
-        v[r] = (n == 0 || n == half) ? mk<T>(A.x, B.x) : mk<T>(A.x - B.y, A.y + B.x);
-      else
-        v[r] = mk<T>(A.x + B.y, B.x - A.y);
-    }
-    small_dft<T, R1, true>(v);
-    Cx<T>* Z = X + (size_t)c * LS + j * R1;
-#pragma unroll
-    for (int r = 0; r < R1; ++r) Z[r] = v[r];
-  }
-  __syncthreads();
-  // ---- inverse pass 2 (X -> Y), the physics (Y -> X), forward pass 1 (X -> Y)
-  if (nin >= 8)
-    stockham_pass_c<T, R2, true, M, R1, true>(X, Y, tw, nin, LS);
-  else
-    stockham_pass_c<T, R2, true, M, R1, false>(X, Y, tw, nin, LS);
-  __syncthreads();
-  zpass_physics<T, Phys>(a, phys, Y, X, P, M, LS, p0, extra);
-  __syncthreads();
-  if (nout >= 8)
-    stockham_pass_c<T, R2, false, M, 1, true>(X, Y, tw, nout, LS);
-  else
-    stockham_pass_c<T, R2, false, M, 1, false>(X, Y, tw, nout, LS);
-  __syncthreads();
-  // ---- forward pass 2: Y -> radix R1 (sub-transform length R2) -> unpack -> global.
-  // Every lane of a warp runs every round (the shuffles need the whole warp);
-  // lanes past the last line compute on zeros and store nothing.
-  const int lane = threadIdx.x & 31;
-  const int partner = (lane & ~(R2 - 1)) | ((R2 - j) & (R2 - 1));
-  const int kzo = a.out_kz;
-  for (int cb = 0; cb < nout; cb += gpc) {
-    const int c = cb + grp;
-    const bool act = c < nout;
-    Cx<T> v[R1];
-#pragma unroll
-    for (int r = 0; r < R1; ++r) v[r] = act ? Y[(size_t)c * LS + j + R2 * r] : zero;
-    // twiddles W_M^{r j} (sub-transform length R2: the table's stride is 1)
-#pragma unroll
-    for (int r = 1; r < R1; ++r) v[r] = cmul(v[r], tw[r * j]);
-    small_dft<T, R1, false>(v);
-    const int g = act ? c / hp : 0, p = 2 * (c - g * hp);
-    const long long pa = p0 + p;
-    const bool oka = act && pa < a.npencils, okb = act && pa + 1 < a.npencils;
-    const long long ps = a.out_pstride[g];
-    Cx<T>* dst = a.out[g] + (oka ? pa * ps : 0);
-#pragma unroll
-    for (int r = 0; r <= R1 / 2; ++r) {
-      if (R2 * r >= kzo) break;  // uniform over the warp
-      Cx<T> pv;
-      pv.x = __shfl_sync(0xffffffffu, v[R1 - 1 - r].x, partner);
-      pv.y = __shfl_sync(0xffffffffu, v[R1 - 1 - r].y, partner);
-      const Cx<T> zk = v[r];
-      const Cx<T> zm = j == 0 ? v[(R1 - r) % R1] : pv;
-      const int q = j + R2 * r;
-      if (q < kzo) {
-        if (oka) dst[q] = mk<T>((T)0.5 * (zk.x + zm.x), (T)0.5 * (zk.y - zm.y));
-        if (okb) dst[ps + q] = mk<T>((T)0.5 * (zk.y + zm.y), (T)0.5 * (zm.x - zk.x));
-      }
-    }
-  }
-}
-
-// Persistent register-direct z-pass (tiles as zpass_kernel).
-template <typename T, class Phys, int FP>
-__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 1) zpass_rr_kernel(ZArgs<T> a, Phys phys) {
-  pdl_trigger();
-  zpass_setup<T, Phys>(a, phys);
-  pdl_wait();
-  const long long ntiles = (a.npencils + a.ppc - 1) / a.ppc;
-  for (long long bx = blockIdx.x; bx < ntiles; bx += gridDim.x) {
-    zpass_rr_tile<T, Phys, FP>(a, phys, (int)bx);
+    zpass_tile<T, Phys, WIDE>(a, phys, (int)bx);
     __syncthreads();
   }
 }
@@ -877,7 +709,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 1) zpass_rr_kernel(Z
 // CTA's consecutive items share a run); a CTA stages the twiddles and the
 // Phys extra (the network's weights) again only when its run changes.  Every
 // run of a batch has the same shape (npencils, ppc, plan).
-template <typename T, class Phys, bool RR, bool WIDE, int FP>
+template <typename T, class Phys, bool WIDE>
 __device__ __forceinline__ void zpass_batch_body(const ZArgs<T>* __restrict__ A, const Phys* __restrict__ phys,
                                                  int runs) {
   pdl_trigger();
@@ -892,33 +724,17 @@ __device__ __forceinline__ void zpass_batch_body(const ZArgs<T>* __restrict__ A,
       if (staged < 0) pdl_wait();
       staged = r;
     }
-    if constexpr (RR)
-      zpass_rr_tile<T, Phys, FP>(A[r], phys[r], bx);
-    else
-      zpass_tile<T, Phys, WIDE, FP>(A[r], phys[r], bx);
+    zpass_tile<T, Phys, WIDE>(A[r], phys[r], bx);
     __syncthreads();  // the next item (or the next run's staging) reuses the shared memory
   }
 }
 
-template <typename T, class Phys, int FP>
-__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 1)
-    zpass_rr_batch(const ZArgs<T>* __restrict__ A, const Phys* __restrict__ phys, int runs) {
-  zpass_batch_body<T, Phys, true, false, FP>(A, phys, runs);
-}
-
-template <typename T, class Phys, bool WIDE, int FP = 0>
+template <typename T, class Phys, bool WIDE>
 __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 1)
     zpass_batch(const ZArgs<T>* __restrict__ A, const Phys* __restrict__ phys, int runs) {
-  zpass_batch_body<T, Phys, false, WIDE, FP>(A, phys, runs);
+  zpass_batch_body<T, Phys, WIDE>(A, phys, runs);
 }
 
-// Closures whose z-pass is compiled with the fixed schedules (the 3/2-padded
-// Navier-Stokes closures: DNS products, Smagorinsky, learned); FP64 only with
-// the default schedule of each length.
-template <class Phys>
-struct phys_fixed_fft {
-  static constexpr bool value = false;
-};
 template <typename T, int FP>
 struct fixed_plan_compiled {
   static constexpr bool value = sizeof(T) == 4 || FP == 1 || FP == 4 || FP == 7;

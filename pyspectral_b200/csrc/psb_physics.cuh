@@ -895,20 +895,82 @@ struct PhysLearned {
       }
     }
   }
-};
-
-template <typename T>
-struct phys_fixed_fft<PhysProducts<T>> {
-  static constexpr bool value = true;
-};
-template <typename T>
-struct phys_fixed_fft<PhysSmag<T>> {
-  static constexpr bool value = true;
-};
-// (the GELU network keeps the runtime schedules: it is not the shipped model)
-template <typename T, int H>
-struct phys_fixed_fft<PhysLearned<T, kActRelu, H>> {
-  static constexpr bool value = true;
+  // The same computation on the register z pass's buffer (psb_zreg.cuh): slot f
+  // holds field f, pencil p's element (i, r) at f*ss + p*LS + i*BP + r, two
+  // consecutive real points per element.  Points are taken in storage order, 16
+  // per tile; the six results of a point go to slots 6..11 (its own last six
+  // gradients, read before the first MMA of the tile).  The inputs are physical
+  // already.
+  template <int A, int B, int BP, int LS>
+  __device__ __forceinline__ void points(T* __restrict__ X, int P, int ss, unsigned char* extra) const {
+    const MlpFwdSmem<H>& s = *reinterpret_cast<const MlpFwdSmem<H>*>(extra);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const int nw = blockDim.x >> 5;
+    const int fst = 2 * ss;
+    const T is2 = (T)1 / (sphys * sphys);
+    int foff[4];
+    float fm[4], fi[4], fc[4];
+    bool fg[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int f = 2 * t + 8 * (q >> 1) + (q & 1);
+      fg[q] = f < 9;
+      foff[q] = fg[q] ? (3 + f) * fst : 0;
+      fm[q] = f < kMlpIn ? s.xmean[f] : 0.f;
+      fi[q] = f < kMlpIn ? s.xistd[f] : 0.f;
+      fc[q] = f == 9 ? (delta - s.xmean[f]) * s.xistd[f] : 0.f;
+    }
+    int ooff[2], ioff[2], joff[2];
+    float ys[2], ym[2];
+#pragma unroll
+    for (int e2 = 0; e2 < 2; ++e2) {
+      const int c = 2 * t + e2;
+      const int ii = c < 3 ? c : (c == 5 ? 1 : 0);
+      const int jj = c < 3 ? c : (c == 3 ? 1 : 2);
+      ooff[e2] = (6 + c) * fst;
+      ioff[e2] = ii * fst;
+      joff[e2] = jj * fst;
+      ys[e2] = c < kMlpOut ? s.ystd[c] : 0.f;
+      ym[e2] = c < kMlpOut ? s.ymean[c] : 0.f;
+    }
+    const int npts = P * A * 2 * B;
+    for (int pt0 = warp * 16; pt0 < npts; pt0 += nw * 16) {
+      int b[2];
+      bool ok[2];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int pt = pt0 + g + 8 * h;
+        ok[h] = pt < npts;
+        const int blk = pt / (2 * B), off = pt - blk * (2 * B);
+        const int p = blk / A, i = blk - p * A;
+        b[h] = ok[h] ? 2 * (p * LS + i * BP) + off : 0;
+      }
+      float v[8];
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const float x = (float)(X[b[h] + foff[q]] * sphys);
+          v[h * 4 + q] = fg[q] ? (x - fm[q]) * fi[q] : fc[q];
+        }
+      uint32_t xa[4];
+      xa[0] = pack_bf16(v[0], v[1]);
+      xa[1] = pack_bf16(v[4], v[5]);
+      xa[2] = pack_bf16(v[2], v[3]);
+      xa[3] = pack_bf16(v[6], v[7]);
+      float y[4];
+      mlp_forward_fast<ACT, H>(s, xa, y);
+      if (t < 3) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int e2 = e & 1, h = e >> 1;
+          if (!ok[h]) continue;
+          const T tau = (T)(y[e] * ys[e2] + ym[e2]);
+          X[b[h] + ooff[e2]] = X[b[h] + ioff[e2]] * X[b[h] + joff[e2]] + tau * is2;
+        }
+      }
+    }
+  }
 };
 
 }  // namespace psb

@@ -1944,10 +1944,12 @@ struct TuneDims {
   bool regx = true, regy = true;  // the x- / y-inverse pass has a register form
   size_t zextra = 0;
   int Ls[5], Fs[5];
+  int zP = 0;  // the register z pass's pencils per CTA and plan (0: none at this length)
+  FFTPlan zplan{};
 };
 
 template <typename T>
-TuneDims tune_dims(psb_ctx* c, int closure) {
+TuneDims tune_dims(psb_ctx* c, int closure, int act, int hidden) {
   TuneDims t;
   if (closure == PSB_DNS) {
     t.Fi = t.Fb = t.Gy = 3, t.Fo = 6, t.maxppc = phys_max_ppc<PhysProducts<T>>::value;
@@ -1968,6 +1970,19 @@ TuneDims tune_dims(psb_ctx* c, int closure) {
     t.zextra = (size_t)phys_is_block<PhysLearned<T>>::extra;
   }
   const int M1 = 3 * c->N1 / 2, M2 = 3 * c->N2 / 2, M3 = 3 * c->N3 / 2;
+  const long long np = (long long)M1 * M2;
+  t.zplan = *plan_for(c, M3);
+  if (!c->use_zrr) {
+  } else if (closure == PSB_DNS) {
+    if (has_reg_z<T, PhysProducts<T>>(M3)) t.zP = reg_z_shape<T, PhysProducts<T>>(M3, np, t.zplan);
+  } else if (closure == PSB_SMAG) {
+    if (has_reg_z<T, PhysSmag<T>>(M3)) t.zP = reg_z_shape<T, PhysSmag<T>>(M3, np, t.zplan);
+  } else if (act == PSB_ACT_RELU) {
+    using Ph32 = PhysLearned<T, kActRelu, 32>;
+    using Ph64 = PhysLearned<T, kActRelu, 64>;
+    if (has_reg_z<T, Ph32>(M3))
+      t.zP = hidden == 32 ? reg_z_shape<T, Ph32>(M3, np, t.zplan) : reg_z_shape<T, Ph64>(M3, np, t.zplan);
+  }
   const int Ls[5] = {M1, M2, M3, M2, M1};
   const int Fs[5] = {t.Fi, t.Fy, 0, 1, t.Fo};
   for (int k = 0; k < 5; ++k) {
@@ -1990,13 +2005,14 @@ void default_pass_shape(psb_ctx* c, const TuneDims& t, int k, psb_pass_shape& sh
   const int nouter = k == 0 || k == 4 ? c->N2 : (k == 1 ? t.Gy * t.Ls[0] : t.Fo * t.Ls[0]);
   const bool reg = k == 0 ? t.regx : (k == 1 ? t.regy : k == 3);
   default_axis_shape<T>(c, t.Ls[k], c->N3 / 2, t.Fs[k], nouter, reg, sh.tile, sh.plan);
+  sh.reg = reg && has_reg_axis(t.Ls[k]);
 }
 
 template <typename T>
 int tune_rhs(psb_ctx* c, int closure, const void* state, const psb_params* p) {
   const int N1 = c->N1, N2 = c->N2, N3 = c->N3, N3h = c->N3h;
   const int M1 = 3 * N1 / 2, M2 = 3 * N2 / 2, M3 = 3 * N3 / 2, Kz = N3 / 2;
-  const TuneDims td = tune_dims<T>(c, closure);
+  const TuneDims td = tune_dims<T>(c, closure, p->mlp_act, p->mlp_hidden);
   const int Fz = td.Fz, Fo = td.Fo, maxppc = td.maxppc, defppc = td.defppc;
   const size_t zextra = td.zextra;
   const size_t esz = sizeof(Cx<T>);
@@ -2019,8 +2035,9 @@ int tune_rhs(psb_ctx* c, int closure, const void* state, const psb_params* p) {
   const int* Ls = td.Ls;
   const int* Fs = td.Fs;
   for (int k : {0, 1, 3, 4}) default_pass_shape<T>(c, td, k, t.pass[k]);
-  t.pass[2].tile = P;
-  t.pass[2].plan = *plan_for(c, M3);
+  t.pass[2].tile = td.zP ? td.zP : P;
+  t.pass[2].plan = td.zplan;
+  t.pass[2].reg = td.zP > 0;
   c->tuned[closure] = t;
   static const char* names[5] = {"x-inverse", "y-inverse", "z-fused", "y-forward", "x-forward+epilogue"};
   const int timing_was = c->timing;
@@ -2049,7 +2066,7 @@ int tune_rhs(psb_ctx* c, int closure, const void* state, const psb_params* p) {
     psb_pass_shape& cur = c->tuned[closure].pass[k];
     const psb_pass_shape inc = cur;
     // a register pass has one shape (the runtime-schedule shapes of its length are slower throughout)
-    if (k != 2 && is_reg_axis(inc.plan)) continue;
+    if (k == 2 ? td.zP > 0 : is_reg_axis(inc.plan)) continue;
     float base = 0.f;
     if ((status = time_pass(k, 6, &base)) != PSB_OK) break;
     std::vector<int> tiles;
@@ -2099,7 +2116,7 @@ int tune_rhs(psb_ctx* c, int closure, const void* state, const psb_params* p) {
 // transform length, the radices the kernels have and the shared-memory budget.
 template <typename T>
 int set_shape(psb_ctx* c, int closure, int k, int tile, const int* radices, int nrad) {
-  const TuneDims td = tune_dims<T>(c, closure);
+  const TuneDims td = tune_dims<T>(c, closure, PSB_ACT_RELU, 32);
   const int L = td.Ls[k];
   if (nrad < 1 || nrad > kMaxPasses) return fail(c, PSB_ERR_ARG, "psb_set_tuned_shape: 1..12 radices");
   long long prod = 1;
@@ -2108,8 +2125,11 @@ int set_shape(psb_ctx* c, int closure, int k, int tile, const int* radices, int 
   q.npass = nrad;
   // the register pass's own radices name it (its tile is fixed)
   FFTPlan rp = q;
-  const bool reg_shape = (k == 0 ? td.regx : (k == 1 ? td.regy : k == 3)) && nrad == 2 && reg_axis_plan(L, rp) &&
-                         radices[0] == rp.radix[0] && radices[1] == rp.radix[1];
+  bool reg_shape = (k == 0 ? td.regx : (k == 1 ? td.regy : k == 3)) && nrad == 2 && reg_axis_plan(L, rp) &&
+                   radices[0] == rp.radix[0] && radices[1] == rp.radix[1];
+  if (k == 2)
+    reg_shape = td.zP > 0 && nrad == 3 && std::equal(radices, radices + 3, td.zplan.radix) && tile >= 1 &&
+                tile <= 128;
   for (int s = 0; s < nrad; ++s) {
     const int r = radices[s];
     if (reg_shape) {
@@ -2128,7 +2148,7 @@ int set_shape(psb_ctx* c, int closure, int k, int tile, const int* radices, int 
     return fail(c, PSB_ERR_SHAPE, "psb_set_tuned_shape: the radices multiply to " + std::to_string(prod) +
                                       ", the pass transforms " + std::to_string(L) + " points");
   const int tmax = k == 2 ? td.maxppc : 32;
-  if (tile < 1 || tile > tmax || (tile & (tile - 1)))
+  if (!(k == 2 && reg_shape) && (tile < 1 || tile > tmax || (tile & (tile - 1))))
     return fail(c, PSB_ERR_ARG, "psb_set_tuned_shape: tile must be a power of two <= " + std::to_string(tmax));
   if (!reg_shape && pass_smem<T>(td, k, tile) > kSmemBudget)
     return fail(c, PSB_ERR_SHAPE, "psb_set_tuned_shape: tile needs more shared memory than the budget");
@@ -2140,14 +2160,16 @@ int set_shape(psb_ctx* c, int closure, int k, int tile, const int* radices, int 
     while (P > 1 && pass_smem<T>(td, 2, P) > kSmemBudget) P /= 2;
     while (P > 1 && ((long long)td.Ls[0] * td.Ls[1] + P - 1) / P < 2 * 148) P /= 2;
     for (int j : {0, 1, 3, 4}) default_pass_shape<T>(c, td, j, t.pass[j]);
-    t.pass[2].tile = P;
-    t.pass[2].plan = *plan_for(c, td.Ls[2]);
+    t.pass[2].tile = td.zP ? td.zP : P;
+    t.pass[2].plan = td.zplan;
+  t.pass[2].reg = td.zP > 0;
     it = c->tuned.emplace(closure, t).first;
   }
   psb_pass_shape& sh = it->second.pass[k];
   sh.tile = tile;
   sh.plan = q;
   sh.wide = wide;
+  sh.reg = reg_shape;
   return PSB_OK;
 }
 

@@ -1,0 +1,8 @@
+// Register z pass, float fields: products and the learned stress, width-64 network.
+#include "psb_z.cuh"
+
+namespace psbh {
+using namespace psb;
+PSB_REG_Z(float, PhysLearned<float, kActRelu, 64>)
+PSB_REG_Z_BATCH(float, PhysLearned<float, kActRelu, 64>)
+}  // namespace psbh
