@@ -146,6 +146,12 @@ struct Batch {
     }
     return false;
   }
+  // The same for the x-forward pass.
+  void generic_x(int& tile, FFTPlan& plan) const {
+    tile = b->tile[4];
+    plan = b->plan[4];
+    if (is_reg_x(plan)) default_x_shape<T>(c, plan.L, d.Kz, Fo, d.N2, false, tile, plan);
+  }
   // Pencils per CTA and plan of the staged z pass: the pass's own shape, or the default
   // where the register pass runs (the persistent ensemble runs the staged one).
   void generic_z(int& P, FFTPlan& plan) const {
@@ -263,10 +269,9 @@ struct Batch {
       e.n2 = d.N2;
       e.n3h = d.N3h;
       e.kz = d.Kz;
-      e.col_tile = b->tile[4];
+      generic_x(e.col_tile, e.plan);
       e.out_map = map_pad32(d.N1);
       e.main_blocks = ((d.Kz + e.col_tile - 1) / e.col_tile) * d.N2;
-      e.plan = b->plan[4];
       e.tw = twiddles<T>(c);
       ae[r] = e;
       pre[r] = pre0;
@@ -330,22 +335,6 @@ struct Batch {
     for (int s = 0; s < p.npass; ++s)
       if (p.radix[s] > 8 || p.radix[s] == 6) return true;
     return false;
-  }
-  // fix(integral_constant<int, ID>) when the pass's plan is a compiled-in
-  // schedule ID (for this precision), else def().
-  template <class Fix, class Def>
-  int by_plan(int pass, Fix fix, Def def) {
-    switch (fixed_plan_id(b->plan[pass])) {
-#define PSB_FIXED_CASE(ID, ...)                                                             \
-  case ID:                                                                                  \
-    if constexpr (fixed_plan_compiled<T, ID>::value) return fix(std::integral_constant<int, ID>{}); \
-    break;
-      PSB_FIXED_PLANS(PSB_FIXED_CASE)
-#undef PSB_FIXED_CASE
-      default:
-        break;
-    }
-    return def();
   }
   template <bool W>
   int launch_w(int pass, int stage) {
@@ -420,24 +409,25 @@ struct Batch {
         return go(zpass_batch<T, Phys, W>);
       }
       default: {
+        const long long pts = (long long)d.N1 * d.N2 * (d.N3h - d.Kz);
+        const int extra = (int)std::min<long long>((pts + 255) / 256, 1024);
+        const double by = (double)R * (esz * Fo * d.M1 * d.N2 * d.Kz + esz * 3.0 * d.N1 * d.N2 * d.N3h *
+                                                                           3.0);
+        if (is_reg_x(b->plan[4]))
+          return reg_x_batch<T, Epi>(c, ae, epi + (size_t)stage * R, d.M1, d.Kz, d.N1, d.N2, d.N3h, R,
+                                     "batch x-forward+epilogue", by);
         const int ct = b->tile[4];
         const int ntile = (d.Kz + ct - 1) / ct;
         const int mainb = ntile * d.N2;
-        const long long pts = (long long)d.N1 * d.N2 * (d.N3h - d.Kz);
-        const int extra = (int)std::min<long long>((pts + 255) / 256, 1024);
         dim3 g(mainb + extra, R);
         const size_t sm = smem_axis(d.M1, Fo, ct);
-        const double by = (double)R * (esz * Fo * d.M1 * d.N2 * d.Kz + esz * 3.0 * d.N1 * d.N2 * d.N3h *
-                                                                           3.0);
         auto go = [&](auto k) {
           set_smem(k, sm);
           LaunchScope s(c, "batch x-forward+epilogue", by);
           launch_pdl(k, g, 256, sm, c->stream, (const XEpiArgs<T>*)ae, (const Epi*)(epi + (size_t)stage * R));
           return launch_ok(c, "batch x-forward+epilogue");
         };
-        return by_plan(
-            4, [&](auto id) { return go(xfwd_epi_batch<T, Epi, false, decltype(id)::value>); },
-            [&] { return go(xfwd_epi_batch<T, Epi, W>); });
+        return go(xfwd_epi_batch<T, Epi, W>);
       }
     }
   }
@@ -481,7 +471,9 @@ struct Batch {
     for (int pass = 0; pass < 5; ++pass) PSB_TRY(launch(pass, 4));
     for (int pass = 0; pass < 5; ++pass) {
       // a register pass has one shape (the runtime-schedule shapes of its length are slower throughout)
-      if (pass == 2 ? reg_z_pass() : reg_pass(pass) && is_reg_axis(b->plan[pass])) continue;
+      if (pass == 2 ? reg_z_pass()
+                    : (pass == 4 ? is_reg_x(b->plan[4]) : reg_pass(pass) && is_reg_axis(b->plan[pass])))
+        continue;
       std::vector<int> tiles;
       if (pass == 2) {
         for (int P : {1, 2, 4, 8})
@@ -552,10 +544,14 @@ PhysLearned<T, ACT, H> mk_learned(psb_ctx* c, const psb_params& p) {
                                 reinterpret_cast<const float*>(p.mlp_norm), (T)s32,
                                 (float)(p.les_delta > 0 ? p.les_delta : c->Delta)};
 }
-template <typename T, bool SMAG>
-EpiNS<T, SMAG> mk_epi(psb_ctx* c, StepIO<T> io, const psb_params& p) {
-  return EpiNS<T, SMAG>{io, ktab<T>(c->kx, c->ky, c->kz), (T)p.nu, p.rotate, (T)p.Om1, (T)p.Om2, (T)p.Om3,
-                        SMAG ? 0 : 1, c->N1 / 2, c->N2 / 2, c->N3 / 2};
+template <typename T>
+EpiNS<T, false> mk_epi(psb_ctx* c, StepIO<T> io, const psb_params& p) {
+  return EpiNS<T, false>{io, ktab<T>(c->kx, c->ky, c->kz), (T)p.nu, p.rotate, (T)p.Om1, (T)p.Om2, (T)p.Om3,
+                         1, c->N1 / 2, c->N2 / 2, c->N3 / 2};
+}
+template <typename T>
+EpiSmagStep<T> mk_epi_smag(psb_ctx* c, StepIO<T> io, const psb_params& p) {
+  return EpiSmagStep<T>{io, ktab<T>(c->kx, c->ky, c->kz), (T)p.nu, p.rotate, (T)p.Om1, (T)p.Om2, (T)p.Om3};
 }
 
 // Default launch shapes: the single-run rules of the library.
@@ -571,7 +567,7 @@ void default_shapes(psb_batch* b, int Fi, int Fb, int Fz, int Fo, int Fy, int Gy
   default_axis_shape<T>(c, d.M1, d.Kz, Fi, d.N2, reg(0), b->tile[0], b->plan[0]);
   default_axis_shape<T>(c, d.M2, d.Kz, Fy, Gy * d.M1, reg(1), b->tile[1], b->plan[1]);
   default_axis_shape<T>(c, d.M2, d.Kz, 1, Fo * d.M1, reg(3), b->tile[3], b->plan[3]);
-  b->tile[4] = pick_ct(d.Kz, Fo, d.M1, esz, d.N2);
+  default_x_shape<T>(c, d.M1, d.Kz, Fo, d.N2, true, b->tile[4], b->plan[4]);
   const int FMAX = std::max(Fz, Fo);
   int P = ppc;
   auto sm = [&](int P) { return (size_t)(d.M3 + 2 * (size_t)((FMAX * P + 1) / 2) * d.M3) * esz + zextra; };
@@ -581,7 +577,6 @@ void default_shapes(psb_batch* b, int Fi, int Fb, int Fz, int Fo, int Fy, int Gy
   while (P > 1 && (np + P - 1) / P * b->nruns < 2 * 148) P /= 2;
   b->tile[2] = P;
   b->plan[2] = *plan_for(c, d.M3);
-  b->plan[4] = *plan_for(c, d.M1);
 }
 
 template <typename T, class Pre, class Phys, class Epi>
@@ -623,16 +618,16 @@ template <typename T>
 int dispatch(psb_batch* b, int nsteps, bool tune) {
   switch (b->closure) {
     case PSB_DNS:
-      return run_batch<T>(b, nsteps, tune, PreCopyN<T, 3>{}, &mk_products<T>, &mk_epi<T, false>);
+      return run_batch<T>(b, nsteps, tune, PreCopyN<T, 3>{}, &mk_products<T>, &mk_epi<T>);
     case PSB_SMAG:
-      return run_batch<T>(b, nsteps, tune, PreStrain<T>{}, &mk_smag<T>, &mk_epi<T, true>);
+      return run_batch<T>(b, nsteps, tune, PreStrain<T>{}, &mk_smag<T>, &mk_epi_smag<T>);
     case PSB_LEARNED:
       // every run of a learned batch has the activation and width of run 0 (psb_batch_set_run)
       if (b->params[0].mlp_act == PSB_ACT_GELU)
-        return run_batch<T>(b, nsteps, tune, PreGradXY<T>{}, &mk_learned<T, kActGelu, 64>, &mk_epi<T, false>);
+        return run_batch<T>(b, nsteps, tune, PreGradXY<T>{}, &mk_learned<T, kActGelu, 64>, &mk_epi<T>);
       if (b->params[0].mlp_hidden == 32)
-        return run_batch<T>(b, nsteps, tune, PreGradXY<T>{}, &mk_learned<T, kActRelu, 32>, &mk_epi<T, false>);
-      return run_batch<T>(b, nsteps, tune, PreGradXY<T>{}, &mk_learned<T, kActRelu, 64>, &mk_epi<T, false>);
+        return run_batch<T>(b, nsteps, tune, PreGradXY<T>{}, &mk_learned<T, kActRelu, 32>, &mk_epi<T>);
+      return run_batch<T>(b, nsteps, tune, PreGradXY<T>{}, &mk_learned<T, kActRelu, 64>, &mk_epi<T>);
     default:
       return fail(b->c, PSB_ERR_UNSUPPORTED, "psb_batch: closure not batched (DNS, SMAG, LEARNED are)");
   }
@@ -725,7 +720,7 @@ __global__ void __launch_bounds__(256, 2) ens_persistent_kernel(const EnsDesc* _
               ens_item<T, PreCopyN<T, 3>, PhysProducts<T>, EpiNS<T, false>>(g, q, pass, stage, i, staged);
               break;
             case kEnsSmag:
-              ens_item<T, PreStrain<T>, PhysSmag<T>, EpiNS<T, true>>(g, q, pass, stage, i, staged);
+              ens_item<T, PreStrain<T>, PhysSmag<T>, EpiSmagStep<T>>(g, q, pass, stage, i, staged);
               break;
             default:
               ens_item<T, PreGradXY<T>, PhysLearned<T, kActRelu, 32>, EpiNS<T, false>>(g, q, pass, stage, i, staged);
@@ -769,6 +764,7 @@ size_t ens_group(psb_batch* b, int kind, EnsGroup& g) {
   {
     FFTPlan plan;
     x.generic_z(t[2], plan);
+    x.generic_x(t[4], plan);
   }
   g.nx[0] = (d.Kz + t[0] - 1) / t[0];
   g.ny[0] = d.N2;
@@ -935,7 +931,7 @@ static int ens_step(psb_ensemble* e, int nsteps, unsigned limit) {
     if (b->closure == PSB_DNS)
       smem = std::max(smem, ens_group<T, PreCopyN<T, 3>, PhysProducts<T>, EpiNS<T, false>>(b, kEnsDns, h.g[i]));
     else if (b->closure == PSB_SMAG)
-      smem = std::max(smem, ens_group<T, PreStrain<T>, PhysSmag<T>, EpiNS<T, true>>(b, kEnsSmag, h.g[i]));
+      smem = std::max(smem, ens_group<T, PreStrain<T>, PhysSmag<T>, EpiSmagStep<T>>(b, kEnsSmag, h.g[i]));
     else
       smem = std::max(smem, ens_group<T, PreGradXY<T>, PhysLearned<T, kActRelu, 32>, EpiNS<T, false>>(
                                 b, kEnsLearnedR32, h.g[i]));

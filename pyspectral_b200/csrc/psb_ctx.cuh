@@ -15,6 +15,7 @@
 #include "../../include/pyspectral_b200.h"
 #include "psb_physics.cuh"
 #include "psb_reg.cuh"
+#include "psb_xreg.cuh"
 #include "psb_zreg.cuh"
 
 // Launch shape of one pass picked by the autotuner: tile (columns per CTA, or
@@ -67,6 +68,7 @@ struct psb_ctx {
   unsigned long long launches = 0;
   int timing = 0;
   int use_tma = 1;          // stage eligible pass inputs with bulk tensor copies
+  bool serial_next = false; // the next launch follows a z pass that ran alone (launch_after_z)
   int use_zrr = 1;          // register z pass where the length has one (0: the staged one)
   int* dstatus = nullptr;   // device status word (a bounded wait gave up), owned
   struct Rec {
@@ -179,19 +181,19 @@ inline int count_mapped(const psb::RowMap& m, int rows) {
 
 constexpr size_t kSmemBudget = 100 * 1024;
 
-// Raise a kernel's dynamic shared-memory limit once per (kernel, device); a
-// fixed table, so that launching never allocates host memory either.  The
-// table is process-wide and shared by every context, so it is guarded by a
-// mutex: host threads that launch on different contexts may meet here.
-struct SmemCache {
-  const void* fn[512];
-  int dev[512];
-  size_t bytes[512];
-  int n = 0;
+// Raise a kernel's dynamic shared-memory limit once per (kernel, device).  A
+// fixed open-addressing table, so that launching never allocates host memory
+// either; process-wide, shared by every context and guarded by a mutex (host
+// threads launch on different contexts).
+struct KernelAttrs {
+  static constexpr int kCap = 4096;
+  const void* fn[kCap] = {};
+  int dev[kCap] = {};
+  size_t bytes[kCap] = {};
   std::mutex mu;
 };
-inline SmemCache& smem_cache() {
-  static SmemCache c;
+inline KernelAttrs& kernel_attrs() {
+  static KernelAttrs c;
   return c;
 }
 template <typename K>
@@ -199,32 +201,35 @@ inline void set_smem(K kernel, size_t smem) {
   if (smem <= 48 * 1024) return;
   int dev = 0;
   cudaGetDevice(&dev);
-  SmemCache& c = smem_cache();
+  KernelAttrs& c = kernel_attrs();
   const void* f = reinterpret_cast<const void*>(kernel);
+  const size_t key = (reinterpret_cast<size_t>(f) >> 4) * 31 + (size_t)dev;
   std::lock_guard<std::mutex> lk(c.mu);
-  for (int i = 0; i < c.n; ++i)
+  for (int p = 0; p < 64; ++p) {
+    const int i = (int)((key + p) % KernelAttrs::kCap);
     if (c.fn[i] == f && c.dev[i] == dev) {
       if (c.bytes[i] >= smem) return;
-      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      c.bytes[i] = smem;
-      return;
+    } else if (c.fn[i] != nullptr) {
+      continue;
     }
-  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (c.n < 512) {
-    c.fn[c.n] = f;
-    c.dev[c.n] = dev;
-    c.bytes[c.n] = smem;
-    ++c.n;
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    c.fn[i] = f;
+    c.dev[i] = dev;
+    c.bytes[i] = smem;
+    return;
   }
+  // no free slot near: set every time
+  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
 }
 
 // Launch of a pipeline kernel (axis, z and x-forward passes) with
 // programmatic stream serialisation: it may start while the previous kernel
 // in the stream drains; the kernels wait for their predecessor (pdl_wait)
 // before touching pipeline data.
+// pdl = false: an ordinary launch, after the previous kernel has ended.
 template <typename... KArgs, typename... Args>
-inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, int block, size_t smem, cudaStream_t stream,
-                              Args... args) {
+inline cudaError_t launch_pdl_if(bool pdl, void (*kernel)(KArgs...), dim3 grid, int block, size_t smem,
+                                 cudaStream_t stream, Args... args) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid;
   cfg.blockDim = dim3((unsigned)block);
@@ -232,10 +237,15 @@ inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, int block, si
   cfg.stream = stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[0].val.programmaticStreamSerializationAllowed = pdl ? 1 : 0;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, int block, size_t smem, cudaStream_t stream,
+                              Args... args) {
+  return launch_pdl_if(true, kernel, grid, block, smem, stream, args...);
 }
 
 // Grid of a persistent kernel: at most (resident CTAs per SM) x SMs of the
@@ -246,10 +256,11 @@ inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, int block, si
 // (kernel, device, shared memory) in a fixed table under a mutex (host threads
 // of several contexts launch).
 struct OccCache {
-  const void* fn[256];
-  int dev[256];
-  size_t smem[256];
-  int per[256], nsm[256];
+  static constexpr int kCap = 1024;
+  const void* fn[kCap];
+  int dev[kCap];
+  size_t smem[kCap];
+  int per[kCap], nsm[kCap];
   int n = 0;
   std::mutex mu;
 };
@@ -274,7 +285,7 @@ inline long long persistent_grid(K kernel, size_t smem, long long ntiles, int bl
     (void)cudaGetLastError();
     return ntiles;
   }
-  if (oc.n < 256) {
+  if (oc.n < OccCache::kCap) {
     oc.fn[oc.n] = f;
     oc.dev[oc.n] = dev;
     oc.smem[oc.n] = smem;
@@ -284,6 +295,16 @@ inline long long persistent_grid(K kernel, size_t smem, long long ntiles, int bl
   }
   return std::min<long long>(ntiles, (long long)per * nsm);
 }
+
+// Programmatic dependent launch into and out of the register z pass.  The z pass
+// takes the largest shared-memory carveout, the axis and x passes a large L1 (their
+// loads in flight land there: with the z pass's carveout t-model's 2x y-forward pass
+// goes from 300 to 410 us), and an SM changes its split only when it is empty.  CTAs
+// that arrive early on an SM of the other kind therefore run with too little of what
+// they need: t-model 128^3 FP64 13.3 ms a step with the overlap, 10.9 without; DNS
+// 256^3 FP32 10.2 against 9.2.  Passes whose data stay in L2 are short and gain from
+// it (32^3 FP64 159 -> 135 us a step, 64^3 Smagorinsky FP64 582 -> 565).
+constexpr double kPdlBytes = 126e6;
 
 inline int pow2_floor(int x) {
   int p = 1;
@@ -401,12 +422,62 @@ int reg_z_batch(psb_ctx* c, const psb::ZArgs<T>* args, const Phys* phys, int M, 
 template <typename T, class Phys>
 int reg_z_shape(int M, long long npencils, FFTPlan& plan);
 
+// ---- register x pass (psb_xreg.cuh; launched by the psb_x_*.cu files) ----
+template <class Epi, class = void>
+struct x_registered {
+  static constexpr bool value = false;
+};
+template <class Epi>
+struct x_registered<Epi, decltype((void)Epi::NACC, void())> {
+  static constexpr bool value = true;
+};
+inline bool reg_x_plan(int L, FFTPlan& p) {
+#define PSB_CASE(LEN, A, B, R)           \
+  case LEN: {                            \
+    const int r[3] = {A, B, R};          \
+    p.npass = 0;                         \
+    for (int v : r)                      \
+      if (v > 1) p.radix[p.npass++] = v; \
+    break;                               \
+  }
+  switch (L) {
+    PSB_REG_X(PSB_CASE)
+    default:
+      return false;
+  }
+#undef PSB_CASE
+  for (int s = p.npass; s < psb::kMaxPasses; ++s) p.radix[s] = 0;
+  return true;
+}
+inline bool has_reg_x(int L) {
+  FFTPlan p{};
+  return reg_x_plan(L, p);
+}
+inline bool is_reg_x(const FFTPlan& p) {
+  FFTPlan q{};
+  return reg_x_plan(p.L, q) && p.npass == q.npass && std::equal(q.radix, q.radix + q.npass, p.radix);
+}
+template <typename T, class Epi>
+int reg_x(psb_ctx* c, const psb::XEpiArgs<T>& e, const Epi& epi, const char* what, double bytes);
+template <typename T, class Epi>
+int reg_x_batch(psb_ctx* c, const psb::XEpiArgs<T>* args, const Epi* epi, int L, int kz, int n1, int n2, int n3h,
+                int runs, const char* what, double bytes);
+
 // Launch shape (tile and radices) of an axis pass that no tuner has touched.
 template <typename T>
 inline void default_axis_shape(psb_ctx* c, int L, int ncols, int F, int nouter, bool reg, int& tile, FFTPlan& plan) {
   plan = *plan_for(c, L);
   if (reg && reg_axis_plan(L, plan))
     tile = psb::reg_cols<T>();
+  else
+    tile = pick_ct(ncols, F, L, sizeof(Cx<T>), nouter);
+}
+
+template <typename T>
+inline void default_x_shape(psb_ctx* c, int L, int ncols, int F, int nouter, bool reg, int& tile, FFTPlan& plan) {
+  plan = *plan_for(c, L);
+  if (reg && reg_x_plan(L, plan))
+    tile = psb::xreg_cols<T>();
   else
     tile = pick_ct(ncols, F, L, sizeof(Cx<T>), nouter);
 }
@@ -512,6 +583,16 @@ template <typename T, class Epi, bool TUNABLE = false>
 int launch_epi(psb_ctx* c, psb::XEpiArgs<T> e, Epi epi, const char* what, const psb_pass_shape* sh = nullptr) {
   const size_t esz = sizeof(Cx<T>);
   const int L = e.plan.L;
+  const double bytes = epi.io_bytes((long long)e.n1 * e.n2 * e.n3h) + (double)esz * Epi::F_IN * L * e.n2 * e.kz;
+  // the register pass of this length (psb_xreg.cuh), where there is one; a tuned shape applies to
+  // the staged ones of the other lengths
+  if constexpr (x_registered<Epi>::value)
+    if (has_reg_x(L)) return reg_x<T, Epi>(c, e, epi, what, bytes);
+  int extra = 0;
+  if (e.n3h > e.kz) {
+    const long long pts = (long long)e.n1 * e.n2 * (e.n3h - e.kz);
+    extra = (int)std::min<long long>((pts + 255) / 256, 1024);
+  }
   e.col_tile = pick_ct(e.kz, Epi::F_IN, L, esz, e.n2);
   if (sh && sh->tile && !sh->reg) {
     e.col_tile = sh->tile;
@@ -519,33 +600,13 @@ int launch_epi(psb_ctx* c, psb::XEpiArgs<T> e, Epi epi, const char* what, const 
   }
   const int ntile = (e.kz + e.col_tile - 1) / e.col_tile;
   e.main_blocks = ntile * e.n2;
-  int extra = 0;
-  if (e.n3h > e.kz) {
-    const long long pts = (long long)e.n1 * e.n2 * (e.n3h - e.kz);
-    extra = (int)std::min<long long>((pts + 255) / 256, 1024);
-  }
   const size_t smem = (size_t)(L + 2 * L * Epi::F_IN * e.col_tile) * esz;
-  const double bytes = epi.io_bytes((long long)e.n1 * e.n2 * e.n3h) + (double)esz * Epi::F_IN * L * e.n2 * e.kz;
   auto go = [&](auto k) {
     set_smem(k, smem);
     LaunchScope scope(c, what, bytes);
     launch_pdl(k, dim3((unsigned)(e.main_blocks + extra)), 256, smem, c->stream, e, epi);
     return launch_ok(c, what);
   };
-  // a compiled two-pass schedule: the first pass loads straight from global memory
-  if constexpr (TUNABLE) {
-    switch (psb::fixed_plan_id(e.plan)) {
-#define PSB_FIXED_CASE(ID, ...)                                                                       \
-  case ID:                                                                                            \
-    if constexpr (psb::fixed_plan_compiled<T, ID>::value && psb::FixedPlan<ID>::Radices::NP == 2) \
-      return go(psb::xfwd_epi_rr_kernel<T, Epi, ID>);                                                 \
-    break;
-      PSB_FIXED_PLANS(PSB_FIXED_CASE)
-#undef PSB_FIXED_CASE
-      default:
-        break;
-    }
-  }
   // the input tile (ct columns x F fields x L rows) staged by bulk tensor copies
   {
     const int nbox = tma_boxes(L);
@@ -564,31 +625,11 @@ int launch_epi(psb_ctx* c, psb::XEpiArgs<T> e, Epi epi, const char* what, const 
                      c->dstatus);
           return launch_ok(c, what);
         };
-        switch (psb::fixed_plan_id(e.plan)) {
-#define PSB_FIXED_CASE(ID, ...) \
-  case ID:                      \
-    if constexpr (psb::fixed_plan_compiled<T, ID>::value) return got(psb::xfwd_epi_tma_kernel<T, Epi, ID>); \
-    break;
-          PSB_FIXED_PLANS(PSB_FIXED_CASE)
-#undef PSB_FIXED_CASE
-          default:
-            break;
-        }
-        if (!plan_is_wide_h(e.plan)) return got(psb::xfwd_epi_tma_kernel<T, Epi, 0>);
+        if (!plan_is_wide_h(e.plan)) return got(psb::xfwd_epi_tma_kernel<T, Epi>);
       }
     }
   }
   if constexpr (TUNABLE) {
-    switch (psb::fixed_plan_id(e.plan)) {
-#define PSB_FIXED_CASE(ID, ...) \
-  case ID:                      \
-    if constexpr (psb::fixed_plan_compiled<T, ID>::value) return go(psb::xfwd_epi_kernel<T, Epi, false, ID>); \
-    break;
-      PSB_FIXED_PLANS(PSB_FIXED_CASE)
-#undef PSB_FIXED_CASE
-      default:
-        break;
-    }
     if (sh && sh->wide) return go(psb::xfwd_epi_kernel<T, Epi, true>);
   }
   return go(psb::xfwd_epi_kernel<T, Epi>);

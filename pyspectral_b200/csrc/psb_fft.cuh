@@ -336,205 +336,6 @@ __device__ Cx<T>* block_fft(Cx<T>* a, Cx<T>* b, const FFTPlan& p, const Cx<T>* _
 }
 
 
-// ---- transforms with a compile-time length and schedule --------------------
-// The Stockham passes with L, the radix and the sub-transform length Ns known
-// to the compiler, over `nlines` lines of length L held at buf[line*ls + j]
-// (the z-pass layout: each line contiguous, consecutive lines `ls` elements
-// apart; the z pass pads ls to an odd stride, 7 modulo 16, so that the same
-// position of consecutive lines falls in different shared-memory banks).
-//
-// LINES_FAST (used when nlines >= 8): consecutive threads take consecutive
-// lines at the same j.  A warp's loads j + r*L/R, its stores (j-k)R + k + r*Ns
-// and its twiddle reads (one k per j: a broadcast) then spread over the banks
-// by the odd line stride, where in the j-fast order the stores of one line
-// land R elements apart and hit one bank up to 16 times per half-warp.
-// Otherwise consecutive threads take consecutive j of a line.  Items are
-// walked as a (fast, slow) counter pair, without a division.
-template <typename T, int R, bool INV, int L, int NS, bool LINES_FAST>
-__device__ __forceinline__ void stockham_pass_c(const Cx<T>* __restrict__ a, Cx<T>* __restrict__ b,
-                                                const Cx<T>* __restrict__ tw, int nlines, int ls) {
-  constexpr int NB = L / R;
-  constexpr int TS = L / (NS * R);
-  const int mf = LINES_FAST ? nlines : NB;
-  const int ms = LINES_FAST ? NB : nlines;
-  const int nt = blockDim.x;
-  int f = threadIdx.x % mf, sl = threadIdx.x / mf;
-  const int df = nt % mf, ds = nt / mf;
-  while (sl < ms) {
-    const int line = LINES_FAST ? f : sl;
-    const int j = LINES_FAST ? sl : f;
-    const int k = j % NS;
-    const Cx<T>* src = a + line * ls + j;
-    Cx<T> v[R];
-#pragma unroll
-    for (int r = 0; r < R; ++r) v[r] = src[r * NB];
-    if constexpr (NS > 1) {
-#pragma unroll
-      for (int r = 1; r < R; ++r) {
-        Cx<T> w = tw[r * k * TS];
-        if (INV) w.y = -w.y;
-        v[r] = cmul(v[r], w);
-      }
-    }
-    small_dft<T, R, INV>(v);
-    Cx<T>* dst = b + line * ls + (j - k) * R + k;
-#pragma unroll
-    for (int r = 0; r < R; ++r) dst[r * NS] = v[r];
-    f += df;
-    sl += ds;
-    if (f >= mf) {
-      f -= mf;
-      ++sl;
-    }
-  }
-}
-// Passes R, Rest... starting at sub-transform length NS; returns the buffer
-// holding the result.  Ends with __syncthreads.
-template <typename T, bool INV, int L, int NS, bool LF, int R, int... Rest>
-__device__ __forceinline__ Cx<T>* fft_c(Cx<T>* a, Cx<T>* b, const Cx<T>* __restrict__ tw, int nlines, int ls) {
-  stockham_pass_c<T, R, INV, L, NS, LF>(a, b, tw, nlines, ls);
-  __syncthreads();
-  if constexpr (sizeof...(Rest) == 0)
-    return b;
-  else
-    return fft_c<T, INV, L, NS * R, LF, Rest...>(b, a, tw, nlines, ls);
-}
-
-// The same for lines adjacent in memory (element j of line f at f + j*es, the
-// axis-pass layout): items walk (line fast, j slow) as a counter pair.
-template <typename T, int R, bool INV, int L, int NS>
-__device__ __forceinline__ void stockham_pass_cs(const Cx<T>* __restrict__ a, Cx<T>* __restrict__ b,
-                                                 const Cx<T>* __restrict__ tw, int nlines, int es) {
-  constexpr int NB = L / R;
-  constexpr int TS = L / (NS * R);
-  const int nt = blockDim.x;
-  int f = threadIdx.x % nlines, j = threadIdx.x / nlines;
-  const int df = nt % nlines, dj = nt / nlines;
-  const int rs = NB * es, ws = NS * es;
-  while (j < NB) {
-    const int k = j % NS;
-    const Cx<T>* src = a + f + j * es;
-    Cx<T> v[R];
-#pragma unroll
-    for (int r = 0; r < R; ++r) v[r] = src[r * rs];
-    if constexpr (NS > 1) {
-#pragma unroll
-      for (int r = 1; r < R; ++r) {
-        Cx<T> w = tw[r * k * TS];
-        if (INV) w.y = -w.y;
-        v[r] = cmul(v[r], w);
-      }
-    }
-    small_dft<T, R, INV>(v);
-    Cx<T>* dst = b + f + ((j - k) * R + k) * es;
-#pragma unroll
-    for (int r = 0; r < R; ++r) dst[r * ws] = v[r];
-    f += df;
-    j += dj;
-    if (f >= nlines) {
-      f -= nlines;
-      ++j;
-    }
-  }
-}
-template <typename T, bool INV, int L, int NS, int R, int... Rest>
-__device__ __forceinline__ Cx<T>* fft_cs(Cx<T>* a, Cx<T>* b, const Cx<T>* __restrict__ tw, int nlines) {
-  stockham_pass_cs<T, R, INV, L, NS>(a, b, tw, nlines, nlines);
-  __syncthreads();
-  if constexpr (sizeof...(Rest) == 0)
-    return b;
-  else
-    return fft_cs<T, INV, L, NS * R, Rest...>(b, a, tw, nlines);
-}
-
-// Schedules compiled in with their length (id, L, radices): the default
-// schedule of each common 3/2-padded length (48, 72, 96, 192: grids of 32,
-// 48, 64 and 128 points) and two-pass orders of it.
-#define PSB_FIXED_PLANS(X) \
-  X(1, 96, 8, 4, 3)        \
-  X(2, 96, 16, 6)          \
-  X(3, 96, 6, 16)          \
-  X(4, 48, 8, 2, 3)        \
-  X(5, 48, 16, 3)          \
-  X(6, 48, 3, 16)          \
-  X(7, 192, 8, 8, 3)       \
-  X(8, 192, 16, 12)        \
-  X(9, 192, 12, 16)        \
-  X(10, 96, 12, 8)         \
-  X(11, 96, 8, 12)         \
-  X(12, 48, 8, 6)          \
-  X(13, 48, 6, 8)          \
-  X(14, 72, 8, 3, 3)       \
-  X(15, 72, 6, 12)         \
-  X(16, 72, 12, 6)
-constexpr int kFixedPlans = 16;
-
-template <int ID>
-struct FixedPlan;
-template <int R1, int R2 = 0, int R3 = 0>
-struct RadixList {
-  static constexpr int NP = R3 ? 3 : (R2 ? 2 : 1), A = R1, B = R2;
-};
-#define PSB_FIXED_PLAN_DEF(ID, LEN, ...)                                                       \
-  template <>                                                                                   \
-  struct FixedPlan<ID> {                                                                        \
-    static constexpr int L = LEN;                                                               \
-    using Radices = RadixList<__VA_ARGS__>; /* NP passes; A, B the first two radices */         \
-    template <typename T, bool INV>                                                             \
-    static __device__ __forceinline__ Cx<T>* run(Cx<T>* a, Cx<T>* b, const Cx<T>* tw, int n,    \
-                                                 int ls) {                                      \
-      if (n >= 8) return fft_c<T, INV, LEN, 1, true, __VA_ARGS__>(a, b, tw, n, ls);             \
-      return fft_c<T, INV, LEN, 1, false, __VA_ARGS__>(a, b, tw, n, ls);                        \
-    }                                                                                           \
-    template <typename T, bool INV>                                                             \
-    static __device__ __forceinline__ Cx<T>* run_adjacent(Cx<T>* a, Cx<T>* b, const Cx<T>* tw, \
-                                                          int n) {                              \
-      return fft_cs<T, INV, LEN, 1, __VA_ARGS__>(a, b, tw, n);                                  \
-    }                                                                                           \
-  };
-PSB_FIXED_PLANS(PSB_FIXED_PLAN_DEF)
-#undef PSB_FIXED_PLAN_DEF
-
-template <int... R>
-constexpr int count_radices() {
-  return (int)sizeof...(R);
-}
-// The compiled-in schedules as a compile-time table, and the id of the
-// two-pass schedule that runs the radices of `id` in the opposite order (0 if
-// `id` is not a two-pass schedule or its reverse is not compiled in).
-struct FixedDesc {
-  int id, L, n, r[3];
-};
-#define PSB_FIXED_PLAN_CDESC(ID, LEN, ...) FixedDesc{ID, LEN, count_radices<__VA_ARGS__>(), {__VA_ARGS__}},
-constexpr FixedDesc kFixedDescs[] = {PSB_FIXED_PLANS(PSB_FIXED_PLAN_CDESC)};
-#undef PSB_FIXED_PLAN_CDESC
-constexpr int fixed_plan_reversed(int id) {
-  for (const FixedDesc& d : kFixedDescs) {
-    if (d.id != id) continue;
-    if (d.n != 2) return 0;
-    for (const FixedDesc& e : kFixedDescs)
-      if (e.L == d.L && e.n == 2 && e.r[0] == d.r[1] && e.r[1] == d.r[0]) return e.id;
-  }
-  return 0;
-}
-
-// Id of the compiled-in schedule equal to p (0 if none).
-__host__ inline int fixed_plan_id(const FFTPlan& p) {
-  struct D {
-    int id, L, n, r[4];
-  };
-#define PSB_FIXED_PLAN_DESC(ID, LEN, ...) D{ID, LEN, count_radices<__VA_ARGS__>(), {__VA_ARGS__}},
-  static const D table[] = {PSB_FIXED_PLANS(PSB_FIXED_PLAN_DESC)};
-#undef PSB_FIXED_PLAN_DESC
-  for (const D& d : table) {
-    if (d.L != p.L || d.n != p.npass) continue;
-    bool same = true;
-    for (int s = 0; s < d.n; ++s) same = same && d.r[s] == p.radix[s];
-    if (same) return d.id;
-  }
-  return 0;
-}
-
 // Stage a length-L twiddle table into shared memory.
 template <typename T>
 __device__ __forceinline__ void stage_twiddles(Cx<T>* tw_s, const Cx<T>* __restrict__ pool, const FFTPlan& p) {

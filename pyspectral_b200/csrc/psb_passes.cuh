@@ -182,16 +182,6 @@ __device__ __forceinline__ int row_of(const RowMap& m, int p, int rows) {
 
 // One CTA of an axis pass: column tile bx, outer index by.
 // smem = tw[L] + 2 * L*lines
-// Transform of `lines` adjacent lines (axis-pass layout): the plan's schedule
-// (FP = 0) or the compiled-in schedule FP (which must equal the plan's).
-template <typename T, bool INV, bool WIDE, int FP>
-__device__ __forceinline__ Cx<T>* axfft(Cx<T>* a, Cx<T>* b, const FFTPlan& p, const Cx<T>* tw, int lines) {
-  if constexpr (FP == 0)
-    return block_fft<T, INV, WIDE>(a, b, p, tw, lines, 1, lines, true);
-  else
-    return FixedPlan<FP>::template run_adjacent<T, INV>(a, b, tw, lines);
-}
-
 // Transform of a staged tile (F fields x ct columns, position-major in bufA)
 // and the store of its output rows.  Must be called by all threads.
 template <typename T, bool INV, int F, bool WIDE>
@@ -735,11 +725,6 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 1)
   zpass_batch_body<T, Phys, WIDE>(A, phys, runs);
 }
 
-template <typename T, int FP>
-struct fixed_plan_compiled {
-  static constexpr bool value = sizeof(T) == 4 || FP == 1 || FP == 4 || FP == 7;
-};
-
 // ---------------------------------------------------------------------------
 template <typename T>
 struct XEpiArgs {
@@ -776,7 +761,7 @@ __device__ __forceinline__ void xfwd_epi_extra(const XEpiArgs<T>& a, const Epi& 
 
 // Transform of a staged tile and the epilogue on its output rows.  Must be
 // called by all threads.
-template <typename T, class Epi, bool WIDE, int FP>
+template <typename T, class Epi, bool WIDE>
 __device__ __forceinline__ void xfwd_transform_epi(const XEpiArgs<T>& a, const Epi& epi, Cx<T>* bufA, Cx<T>* bufB,
                                                    const Cx<T>* tw, int o, int c0) {
   constexpr int F = Epi::F_IN;
@@ -788,7 +773,7 @@ __device__ __forceinline__ void xfwd_transform_epi(const XEpiArgs<T>& a, const E
   const int c = threadIdx.x % ct, r0 = threadIdx.x / ct, dr = nt / ct;
   const int col = c0 + c;
   const bool colok = col < a.kz;
-  Cx<T>* res = axfft<T, false, WIDE, FP>(bufA, bufB, a.plan, tw, lines);
+  Cx<T>* res = block_fft<T, false, WIDE>(bufA, bufB, a.plan, tw, lines, 1, lines, true);
   // threads past the last full row of columns would repeat a (row, column)
   // (only when ct does not divide the CTA size): the epilogue is not idempotent
   if (!colok || threadIdx.x >= dr * ct) return;
@@ -802,7 +787,7 @@ __device__ __forceinline__ void xfwd_transform_epi(const XEpiArgs<T>& a, const E
 
 // One CTA of the x-forward epilogue pass: block bx of gx = main_blocks + extra;
 // main block b -> (col tile b % ntile, outer b / ntile)
-template <typename T, class Epi, bool WIDE = false, int FP = 0>
+template <typename T, class Epi, bool WIDE = false>
 __device__ __forceinline__ void xfwd_epi_body(const XEpiArgs<T>& a, const Epi& epi, int bx, int gx) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   constexpr int F = Epi::F_IN;
@@ -848,7 +833,7 @@ __device__ __forceinline__ void xfwd_epi_body(const XEpiArgs<T>& a, const Epi& e
     }
   }
   __syncthreads();
-  xfwd_transform_epi<T, Epi, WIDE, FP>(a, epi, bufA, bufB, tw, o, c0);
+  xfwd_transform_epi<T, Epi, WIDE>(a, epi, bufA, bufB, tw, o, c0);
 }
 
 // TMA-staged x-forward epilogue pass: the tile (ct columns x F fields x L
@@ -856,7 +841,7 @@ __device__ __forceinline__ void xfwd_epi_body(const XEpiArgs<T>& a, const Epi& e
 // through map, a 4-D view (columns, fields, rows, outer index) of a.in.  A
 // copy that does not complete within the poll limit raises *status and the
 // CTA hands NaN to the epilogue in place of its tile.
-template <typename T, class Epi, int FP = 0>
+template <typename T, class Epi>
 __global__ void __launch_bounds__(256) xfwd_epi_tma_kernel(XEpiArgs<T> a, Epi epi,
                                                            const __grid_constant__ CUtensorMap map, int nbox,
                                                            int* status) {
@@ -904,85 +889,19 @@ __global__ void __launch_bounds__(256) xfwd_epi_tma_kernel(XEpiArgs<T> a, Epi ep
     for (int l = threadIdx.x; l < L * lines; l += blockDim.x) bufA[l] = mk<T>(nan_of<T>(), nan_of<T>());
     __syncthreads();
   }
-  xfwd_transform_epi<T, Epi, false, FP>(a, epi, bufA, bufB, tw, o, c0);
-}
-
-// The x-forward epilogue pass with a two-pass compiled schedule: the first
-// pass loads its elements straight from the input rows, the second writes the
-// transformed tile to shared memory for the epilogue (which needs every field
-// of a point in one thread).  smem = L twiddles + 2 L F ct elements.
-template <typename T, class Epi, int FP>
-__global__ void __launch_bounds__(256) xfwd_epi_rr_kernel(XEpiArgs<T> a, Epi epi) {
-  using FPl = FixedPlan<FP>;
-  constexpr int L = FPl::L, R1 = FPl::Radices::A, R2 = FPl::Radices::B;
-  static_assert(FPl::Radices::NP == 2 && R1 * R2 == L, "two-pass schedules only");
-  constexpr int F = Epi::F_IN, NB1 = L / R1, NB2 = L / R2;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  pdl_trigger();
-  if ((int)blockIdx.x >= a.main_blocks) {
-    pdl_wait();
-    xfwd_epi_extra<T, Epi>(a, epi, blockIdx.x, gridDim.x);
-    return;
-  }
-  Cx<T>* tw = reinterpret_cast<Cx<T>*>(smem_raw);
-  const int ct = a.col_tile, lines = F * ct;
-  Cx<T>* X = tw + L;
-  Cx<T>* Y = X + (size_t)L * lines;
-  const int ntile = (a.kz + ct - 1) / ct;
-  const int o = blockIdx.x / ntile;
-  const int c0 = (blockIdx.x % ntile) * ct;
-  const Cx<T> zero = mk<T>(0, 0);
-  stage_twiddles(tw, a.tw, a.plan);
-  pdl_wait();
-  const Cx<T>* inb = a.in + (long long)o * a.in_ostride;
-  for (Walk2 w(lines); w.s < NB1; w.next()) {
-    const int line = w.f, j1 = w.s;
-    const int f = line / ct, col = c0 + (line - f * ct);
-    Cx<T> v[R1];
-#pragma unroll
-    for (int r = 0; r < R1; ++r)
-      v[r] = col < a.kz ? inb[f * a.in_fstride + (j1 + r * NB1) * a.in_rstride + col] : zero;
-    small_dft<T, R1, false>(v);
-#pragma unroll
-    for (int r = 0; r < R1; ++r) X[(size_t)(j1 * R1 + r) * lines + line] = v[r];
-  }
-  __syncthreads();
-  for (Walk2 w(lines); w.s < NB2; w.next()) {
-    const int line = w.f, j2 = w.s;
-    const int k = j2 % R1;
-    Cx<T> v[R2];
-#pragma unroll
-    for (int r = 0; r < R2; ++r) v[r] = X[(size_t)(j2 + r * NB2) * lines + line];
-#pragma unroll
-    for (int r = 1; r < R2; ++r) v[r] = cmul(v[r], tw[r * k]);
-    small_dft<T, R2, false>(v);
-#pragma unroll
-    for (int r = 0; r < R2; ++r) Y[(size_t)((j2 - k) * R2 + k + r * R1) * lines + line] = v[r];
-  }
-  __syncthreads();
-  const int nt = blockDim.x;
-  const int c = threadIdx.x % ct, r0 = threadIdx.x / ct, dr = nt / ct;
-  const int col = c0 + c;
-  if (col >= a.kz || threadIdx.x >= dr * ct) return;
-  Cx<T> P[F];
-  for (int i1 = r0; i1 < a.n1; i1 += dr) {
-    const int j = a.out_map(i1);
-#pragma unroll
-    for (int f = 0; f < F; ++f) P[f] = j >= 0 ? Y[(size_t)j * lines + f * ct + c] : zero;
-    epi(i1, o, col, P);
-  }
+  xfwd_transform_epi<T, Epi, false>(a, epi, bufA, bufB, tw, o, c0);
 }
 
 // grid = main_blocks + extra
-template <typename T, class Epi, bool WIDE = false, int FP = 0>
+template <typename T, class Epi, bool WIDE = false>
 __global__ void __launch_bounds__(256) xfwd_epi_kernel(XEpiArgs<T> a, Epi epi) {
-  xfwd_epi_body<T, Epi, WIDE, FP>(a, epi, blockIdx.x, gridDim.x);
+  xfwd_epi_body<T, Epi, WIDE>(a, epi, blockIdx.x, gridDim.x);
 }
 
 // Batched: grid = (main_blocks + extra, runs); run blockIdx.y reads A[y], epi[y].
-template <typename T, class Epi, bool WIDE, int FP = 0>
+template <typename T, class Epi, bool WIDE>
 __global__ void __launch_bounds__(256) xfwd_epi_batch(const XEpiArgs<T>* __restrict__ A, const Epi* __restrict__ epi) {
-  xfwd_epi_body<T, Epi, WIDE, FP>(A[blockIdx.y], epi[blockIdx.y], blockIdx.x, gridDim.x);
+  xfwd_epi_body<T, Epi, WIDE>(A[blockIdx.y], epi[blockIdx.y], blockIdx.x, gridDim.x);
 }
 
 }  // namespace psb

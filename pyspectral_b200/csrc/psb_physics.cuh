@@ -56,30 +56,54 @@ struct StepIO {
     if (w0_out) b += (double)sizeof(Cx<T>) * npts * 3;
     return b;
   }
+  // What finish() reads of one mode and field, so that a caller can issue the
+  // loads of several modes before the first store.
+  struct Old {
+    Cx<T> base, c;
+  };
+  // q: the state at this mode, when the caller has read it (stage 1 starts from it)
+  __device__ __forceinline__ Old fetch(long long s, int f, Cx<T> q) const {
+    const long long e = f * fstride + s;
+    Old o;
+    o.base = q;
+    o.c = mk<T>(0, 0);
+    if (mode == kStageMid || mode == kStageLast) o.base = Q0[e];
+    if (mode != kRHS && comp != nullptr) o.c = comp[e];
+    return o;
+  }
   // Q = Q0 + dt*c*RHS  (PySpectral/src/PySpec_3d.py:104), Kahan-compensated when comp != null.
-  __device__ __forceinline__ void finish(long long s, int f, Cx<T> R) const {
+  __device__ __forceinline__ void finish(long long s, int f, Cx<T> R, const Old& o) const {
     const long long e = f * fstride + s;
     if (mode == kRHS) {
       rhs_out[e] = R;
       return;
     }
-    Cx<T> base;
-    if (mode == kStage1) {
-      base = Q[e];
-      Q0[e] = base;
-    } else {
-      base = Q0[e];
-    }
+    if (mode == kStage1) Q0[e] = o.base;
     const Cx<T> inc = dtc * R;
     if (comp == nullptr) {
-      Q[e] = base + inc;
+      Q[e] = o.base + inc;
     } else {
-      const Cx<T> c = comp[e];
-      const Cx<T> y = inc - c;
-      const Cx<T> t = base + y;
-      if (mode == kStageLast) comp[e] = (t - base) - y;
+      const Cx<T> y = inc - o.c;
+      const Cx<T> t = o.base + y;
+      if (mode == kStageLast) comp[e] = (t - o.base) - y;
       Q[e] = t;
     }
+  }
+  __device__ __forceinline__ void finish(long long s, int f, Cx<T> R) const {
+    finish(s, f, R, fetch(s, f, mode == kStage1 ? Q[f * fstride + s] : mk<T>(0, 0)));
+  }
+};
+
+// The state of NF fields at a mode and what the RK stage needs beside it.
+template <typename T, int NF>
+struct StateIn {
+  Cx<T> q[NF];
+  typename StepIO<T>::Old o[NF];
+  __device__ __forceinline__ void load(const StepIO<T>& io, long long s) {
+#pragma unroll
+    for (int f = 0; f < NF; ++f) q[f] = io.Q[f * io.fstride + s];
+#pragma unroll
+    for (int f = 0; f < NF; ++f) o[f] = io.fetch(s, f, q[f]);
   }
 };
 
@@ -173,10 +197,69 @@ struct KTabs {
   const double *k1, *k2, *k3;
 };
 
-// DNS / Smagorinsky epilogue (PySpectral/src/RHSfunctions.py:29-50, :164-232)
+// Spectral epilogues in two halves.  acc(f, k1, k2, k3, v, D) adds product
+// spectrum f to NACC accumulators D[m][r] of R modes that differ in k1 only;
+// ld(i1, i2, i3) reads what one mode needs beside its products, and fin(i1, i2,
+// i3, D, in) forms the mode's right-hand side from its NACC sums and stores it
+// (apart, so that the loads of several modes are in flight together).  The right-hand sides are linear in the products, so a thread
+// needs the sums (the divergence k_j P_ij, and what else a closure contracts)
+// and not the products: the register x pass (psb_xreg.cuh) takes the fields one
+// after another.  operator() is both for one mode with its F_IN products.
+template <int R, typename T>
+__device__ __forceinline__ void acc_row(T k, const Cx<T>* v, Cx<T>* D) {
+#pragma unroll
+  for (int r = 0; r < R; ++r) D[r] = mk<T>(D[r].x + k * v[r].x, D[r].y + k * v[r].y);
+}
+template <int R, typename T>
+__device__ __forceinline__ void acc_row(const T* k, const Cx<T>* v, Cx<T>* D) {
+#pragma unroll
+  for (int r = 0; r < R; ++r) D[r] = mk<T>(D[r].x + k[r] * v[r].x, D[r].y + k[r] * v[r].y);
+}
+// D_i += k_j P_ij for symmetric product f of 11, 22, 33, 12, 13, 23
+template <int R, typename T>
+__device__ __forceinline__ void acc_sym(int f, const T* k1, T k2, T k3, const Cx<T>* v, Cx<T> (*D)[R]) {
+  switch (f) {
+    case 0:
+      acc_row<R>(k1, v, D[0]);
+      break;
+    case 1:
+      acc_row<R>(k2, v, D[1]);
+      break;
+    case 2:
+      acc_row<R>(k3, v, D[2]);
+      break;
+    case 3:
+      acc_row<R>(k2, v, D[0]);
+      acc_row<R>(k1, v, D[1]);
+      break;
+    case 4:
+      acc_row<R>(k3, v, D[0]);
+      acc_row<R>(k1, v, D[2]);
+      break;
+    default:
+      acc_row<R>(k3, v, D[1]);
+      acc_row<R>(k2, v, D[2]);
+      break;
+  }
+}
+// both halves for one mode
+template <typename T, class Epi>
+__device__ __forceinline__ void epi_point(const Epi& e, int i1, int i2, int i3, const Cx<T>* P) {
+  const KTabs<T> kt = e.ktabs();
+  const T k1 = (T)kt.k1[i1], k2 = (T)kt.k2[i2], k3 = (T)kt.k3[i3];
+  Cx<T> D[Epi::NACC][1];
+#pragma unroll
+  for (int m = 0; m < Epi::NACC; ++m) D[m][0] = mk<T>(0, 0);
+#pragma unroll
+  for (int f = 0; f < Epi::F_IN; ++f) e.template acc<1>(f, &k1, k2, k3, P + f, D);
+  e.fin(i1, i2, i3, &D[0][0], e.ld(i1, i2, i3));
+}
+
+// DNS / Smagorinsky epilogue (PySpectral/src/RHSfunctions.py:29-50, :164-232).
+// Sums: k_j (u_i u_j)^, and k_j tau_ij^ for Smagorinsky with the closure force kept.
 template <typename T, bool SMAG>
 struct EpiNS {
-  static constexpr int F_IN = SMAG ? 12 : 6;
+  static constexpr int F_IN = SMAG ? 12 : 6, NACC = SMAG ? 6 : 3;
   __host__ double io_bytes(long long npts) const { return io.bytes(npts, 3); }
   StepIO<T> io;
   KTabs<T> k;
@@ -185,60 +268,119 @@ struct EpiNS {
   T Om1, Om2, Om3;
   int zero_nyq;  // unpad(pad(uhat)) on read (:10-12); absent in SMAG
   int ny1, ny2, ny3;
-  __device__ void operator()(int i1, int i2, int i3, const Cx<T>* P) const {
-    const long long s = io.sidx(i1, i2, i3);
-    Cx<T> u = io.Q[s], v = io.Q[io.fstride + s], w = io.Q[2 * io.fstride + s];
-    if (zero_nyq && (i1 == ny1 || i2 == ny2 || i3 == ny3)) u = v = w = mk<T>(0, 0);
-    const T k1 = (T)k.k1[i1], k2 = (T)k.k2[i2], k3 = (T)k.k3[i3];
-    T ksq, ksqi;
-    ksq_pair(k1, k2, k3, ksq, ksqi);
-    const Cx<T> uu = P[0], vv = P[1], ww = P[2], uv = P[3], uw = P[4], vw = P[5];
-    Cx<T> ph = ksqi * ((-k1 * k1) * uu - (k2 * k2) * vv - (k3 * k3) * ww - ((T)2 * k1 * k2) * uv -
-                       ((T)2 * k1 * k3) * uw - ((T)2 * k2 * k3) * vw);
-    Cx<T> cu = mk<T>(0, 0), cv = cu, cw = cu;
-    if (rotate) {
-      cu = Om3 * v - Om2 * w;
-      cv = Om1 * w - Om3 * u;
-      cw = Om2 * u - Om1 * v;
-      // phat -= 2 ksqr_i 1j (k . (u x Om)) (:33-36)
-      const Cx<T> kd = k1 * cu + k2 * cv + k3 * cw;
-      ph = ph - ((T)2 * ksqi) * mul_i(kd);
-    }
-    Cx<T> ru = mik(k1, uu) + mik(k2, uv) + mik(k3, uw) + mik(k1, ph) - (nu * ksq) * u;
-    Cx<T> rv = mik(k1, uv) + mik(k2, vv) + mik(k3, vw) + mik(k2, ph) - (nu * ksq) * v;
-    Cx<T> rw = mik(k1, uw) + mik(k2, vw) + mik(k3, ww) + mik(k3, ph) - (nu * ksq) * w;
+  __device__ __forceinline__ KTabs<T> ktabs() const { return k; }
+  template <int R>
+  __device__ __forceinline__ void acc(int f, const T* k1, T k2, T k3, const Cx<T>* v, Cx<T> (*D)[R]) const {
     if constexpr (SMAG) {
-      // projected SGS divergence (:215-222); note 1j*k_i*(1j*ksqr_i*(kk:tau))
-      const Cx<T> t11 = P[6], t22 = P[7], t33 = P[8], t12 = P[9], t13 = P[10], t23 = P[11];
-      const Cx<T> kk = (k1 * k1) * t11 + (k2 * k2) * t22 + (k3 * k3) * t33 + ((T)2 * k1 * k2) * t12 +
-                       ((T)2 * k1 * k3) * t13 + ((T)2 * k2 * k3) * t23;
-      const Cx<T> proj = mul_i(ksqi * kk);
-      const Cx<T> w0u = mik(k1, t11) + mik(k2, t12) + mik(k3, t13) + pik(k1, proj);
-      const Cx<T> w0v = mik(k1, t12) + mik(k2, t22) + mik(k3, t23) + pik(k2, proj);
-      const Cx<T> w0w = mik(k1, t13) + mik(k2, t23) + mik(k3, t33) + pik(k3, proj);
-      ru = ru + w0u;
-      rv = rv + w0v;
-      rw = rw + w0w;
-      if (io.w0_out) {
-        io.w0_out[s] = w0u;
-        io.w0_out[io.fstride + s] = w0v;
-        io.w0_out[2 * io.fstride + s] = w0w;
+      if (f >= 6) {
+        acc_sym<R>(f - 6, k1, k2, k3, v, D + 3);
+        return;
       }
     }
-    if (rotate) {  // + 2 u x Om (:47-50)
-      ru = ru + (T)2 * cu;
-      rv = rv + (T)2 * cv;
-      rw = rw + (T)2 * cw;
-    }
-    if (io.read_out) {
-      io.read_out[s] = u;
-      io.read_out[io.fstride + s] = v;
-      io.read_out[2 * io.fstride + s] = w;
-    }
-    io.finish(s, 0, ru);
-    io.finish(s, 1, rv);
-    io.finish(s, 2, rw);
+    acc_sym<R>(f, k1, k2, k3, v, D);
   }
+  using In = StateIn<T, 3>;
+  __device__ __forceinline__ In ld(int i1, int i2, int i3) const {
+    In in;
+    in.load(io, io.sidx(i1, i2, i3));
+    return in;
+  }
+  __device__ __forceinline__ void fin(int i1, int i2, int i3, const Cx<T>* D, const In& in) const {
+    const long long s = io.sidx(i1, i2, i3);
+    Cx<T> u[3] = {in.q[0], in.q[1], in.q[2]};
+    if (zero_nyq && (i1 == ny1 || i2 == ny2 || i3 == ny3)) u[0] = u[1] = u[2] = mk<T>(0, 0);
+    const T kv[3] = {(T)k.k1[i1], (T)k.k2[i2], (T)k.k3[i3]};
+    T ksq, ksqi;
+    ksq_pair(kv[0], kv[1], kv[2], ksq, ksqi);
+    Cx<T> ph = (-ksqi) * (kv[0] * D[0] + kv[1] * D[1] + kv[2] * D[2]);
+    Cx<T> c[3];
+    if (rotate) {
+      c[0] = Om3 * u[1] - Om2 * u[2];
+      c[1] = Om1 * u[2] - Om3 * u[0];
+      c[2] = Om2 * u[0] - Om1 * u[1];
+      // phat -= 2 ksqr_i 1j (k . (u x Om)) (:33-36)
+      ph = ph - ((T)2 * ksqi) * mul_i(kv[0] * c[0] + kv[1] * c[1] + kv[2] * c[2]);
+    }
+    // projected SGS divergence (:215-222); note 1j*k_i*(1j*ksqr_i*(kk:tau))
+    Cx<T> kk = mk<T>(0, 0);
+    if constexpr (SMAG) kk = ksqi * (kv[0] * D[3] + kv[1] * D[4] + kv[2] * D[5]);
+#pragma unroll
+    for (int m = 0; m < 3; ++m) {
+      Cx<T> r = mul_mi(D[m]) + mik(kv[m], ph) - (nu * ksq) * u[m];
+      if constexpr (SMAG) {
+        const Cx<T> w0 = mul_mi(D[3 + m]) - kv[m] * kk;
+        r = r + w0;
+        if (io.w0_out) io.w0_out[m * io.fstride + s] = w0;
+      }
+      if (rotate) r = r + (T)2 * c[m];  // + 2 u x Om (:47-50)
+      if (io.read_out) io.read_out[m * io.fstride + s] = u[m];
+      io.finish(s, m, r, in.o[m]);
+    }
+  }
+  __device__ void operator()(int i1, int i2, int i3, const Cx<T>* P) const { epi_point<T>(*this, i1, i2, i3, P); }
+};
+
+// The Smagorinsky epilogue when the closure force itself is not asked for (RK
+// stages).  The divergence is linear, so u_i u_j and tau_ij share three sums
+// k_j (u_i u_j + tau_ij)^; the projections differ (1j*ksqr_i against ksqr_i),
+// which needs the scalar kk:tau^ as well.  With C = uu + tau and s = ksqr_i kk:tau,
+//   -1j k_j uu_ij - 1j k_i phat + w0_i = -1j (k_j C_ij - k_i ksqr_i kk:C) - (1 + 1j) k_i s.
+template <typename T>
+struct EpiSmagStep {
+  static constexpr int F_IN = 12, NACC = 4;
+  __host__ double io_bytes(long long npts) const { return io.bytes(npts, 3); }
+  StepIO<T> io;
+  KTabs<T> k;
+  T nu;
+  int rotate;
+  T Om1, Om2, Om3;
+  __device__ __forceinline__ KTabs<T> ktabs() const { return k; }
+  template <int R>
+  __device__ __forceinline__ void acc(int f, const T* k1, T k2, T k3, const Cx<T>* v, Cx<T> (*D)[R]) const {
+    if (f < 6) {
+      acc_sym<R>(f, k1, k2, k3, v, D);
+      return;
+    }
+    acc_sym<R>(f - 6, k1, k2, k3, v, D);
+    T kk[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+      kk[r] = f == 6 ? k1[r] * k1[r]
+                     : (f == 7 ? k2 * k2
+                               : (f == 8 ? k3 * k3
+                                         : (f == 9 ? (T)2 * k1[r] * k2 : (f == 10 ? (T)2 * k1[r] * k3 : (T)2 * k2 * k3))));
+    acc_row<R>(kk, v, D[3]);
+  }
+  using In = StateIn<T, 3>;
+  __device__ __forceinline__ In ld(int i1, int i2, int i3) const {
+    In in;
+    in.load(io, io.sidx(i1, i2, i3));
+    return in;
+  }
+  __device__ __forceinline__ void fin(int i1, int i2, int i3, const Cx<T>* D, const In& in) const {
+    const long long s = io.sidx(i1, i2, i3);
+    const Cx<T> u[3] = {in.q[0], in.q[1], in.q[2]};
+    const T kv[3] = {(T)k.k1[i1], (T)k.k2[i2], (T)k.k3[i3]};
+    T ksq, ksqi;
+    ksq_pair(kv[0], kv[1], kv[2], ksq, ksqi);
+    Cx<T> ph = (-ksqi) * (kv[0] * D[0] + kv[1] * D[1] + kv[2] * D[2]);
+    Cx<T> c[3];
+    if (rotate) {
+      c[0] = Om3 * u[1] - Om2 * u[2];
+      c[1] = Om1 * u[2] - Om3 * u[0];
+      c[2] = Om2 * u[0] - Om1 * u[1];
+      ph = ph - ((T)2 * ksqi) * mul_i(kv[0] * c[0] + kv[1] * c[1] + kv[2] * c[2]);
+    }
+    const Cx<T> t = mk<T>(ksqi * (D[3].x - D[3].y), ksqi * (D[3].x + D[3].y));  // (1 + 1j) s
+#pragma unroll
+    for (int m = 0; m < 3; ++m) {
+      Cx<T> r = mul_mi(D[m]) + mik(kv[m], ph) - kv[m] * t - (nu * ksq) * u[m];
+      if (rotate) r = r + (T)2 * c[m];
+      if (io.read_out) io.read_out[m * io.fstride + s] = u[m];
+      io.finish(s, m, r, in.o[m]);
+    }
+  }
+  __device__ void operator()(int i1, int i2, int i3, const Cx<T>* P) const { epi_point<T>(*this, i1, i2, i3, P); }
 };
 
 // ---- MHD (2/3 rule, unpadded), PySpectral/src_MPI/RHSfunctions.py:95-175 ------
@@ -273,9 +415,34 @@ struct PhysMHD {
   }
 };
 
+// sums of the MHD products: k_j N_ij (3) and the curl k x X of X = u x B (3)
+template <int R, typename T>
+__device__ __forceinline__ void acc_mhd(int f, const T* k1, T k2, T k3, const Cx<T>* v, Cx<T> (*D)[R]) {
+  T m1[R];
+  switch (f) {
+    case 6:
+      acc_row<R>(k3, v, D[4]);
+      acc_row<R>(-k2, v, D[5]);
+      break;
+    case 7:
+      acc_row<R>(-k3, v, D[3]);
+      acc_row<R>(k1, v, D[5]);
+      break;
+    case 8:
+#pragma unroll
+      for (int r = 0; r < R; ++r) m1[r] = -k1[r];
+      acc_row<R>(k2, v, D[3]);
+      acc_row<R>(m1, v, D[4]);
+      break;
+    default:
+      acc_sym<R>(f, k1, k2, k3, v, D);
+      break;
+  }
+}
+
 template <typename T>
 struct EpiMHD {
-  static constexpr int F_IN = 9;
+  static constexpr int F_IN = 9, NACC = 6;
   __host__ double io_bytes(long long npts) const {
     return io.bytes(npts, 6) + (force ? (double)sizeof(Cx<T>) * npts * 3 : 0.0);
   }
@@ -284,39 +451,45 @@ struct EpiMHD {
   const double *m1, *m2, *m3;
   const Cx<T>* force;  // 3 fields or null
   T nu, eta;
-  __device__ void operator()(int i1, int i2, int i3, const Cx<T>* P) const {
+  __device__ __forceinline__ KTabs<T> ktabs() const { return k; }
+  template <int R>
+  __device__ __forceinline__ void acc(int f, const T* k1, T k2, T k3, const Cx<T>* v, Cx<T> (*A)[R]) const {
+    acc_mhd<R>(f, k1, k2, k3, v, A);
+  }
+  struct In {
+    StateIn<T, 6> st;
+    Cx<T> force[3];
+  };
+  __device__ __forceinline__ In ld(int i1, int i2, int i3) const {
+    const long long s = io.sidx(i1, i2, i3);
+    In in;
+    in.st.load(io, s);
+#pragma unroll
+    for (int f = 0; f < 3; ++f) in.force[f] = force ? force[f * io.fstride + s] : mk<T>(0, 0);
+    return in;
+  }
+  __device__ __forceinline__ void fin(int i1, int i2, int i3, const Cx<T>* A, const In& in) const {
     const long long s = io.sidx(i1, i2, i3);
     const T D = (T)(m1[i1] * m2[i2] * m3[i3]);
-    Cx<T> st[6];
-#pragma unroll
-    for (int f = 0; f < 6; ++f) st[f] = D * io.Q[f * io.fstride + s];
-    const T k1 = (T)k.k1[i1], k2 = (T)k.k2[i2], k3 = (T)k.k3[i3];
+    const T kv[3] = {(T)k.k1[i1], (T)k.k2[i2], (T)k.k3[i3]};
     T ksq, ksqi;
-    ksq_pair(k1, k2, k3, ksq, ksqi);
-    const Cx<T> n0 = P[0], n1 = P[1], n2 = P[2], n3 = P[3], n4 = P[4], n5 = P[5];
-    const Cx<T> x0 = P[6], x1 = P[7], x2 = P[8];
-    const Cx<T> ph = ksqi * ((-k1 * k1) * n0 - (k2 * k2) * n1 - (k3 * k3) * n2 - ((T)2 * k1 * k2) * n3 -
-                             ((T)2 * k1 * k3) * n4 - ((T)2 * k2 * k3) * n5);
-    Cx<T> f0 = mk<T>(0, 0), f1 = f0, f2 = f0;
-    if (force) {
-      f0 = force[s];
-      f1 = force[io.fstride + s];
-      f2 = force[2 * io.fstride + s];
-    }
-    Cx<T> r[6];
-    r[0] = D * (mik(k1, n0) + mik(k2, n3) + mik(k3, n4) + mik(k1, ph) - (nu * ksq) * st[0] + f0);
-    r[1] = D * (mik(k1, n3) + mik(k2, n1) + mik(k3, n5) + mik(k2, ph) - (nu * ksq) * st[1] + f1);
-    r[2] = D * (mik(k1, n4) + mik(k2, n5) + mik(k3, n2) + mik(k3, ph) - (nu * ksq) * st[2] + f2);
-    r[3] = D * ((pik(k2, x2) - pik(k3, x1)) - (eta * ksq) * st[3]);
-    r[4] = D * ((pik(k3, x0) - pik(k1, x2)) - (eta * ksq) * st[4]);
-    r[5] = D * ((pik(k1, x1) - pik(k2, x0)) - (eta * ksq) * st[5]);
-    if (io.read_out) {
+    ksq_pair(kv[0], kv[1], kv[2], ksq, ksqi);
+    const Cx<T> ph = (-ksqi) * (kv[0] * A[0] + kv[1] * A[1] + kv[2] * A[2]);
 #pragma unroll
-      for (int f = 0; f < 6; ++f) io.read_out[f * io.fstride + s] = st[f];
+    for (int f = 0; f < 6; ++f) {
+      const Cx<T> st = D * in.st.q[f];
+      Cx<T> r;
+      if (f < 3) {
+        r = mul_mi(A[f]) + mik(kv[f], ph) - (nu * ksq) * st;
+        r = r + in.force[f];
+      } else {
+        r = mul_i(A[f]) - (eta * ksq) * st;
+      }
+      if (io.read_out) io.read_out[f * io.fstride + s] = st;
+      io.finish(s, f, D * r, in.st.o[f]);
     }
-#pragma unroll
-    for (int f = 0; f < 6; ++f) io.finish(s, f, r[f]);
   }
+  __device__ void operator()(int i1, int i2, int i3, const Cx<T>* P) const { epi_point<T>(*this, i1, i2, i3, P); }
 };
 
 // ---- 2x-padded memory closures: t-model, static/dynamic tau-model -----------
@@ -334,7 +507,7 @@ __device__ __forceinline__ bool in_p_axis(int i, int N) { return i < N / 2 || i 
 // the dynamic model is stored on the compact G2 box.
 template <typename T>
 struct EpiPL {
-  static constexpr int F_IN = 6;
+  static constexpr int F_IN = 6, NACC = 3;
   // npts = 2x-grid points: q part written everywhere, resolved state read / PL_p written on the N grid
   __host__ double io_bytes(long long npts) const {
     const double e = (double)sizeof(Cx<T>);
@@ -356,7 +529,16 @@ struct EpiPL {
   Cx<T>* Lbox;         // (3, 2kfb-1, 2kfb-1, kfb) Leonard pieces, or null
   int kfb;             // box half-size (test-filter kf)
   Cx<T>* PLfull;       // (3, 2N1, 2N2, N3+1) PL on the whole 2x grid, or null
-  __device__ void operator()(int i1, int i2, int i3, const Cx<T>* P) const {
+  __device__ __forceinline__ KTabs<T> ktabs() const { return kf; }
+  template <int R>
+  __device__ __forceinline__ void acc(int f, const T* k1, T k2, T k3, const Cx<T>* v, Cx<T> (*D)[R]) const {
+    acc_sym<R>(f, k1, k2, k3, v, D);
+  }
+  __device__ void operator()(int i1, int i2, int i3, const Cx<T>* P) const { epi_point<T>(*this, i1, i2, i3, P); }
+  struct In {
+    Cx<T> u, v, w;
+  };
+  __device__ __forceinline__ In ld(int i1, int i2, int i3) const {
     const int n1 = unpad2x_idx(i1, N1), n2 = unpad2x_idx(i2, N2);
     const int n3 = i3 < N3 / 2 ? i3 : -1;
     Cx<T> u = mk<T>(0, 0), v = u, w = u;
@@ -369,19 +551,21 @@ struct EpiPL {
       v = g * Q[fstride_n + s];
       w = g * Q[2 * fstride_n + s];
     }
+    return In{u, v, w};
+  }
+  __device__ __forceinline__ void fin(int i1, int i2, int i3, const Cx<T>* D, const In& in) const {
+    const int n1 = unpad2x_idx(i1, N1), n2 = unpad2x_idx(i2, N2);
+    const int n3 = i3 < N3 / 2 ? i3 : -1;
+    const Cx<T> u = in.u, v = in.v, w = in.w;
     const T k1 = (T)kf.k1[i1], k2 = (T)kf.k2[i2], k3 = (T)kf.k3[i3];
     T ksq, ksqi;
     ksq_pair(k1, k2, k3, ksq, ksqi);
-    const Cx<T> uu = P[0], vv = P[1], ww = P[2], uv = P[3], uw = P[4], vw = P[5];
-    Cx<T> ph = ksqi * ((-k1 * k1) * uu - (k2 * k2) * vv - (k3 * k3) * ww - ((T)2 * k1 * k2) * uv -
-                       ((T)2 * k1 * k3) * uw - ((T)2 * k2 * k3) * vw);
+    Cx<T> ph = (-ksqi) * (k1 * D[0] + k2 * D[1] + k3 * D[2]);
     if (rotate) {
       const Cx<T> cu = Om3 * v - Om2 * w, cv = Om1 * w - Om3 * u, cw = Om2 * u - Om1 * v;
       ph = ph - ((T)2 * ksqi) * mul_i(k1 * cu + k2 * cv + k3 * cw);
     }
-    const Cx<T> au = mik(k1, uu) + mik(k2, uv) + mik(k3, uw);
-    const Cx<T> av = mik(k1, uv) + mik(k2, vv) + mik(k3, vw);
-    const Cx<T> aw = mik(k1, uw) + mik(k2, vw) + mik(k3, ww);
+    const Cx<T> au = mul_mi(D[0]), av = mul_mi(D[1]), aw = mul_mi(D[2]);
     const Cx<T> pu = au + mik(k1, ph) - (nu * ksq) * u;
     const Cx<T> pv = av + mik(k2, ph) - (nu * ksq) * v;
     const Cx<T> pw = aw + mik(k3, ph) - (nu * ksq) * w;
@@ -442,7 +626,7 @@ struct PhysPLQL {
 // is stored and the RHS is formed later (dynamic tau-model).
 template <typename T>
 struct EpiPLQL {
-  static constexpr int F_IN = 9;
+  static constexpr int F_IN = 9, NACC = 3;
   __host__ double io_bytes(long long npts) const {
     if (plql_out) return (double)sizeof(Cx<T>) * npts * 3;
     return io.bytes(npts, 3) + (double)sizeof(Cx<T>) * npts * 3;  // + PL_p read
@@ -455,31 +639,45 @@ struct EpiPLQL {
   T Om1, Om2, Om3;
   int ny1, ny2, ny3;
   Cx<T>* plql_out;  // if non-null: store PLQL and stop
-  __device__ void operator()(int i1, int i2, int i3, const Cx<T>* P) const {
+  // products u_j (PL_q)_i, 3 j + i: k_j (u_j q_i + u_i q_j) in sum i
+  __device__ __forceinline__ KTabs<T> ktabs() const { return k; }
+  template <int R>
+  __device__ __forceinline__ void acc(int f, const T* k1, T k2, T k3, const Cx<T>* v, Cx<T> (*D)[R]) const {
+    const int j = f / 3, i = f - 3 * j;
+    if (i == j) acc_sym<R>(i, k1, k2, k3, v, D);
+    acc_sym<R>(i == j ? i : i + j + 2, k1, k2, k3, v, D);
+  }
+  __device__ void operator()(int i1, int i2, int i3, const Cx<T>* P) const { epi_point<T>(*this, i1, i2, i3, P); }
+  struct In {
+    StateIn<T, 3> st;
+    Cx<T> pl[3];
+  };
+  __device__ __forceinline__ In ld(int i1, int i2, int i3) const {
+    In in{};
+    if (plql_out) return in;
+    const long long s = io.sidx(i1, i2, i3);
+    in.st.load(io, s);
+#pragma unroll
+    for (int f = 0; f < 3; ++f) in.pl[f] = PLp[f * io.fstride + s];
+    return in;
+  }
+  __device__ __forceinline__ void fin(int i1, int i2, int i3, const Cx<T>* D, const In& in) const {
     const long long s = io.sidx(i1, i2, i3);
     const T k1 = (T)k.k1[i1], k2 = (T)k.k2[i2], k3 = (T)k.k3[i3];
     T ksq, ksqi;
     ksq_pair(k1, k2, k3, ksq, ksqi);
-    const Cx<T> upu = P[0], upv = P[1], upw = P[2], vpu = P[3], vpv = P[4], vpw = P[5], wpu = P[6],
-                wpv = P[7], wpw = P[8];
-    const Cx<T> pt = ((T)2 * ksqi) * ((k1 * k1) * upu + (k2 * k2) * vpv + (k3 * k3) * wpw +
-                                      (k1 * k2) * (upv + vpu) + (k1 * k3) * (upw + wpu) + (k2 * k3) * (vpw + wpv));
-    const Cx<T> Lu = mik(k1, upu) + mik(k2, vpu) + mik(k3, wpu) + mik(k1, upu) + mik(k2, upv) + mik(k3, upw) +
-                     pik(k1, pt);
-    const Cx<T> Lv = mik(k1, upv) + mik(k2, vpv) + mik(k3, wpv) + mik(k1, vpu) + mik(k2, vpv) + mik(k3, vpw) +
-                     pik(k2, pt);
-    const Cx<T> Lw = mik(k1, upw) + mik(k2, vpw) + mik(k3, wpw) + mik(k1, wpu) + mik(k2, wpv) + mik(k3, wpw) +
-                     pik(k3, pt);
+    const Cx<T> pt = ksqi * (k1 * D[0] + k2 * D[1] + k3 * D[2]);
+    const Cx<T> Lu = mul_mi(D[0]) + pik(k1, pt), Lv = mul_mi(D[1]) + pik(k2, pt), Lw = mul_mi(D[2]) + pik(k3, pt);
     if (plql_out) {
       plql_out[s] = Lu;
       plql_out[io.fstride + s] = Lv;
       plql_out[2 * io.fstride + s] = Lw;
       return;
     }
-    Cx<T> u = io.Q[s], v = io.Q[io.fstride + s], w = io.Q[2 * io.fstride + s];
+    Cx<T> u = in.st.q[0], v = in.st.q[1], w = in.st.q[2];
     if (i1 == ny1 || i2 == ny2 || i3 == ny3) u = v = w = mk<T>(0, 0);
     const Cx<T> w0u = coef * Lu, w0v = coef * Lv, w0w = coef * Lw;
-    Cx<T> ru = PLp[s] + w0u, rv = PLp[io.fstride + s] + w0v, rw = PLp[2 * io.fstride + s] + w0w;
+    Cx<T> ru = in.pl[0] + w0u, rv = in.pl[1] + w0v, rw = in.pl[2] + w0w;
     if (rotate) {
       ru = ru + (T)2 * (Om3 * v - Om2 * w);
       rv = rv + (T)2 * (Om1 * w - Om3 * u);
@@ -495,9 +693,9 @@ struct EpiPLQL {
       io.read_out[io.fstride + s] = v;
       io.read_out[2 * io.fstride + s] = w;
     }
-    io.finish(s, 0, ru);
-    io.finish(s, 1, rv);
-    io.finish(s, 2, rw);
+    io.finish(s, 0, ru, in.st.o[0]);
+    io.finish(s, 1, rv, in.st.o[1]);
+    io.finish(s, 2, rw, in.st.o[2]);
   }
 };
 
@@ -555,25 +753,26 @@ struct EpiPLQLFull {
 // p = the 2/3-rule set, L evaluated without aliasing on the 2x grid, QL its q
 // part, PLQL the linearisation of L about (u, B) in the direction QL.
 
-// Nonlinear MHD operator from the nine product spectra (u_iu_j - B_iB_j for
-// 11,22,33,12,13,23, then u x B): momentum with the pressure projection and the
-// induction curl, as in EpiMHD without dissipation, forcing and mask.
+// Nonlinear MHD operator from the six sums of the nine product spectra
+// (acc_mhd): momentum with the pressure projection and the induction curl, as
+// in EpiMHD without dissipation, forcing and mask.
 template <typename T>
-__device__ __forceinline__ void mhd_nonlinear(T k1, T k2, T k3, T ksqi, const Cx<T>* P, Cx<T>* r) {
-  const Cx<T> ph = ksqi * ((-k1 * k1) * P[0] - (k2 * k2) * P[1] - (k3 * k3) * P[2] - ((T)2 * k1 * k2) * P[3] -
-                           ((T)2 * k1 * k3) * P[4] - ((T)2 * k2 * k3) * P[5]);
-  r[0] = mik(k1, P[0]) + mik(k2, P[3]) + mik(k3, P[4]) + mik(k1, ph);
-  r[1] = mik(k1, P[3]) + mik(k2, P[1]) + mik(k3, P[5]) + mik(k2, ph);
-  r[2] = mik(k1, P[4]) + mik(k2, P[5]) + mik(k3, P[2]) + mik(k3, ph);
-  r[3] = pik(k2, P[8]) - pik(k3, P[7]);
-  r[4] = pik(k3, P[6]) - pik(k1, P[8]);
-  r[5] = pik(k1, P[7]) - pik(k2, P[6]);
+__device__ __forceinline__ void mhd_nonlinear(T k1, T k2, T k3, const Cx<T>* A, Cx<T>* r) {
+  T ksq, ksqi;
+  ksq_pair(k1, k2, k3, ksq, ksqi);
+  const Cx<T> ph = (-ksqi) * (k1 * A[0] + k2 * A[1] + k3 * A[2]);
+  r[0] = mul_mi(A[0]) + mik(k1, ph);
+  r[1] = mul_mi(A[1]) + mik(k2, ph);
+  r[2] = mul_mi(A[2]) + mik(k3, ph);
+  r[3] = mul_i(A[3]);
+  r[4] = mul_i(A[4]);
+  r[5] = mul_i(A[5]);
 }
 
 // 2x-grid epilogue: QL = L(u, B) on the modes outside the 2/3-rule set.
 template <typename T>
 struct EpiMHDQ {
-  static constexpr int F_IN = 9;
+  static constexpr int F_IN = 9, NACC = 6;
   __host__ double io_bytes(long long npts) const { return (double)sizeof(Cx<T>) * 6 * npts; }
   KTabs<T> kf;                 // 2x-grid wavenumbers
   const double *m1, *m2, *m3;  // N-grid 2/3-rule masks
@@ -582,7 +781,15 @@ struct EpiMHDQ {
   long long fstride_2x;
   T scale;  // 2x-grid transform sums -> N-grid convention (1/8)
   Cx<T>* QL;  // (6, 2N1, 2N2, N3+1)
-  __device__ void operator()(int i1, int i2, int i3, const Cx<T>* P) const {
+  __device__ __forceinline__ KTabs<T> ktabs() const { return kf; }
+  template <int R>
+  __device__ __forceinline__ void acc(int f, const T* k1, T k2, T k3, const Cx<T>* v, Cx<T> (*A)[R]) const {
+    acc_mhd<R>(f, k1, k2, k3, v, A);
+  }
+  __device__ void operator()(int i1, int i2, int i3, const Cx<T>* P) const { epi_point<T>(*this, i1, i2, i3, P); }
+  struct In {};
+  __device__ __forceinline__ In ld(int, int, int) const { return In{}; }
+  __device__ __forceinline__ void fin(int i1, int i2, int i3, const Cx<T>* A, const In&) const {
     const int n1 = unpad2x_idx(i1, N1), n2 = unpad2x_idx(i2, N2);
     const bool resolved = n1 >= 0 && n2 >= 0 && i3 < n3h && m1[n1] * m2[n2] * m3[i3] != 0.0;
     const long long s = ((long long)i1 * nf2 + i2) * nf3h + i3;
@@ -591,16 +798,10 @@ struct EpiMHDQ {
 #pragma unroll
       for (int f = 0; f < 6; ++f) r[f] = mk<T>(0, 0);
     } else {
-      Cx<T> Ps[9];
-#pragma unroll
-      for (int m = 0; m < 9; ++m) Ps[m] = scale * P[m];
-      const T k1 = (T)kf.k1[i1], k2 = (T)kf.k2[i2], k3 = (T)kf.k3[i3];
-      T ksq, ksqi;
-      ksq_pair(k1, k2, k3, ksq, ksqi);
-      mhd_nonlinear(k1, k2, k3, ksqi, Ps, r);
+      mhd_nonlinear((T)kf.k1[i1], (T)kf.k2[i2], (T)kf.k3[i3], A, r);
     }
 #pragma unroll
-    for (int f = 0; f < 6; ++f) QL[f * fstride_2x + s] = r[f];
+    for (int f = 0; f < 6; ++f) QL[f * fstride_2x + s] = scale * r[f];
   }
 };
 
@@ -628,7 +829,7 @@ struct PhysMHDLin {
 // RK stage update.
 template <typename T>
 struct EpiMHDT {
-  static constexpr int F_IN = 9;
+  static constexpr int F_IN = 9, NACC = 6;
   __host__ double io_bytes(long long npts) const {
     return io.bytes(npts, 6) + (double)sizeof(Cx<T>) * 6 * npts + (w0_out ? (double)sizeof(Cx<T>) * 6 * npts : 0.0);
   }
@@ -638,20 +839,54 @@ struct EpiMHDT {
   const Cx<T>* rhs6;  // plain MHD RHS (6 fields)
   T coef;             // Ct t / 8 (2x-grid sums -> N-grid convention)
   Cx<T>* w0_out;      // memory term (6 fields) or null
-  __device__ void operator()(int i1, int i2, int i3, const Cx<T>* P) const {
+  __device__ __forceinline__ KTabs<T> ktabs() const { return k; }
+  template <int R>
+  __device__ __forceinline__ void acc(int f, const T* k1, T k2, T k3, const Cx<T>* v, Cx<T> (*A)[R]) const {
+    acc_mhd<R>(f, k1, k2, k3, v, A);
+  }
+  __device__ void operator()(int i1, int i2, int i3, const Cx<T>* P) const { epi_point<T>(*this, i1, i2, i3, P); }
+  struct In {
+    typename StepIO<T>::Old o[6];
+    Cx<T> r[6];
+  };
+  __device__ __forceinline__ In ld(int i1, int i2, int i3) const {
+    const long long s = io.sidx(i1, i2, i3);
+    In in;
+#pragma unroll
+    for (int f = 0; f < 6; ++f) {
+      in.r[f] = rhs6[f * io.fstride + s];
+      in.o[f] = io.fetch(s, f, io.mode == kStage1 ? io.Q[f * io.fstride + s] : mk<T>(0, 0));
+    }
+    return in;
+  }
+  __device__ __forceinline__ void fin(int i1, int i2, int i3, const Cx<T>* A, const In& in) const {
     const long long s = io.sidx(i1, i2, i3);
     const T D = (T)(m1[i1] * m2[i2] * m3[i3]);
-    const T k1 = (T)k.k1[i1], k2 = (T)k.k2[i2], k3 = (T)k.k3[i3];
-    T ksq, ksqi;
-    ksq_pair(k1, k2, k3, ksq, ksqi);
     Cx<T> r[6];
-    mhd_nonlinear(k1, k2, k3, ksqi, P, r);
+    mhd_nonlinear((T)k.k1[i1], (T)k.k2[i2], (T)k.k3[i3], A, r);
 #pragma unroll
     for (int f = 0; f < 6; ++f) {
       const Cx<T> w0 = (coef * D) * r[f];
       if (w0_out) w0_out[f * io.fstride + s] = w0;
-      io.finish(s, f, rhs6[f * io.fstride + s] + w0);
+      io.finish(s, f, in.r[f] + w0, in.o[f]);
     }
+  }
+};
+
+// Stores the F product spectra.
+template <typename T, int F>
+struct EpiStore {
+  static constexpr int F_IN = F, NACC = 0;  // no sums: put() stores each field's modes as they come
+  Cx<T>* out;
+  long long fstride;
+  int n2, n3h;
+  __host__ double io_bytes(long long npts) const { return (double)sizeof(Cx<T>) * npts * F; }
+  __device__ __forceinline__ void put(int f, int i1, int i2, int i3, Cx<T> v) const {
+    out[f * fstride + ((long long)i1 * n2 + i2) * n3h + i3] = v;
+  }
+  __device__ void operator()(int i1, int i2, int i3, const Cx<T>* P) const {
+#pragma unroll
+    for (int m = 0; m < F; ++m) put(m, i1, i2, i3, P[m]);
   }
 };
 

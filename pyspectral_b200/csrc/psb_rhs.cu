@@ -766,20 +766,6 @@ int run_mhd_tmodel(psb_ctx* c, StepIO<T> io, const psb_params* p) {
 // part).  The Smagorinsky epilogue then runs on the stored u spectra with
 // tau = -2 Cs^2 Delta^2 (|S| S)^ read from the device: no host round trip.
 // ---------------------------------------------------------------------------
-template <typename T, int F>
-struct EpiStore {
-  static constexpr int F_IN = F;
-  Cx<T>* out;
-  long long fstride;
-  int n2, n3h;
-  __host__ double io_bytes(long long npts) const { return (double)sizeof(Cx<T>) * npts * F; }
-  __device__ void operator()(int i1, int i2, int i3, const Cx<T>* P) const {
-    const long long s = ((long long)i1 * n2 + i2) * n3h + i3;
-#pragma unroll
-    for (int m = 0; m < F; ++m) out[m * fstride + s] = P[m];
-  }
-};
-
 // myFilter(uhat, kL) (src/Classes.py:1271-1279) on load, then the strain of PreStrain
 template <typename T>
 struct PreStrainFiltered {
@@ -1803,9 +1789,14 @@ int rhs_dispatch(psb_ctx* c, int closure, StepIO<T> io, const psb_params* p, dou
     case PSB_SMAG: {
       const bool smag = closure == PSB_SMAG;
       if (smag) {
+        const double csd2 = 0.16 * c->Delta * 0.16 * c->Delta;
+        if (!io.w0_out)
+          return run_ns32<T>(c, Qin, PreStrain<T>{}, PhysSmag<T>{(T)csd2},
+                             EpiSmagStep<T>{io, ktabs<T>(c->kx, c->ky, c->kz), (T)p->nu, p->rotate, (T)p->Om1,
+                                            (T)p->Om2, (T)p->Om3},
+                             ts);
         EpiNS<T, true> epi{io, ktabs<T>(c->kx, c->ky, c->kz), (T)p->nu, p->rotate, (T)p->Om1, (T)p->Om2,
                            (T)p->Om3, 0, c->N1 / 2, c->N2 / 2, c->N3 / 2};
-        const double csd2 = 0.16 * c->Delta * 0.16 * c->Delta;
         return run_ns32<T>(c, Qin, PreStrain<T>{}, PhysSmag<T>{(T)csd2}, epi, ts);
       }
       EpiNS<T, false> epi{io, ktabs<T>(c->kx, c->ky, c->kz), (T)p->nu, p->rotate, (T)p->Om1, (T)p->Om2,
@@ -2002,7 +1993,12 @@ size_t pass_smem(const TuneDims& t, int k, int tile) {
 // Untuned shape of axis pass k (x-inverse, y-inverse, y-forward, x-forward).
 template <typename T>
 void default_pass_shape(psb_ctx* c, const TuneDims& t, int k, psb_pass_shape& sh) {
-  const int nouter = k == 0 || k == 4 ? c->N2 : (k == 1 ? t.Gy * t.Ls[0] : t.Fo * t.Ls[0]);
+  if (k == 4) {
+    default_x_shape<T>(c, t.Ls[4], c->N3 / 2, t.Fs[4], c->N2, true, sh.tile, sh.plan);
+    sh.reg = has_reg_x(t.Ls[4]);
+    return;
+  }
+  const int nouter = k == 0 ? c->N2 : (k == 1 ? t.Gy * t.Ls[0] : t.Fo * t.Ls[0]);
   const bool reg = k == 0 ? t.regx : (k == 1 ? t.regy : k == 3);
   default_axis_shape<T>(c, t.Ls[k], c->N3 / 2, t.Fs[k], nouter, reg, sh.tile, sh.plan);
   sh.reg = reg && has_reg_axis(t.Ls[k]);
@@ -2066,7 +2062,7 @@ int tune_rhs(psb_ctx* c, int closure, const void* state, const psb_params* p) {
     psb_pass_shape& cur = c->tuned[closure].pass[k];
     const psb_pass_shape inc = cur;
     // a register pass has one shape (the runtime-schedule shapes of its length are slower throughout)
-    if (k == 2 ? td.zP > 0 : is_reg_axis(inc.plan)) continue;
+    if (inc.reg) continue;
     float base = 0.f;
     if ((status = time_pass(k, 6, &base)) != PSB_OK) break;
     std::vector<int> tiles;
@@ -2127,6 +2123,8 @@ int set_shape(psb_ctx* c, int closure, int k, int tile, const int* radices, int 
   FFTPlan rp = q;
   bool reg_shape = (k == 0 ? td.regx : (k == 1 ? td.regy : k == 3)) && nrad == 2 && reg_axis_plan(L, rp) &&
                    radices[0] == rp.radix[0] && radices[1] == rp.radix[1];
+  if (k == 4)
+    reg_shape = reg_x_plan(L, rp) && nrad == rp.npass && std::equal(radices, radices + nrad, rp.radix);
   if (k == 2)
     reg_shape = td.zP > 0 && nrad == 3 && std::equal(radices, radices + 3, td.zplan.radix) && tile >= 1 &&
                 tile <= 128;
@@ -2188,22 +2186,8 @@ template int sgs_dns_run<float>(psb_ctx*, const void*, void*, void*);
 
 // The six dealiased product spectra (uuhat.. of src/RHSfunctions.py:18-23).
 template <typename T>
-struct EpiProducts {
-  static constexpr int F_IN = 6;
-  Cx<T>* out;
-  long long fstride;
-  int n2, n3h;
-  __host__ double io_bytes(long long npts) const { return (double)sizeof(Cx<T>) * npts * 6; }
-  __device__ void operator()(int i1, int i2, int i3, const Cx<T>* P) const {
-    const long long s = ((long long)i1 * n2 + i2) * n3h + i3;
-#pragma unroll
-    for (int m = 0; m < 6; ++m) out[m * fstride + s] = P[m];
-  }
-};
-
-template <typename T>
 int products_run(psb_ctx* c, const void* fields, void* out6) {
-  EpiProducts<T> epi{reinterpret_cast<Cx<T>*>(out6), (long long)c->N1 * c->N2 * c->N3h, c->N2, c->N3h};
+  EpiStore<T, 6> epi{reinterpret_cast<Cx<T>*>(out6), (long long)c->N1 * c->N2 * c->N3h, c->N2, c->N3h};
   return run_ns32<T>(c, reinterpret_cast<const Cx<T>*>(fields), PreCopyN<T, 3>{}, PhysProducts<T>{}, epi);
 }
 template int products_run<double>(psb_ctx*, const void*, void*);
@@ -2212,7 +2196,7 @@ template int products_run<float>(psb_ctx*, const void*, void*);
 // the six products of Gf u (the sharp-cutoff filtered field; transfer of the resolved scales)
 template <typename T>
 int products_filtered_run(psb_ctx* c, const void* fields, void* out6) {
-  EpiProducts<T> epi{reinterpret_cast<Cx<T>*>(out6), (long long)c->N1 * c->N2 * c->N3h, c->N2, c->N3h};
+  EpiStore<T, 6> epi{reinterpret_cast<Cx<T>*>(out6), (long long)c->N1 * c->N2 * c->N3h, c->N2, c->N3h};
   return run_ns32<T>(c, reinterpret_cast<const Cx<T>*>(fields), PreMask3<T>{c->gx, c->gy, c->gz},
                      PhysProducts<T>{}, epi);
 }

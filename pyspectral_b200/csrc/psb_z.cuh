@@ -23,9 +23,11 @@ int launch_reg_zp(psb_ctx* c, const psb::ZArgs<T>& z, const Phys& phys, const ch
   const size_t smem = psb::z_reg_smem<Phys, T, A, B>(P);
   auto k = psb::zreg_kernel<T, Phys, A, B, P32>;
   set_smem(k, smem);
-  const long long g = persistent_grid(k, smem, (z.npencils + P - 1) / P * psb::Mid<Phys>::JOBS, psb::ZPlan<T, A, B>::NT);
+  const long long g = persistent_grid(k, smem, (z.npencils + P - 1) / P * psb::Mid<Phys>::JOBS,
+                                      psb::ZPlan<T, A, B>::NT);
   LaunchScope scope(c, what, bytes);
-  launch_pdl(k, dim3((unsigned)g), psb::ZPlan<T, A, B>::NT, smem, c->stream, z, phys, P);
+  c->serial_next = bytes > kPdlBytes;
+  launch_pdl_if(!c->serial_next, k, dim3((unsigned)g), psb::ZPlan<T, A, B>::NT, smem, c->stream, z, phys, P);
   return launch_ok(c, what);
 }
 
@@ -49,9 +51,11 @@ int launch_reg_z_batch(psb_ctx* c, const psb::ZArgs<T>* args, const Phys* phys, 
   const size_t smem = psb::z_reg_smem<Phys, T, A, B>(P);
   auto k = psb::zreg_batch<T, Phys, A, B>;
   set_smem(k, smem);
-  const long long g = persistent_grid(k, smem, (npencils + P - 1) / P * psb::Mid<Phys>::JOBS * runs, psb::ZPlan<T, A, B>::NT);
+  const long long g = persistent_grid(k, smem, (npencils + P - 1) / P * psb::Mid<Phys>::JOBS * runs,
+                                      psb::ZPlan<T, A, B>::NT);
   LaunchScope scope(c, what, bytes);
-  launch_pdl(k, dim3((unsigned)g), psb::ZPlan<T, A, B>::NT, smem, c->stream, args, phys, runs, P);
+  c->serial_next = bytes > kPdlBytes;
+  launch_pdl_if(!c->serial_next, k, dim3((unsigned)g), psb::ZPlan<T, A, B>::NT, smem, c->stream, args, phys, runs, P);
   return launch_ok(c, what);
 }
 
