@@ -550,7 +550,7 @@ int launch_z(psb_ctx* c, psb::ZArgs<T> z, Phys phys, const char* what, double ex
   double bytes = extra_bytes + (double)esz * z.npencils * Phys::F_OUT * z.out_kz;
   // a field formed as d/dz of another input re-reads that input's line: no new bytes
   for (int f = 0; f < Phys::F_IN; ++f)
-    if (!z.dz[f]) bytes += (double)esz * z.npencils * z.in_kz[f];
+    if (!z.dz[f] || z.in2[f]) bytes += (double)esz * z.npencils * z.in_kz[f];
   // the register z pass of this length (psb_zreg.cuh), where there is one; a tuned shape applies to
   // the staged one
   if constexpr (z_registered<Phys>::value)
@@ -695,6 +695,8 @@ void set_z_inputs(psb::ZArgs<T>& z, const Cx<T>* B, long long fsP, int Kz, const
     z.in_pstride[f] = Kz;
     z.in_kz[f] = Kz;
     z.dz[f] = der ? 1 : 0;
+    if constexpr (psb::pre_has_zsrc2<Pre>::value)
+      if (Pre::zsrc2(f) >= 0) z.in2[f] = B + Pre::zsrc2(f) * fsP;
   }
   z.k3 = k3;
 }

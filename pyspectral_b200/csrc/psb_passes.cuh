@@ -144,11 +144,12 @@ struct AxisArgs {
 enum FieldKind : unsigned char {
   kCopy = 0,   // s[a]
   kIkRow = 1,  // i k_row s[a]
+  kIkMean = 2, // (i k_row s[a] + s[b]) / 2
 };
 template <typename T>
 struct FieldTab {
   int nf = 0;
-  unsigned char kind[12] = {}, sa[12] = {};
+  unsigned char kind[12] = {}, sa[12] = {}, sb[12] = {};
   // optional separable factors (m1[row] m2[outer] m3[col]), applied in this order
   const double *m1 = nullptr, *m2 = nullptr, *m3 = nullptr;
   const double *f1 = nullptr, *f2 = nullptr, *f3 = nullptr;
@@ -385,6 +386,7 @@ struct ZArgs {
   const Cx<T>* tw;
   unsigned char dz[kMaxZFields];  // 1: input field f enters as i*k3 times the stored spectrum (a d/dz)
   const double* k3;               // k3 wavenumbers of the stored entries (for dz)
+  const Cx<T>* in2[kMaxZFields];  // non-null: field f is the mean of what in[f] gives and this stored spectrum
 };
 
 // Pre functors may leave derivatives along z to the z-pass: Pre::Z_DERIVED
@@ -397,6 +399,15 @@ struct pre_z_derived {
 template <class P>
 struct pre_z_derived<P, decltype((void)P::Z_DERIVED, void())> {
   static constexpr int value = P::Z_DERIVED;
+};
+// Pre::zsrc2(f): the stored field whose mean with that is input f, or -1.
+template <class P, class = void>
+struct pre_has_zsrc2 {
+  static constexpr bool value = false;
+};
+template <class P>
+struct pre_has_zsrc2<P, decltype((void)P::zsrc2(0), void())> {
+  static constexpr bool value = true;
 };
 // Fields after the y-inverse pass (Pre::F_B; default: the x pass's F_DST) and
 // the y-inverse pass's own Pre (Pre::YPass; default: a copy).
@@ -540,7 +551,7 @@ __device__ __forceinline__ void zpass_tile(const ZArgs<T>& a, const Phys& phys, 
       constexpr int U = 4;
       const int hp = P >> 1, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
       for (int cb = threadIdx.x >> 5; cb < nin; cb += U * nw) {
-        const Cx<T>* src[U];
+        const Cx<T>*src[U], *src2[U];
         long long ps[U];
         int kz[U];
         bool oka[U], okb[U], dz[U];
@@ -556,6 +567,7 @@ __device__ __forceinline__ void zpass_tile(const ZArgs<T>& a, const Phys& phys, 
           okb[u] = pa + 1 < a.npencils;
           ps[u] = a.in_pstride[f];
           src[u] = a.in[f] + (oka[u] ? pa * ps[u] : 0);
+          src2[u] = a.in2[f] ? a.in2[f] + (oka[u] ? pa * ps[u] : 0) : nullptr;
           dz[u] = c < nin && a.dz[f] != 0;
           anydz |= dz[u];
           kzmax = max(kzmax, kz[u]);
@@ -577,6 +589,10 @@ __device__ __forceinline__ void zpass_tile(const ZArgs<T>& a, const Phys& phys, 
             if (dz[u]) {
               va = mk<T>(-kk * va.y, kk * va.x);
               vb = mk<T>(-kk * vb.y, kk * vb.x);
+            }
+            if (src2[u]) {
+              va = (T)0.5 * (va + (oka[u] ? src2[u][k] : zero));
+              vb = (T)0.5 * (vb + (okb[u] ? src2[u][ps[u] + k] : zero));
             }
             Cx<T>* Z = X + (size_t)(cb + u * nw) * LS;
             if (k == 0 || k == half) {
@@ -612,6 +628,7 @@ __device__ __forceinline__ void zpass_tile(const ZArgs<T>& a, const Phys& phys, 
           const T kk = (T)a.k3[k];
           v = mk<T>(-kk * v.y, kk * v.x);
         }
+        if (a.in2[f]) v = (T)0.5 * (v + a.in2[f][pen * a.in_pstride[f] + k]);
         if (part == 0) A = v; else B = v;
       }
       Cx<T>* Z = X + (size_t)c * LS;

@@ -131,23 +131,66 @@ struct PreCopyN {
   __host__ FieldTab<T> fields() const { return copy_fields<T>(F); }
 };
 
-// (u,v,w) -> (u,v,w,S11,S22,S33,S12,S13,S23), S_ij = (i/2)(k_j u_i + k_i u_j)
-// (PySpectral/src/RHSfunctions.py:174-179)
+// The strain S_ij = (i/2)(k_j u_i + k_i u_j) (PySpectral/src/RHSfunctions.py:174-179)
+// is formed as late as its derivatives allow, so that the passes carry fewer
+// fields than the nine the z pass needs: the x pass u and i k1 u (6), the y pass
+// (u, v, w, S11, S22, S12, dw/dx, dw/dy) (8), and the z pass completes
+// S33 = i k3 w, S13 = (i k3 u + dw/dx)/2 and S23 = (i k3 v + dw/dy)/2 on load.
 template <typename T>
-struct PreStrain {
-  static constexpr int F_SRC = 3, F_DST = 9;
-  __device__ void operator()(int i, int o, int c, const AxisArgs<T>& a, const Cx<T>* s, Cx<T>* d) const {
-    const T k1 = (T)a.k_row[i], k2 = (T)a.k_outer[o], k3 = (T)a.k_col[c];
+struct PreYStrain {
+  static constexpr int F_SRC = 6, F_DST = 8, GROUPS = 1, IN_FIELDS = 1, OUT_FIELDS = 1;
+  __host__ FieldTab<T> fields() const {
+    const unsigned char sa[8] = {0, 1, 2, 3, 1, 0, 5, 2};
+    const unsigned char kind[8] = {kCopy, kCopy, kCopy, kCopy, kIkRow, kIkMean, kCopy, kIkRow};
+    FieldTab<T> t;
+    t.nf = 8;
+    for (int g = 0; g < 8; ++g) {
+      t.sa[g] = sa[g];
+      t.kind[g] = kind[g];
+    }
+    t.sb[5] = 4;
+    return t;
+  }
+  __device__ void operator()(int i, int, int, const AxisArgs<T>& a, const Cx<T>* s, Cx<T>* d) const {
+    const T k2 = (T)a.k_row[i];
     d[0] = s[0];
     d[1] = s[1];
     d[2] = s[2];
-    d[3] = pik(k1, s[0]);
+    d[3] = s[3];
     d[4] = pik(k2, s[1]);
-    d[5] = pik(k3, s[2]);
-    d[6] = (T)0.5 * (pik(k2, s[0]) + pik(k1, s[1]));
-    d[7] = (T)0.5 * (pik(k3, s[0]) + pik(k1, s[2]));
-    d[8] = (T)0.5 * (pik(k3, s[1]) + pik(k2, s[2]));
+    d[5] = (T)0.5 * (pik(k2, s[0]) + s[4]);
+    d[6] = s[5];
+    d[7] = pik(k2, s[2]);
   }
+};
+template <typename T>
+struct PreStrain {
+  static constexpr int F_SRC = 3, F_DST = 6, F_B = 8, Z_DERIVED = 1;
+  using YPass = PreYStrain<T>;
+  __host__ FieldTab<T> fields() const {
+    FieldTab<T> t;
+    t.nf = 6;
+    for (int g = 0; g < 6; ++g) {
+      t.sa[g] = (unsigned char)(g % 3);
+      t.kind[g] = g < 3 ? kCopy : kIkRow;
+    }
+    return t;
+  }
+  __device__ void operator()(int i, int, int, const AxisArgs<T>& a, const Cx<T>* s, Cx<T>* d) const {
+    const T k1 = (T)a.k_row[i];
+#pragma unroll
+    for (int f = 0; f < 3; ++f) {
+      d[f] = s[f];
+      d[3 + f] = pik(k1, s[f]);
+    }
+  }
+  // z-pass inputs u, v, w, S11, S22, S33, S12, S13, S23
+  __host__ static void zsrc(int f, int& src, bool& der) {
+    const int s[9] = {0, 1, 2, 3, 4, 2, 5, 0, 1};
+    src = s[f];
+    der = f == 5 || f >= 7;
+  }
+  __host__ static int zsrc2(int f) { return f < 7 ? -1 : f - 1; }
 };
 
 // u_i u_j in physical space (PySpectral/src/RHSfunctions.py:18-23)

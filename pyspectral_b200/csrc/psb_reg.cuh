@@ -91,12 +91,20 @@ __device__ __forceinline__ void axis_reg_body(const AxisArgs<T>& a, const FieldT
         v[s] = (i >= 0 ? (T)(ft.f1[i] * mc * m3) : (T)0) * v[s];
       }
     }
-    if (ft.kind[g] == kIkRow) {
+    if (ft.kind[g] != kCopy) {
 #pragma unroll
       for (int s = 0; s < A; ++s) {
         const int i = row_of(a.in_map, j + B * s, a.in_rows);
         const T k = i >= 0 ? (T)a.k_row[i] : (T)0;
         v[s] = mk<T>(-k * v[s].y, k * v[s].x);
+      }
+    }
+    if (ft.kind[g] == kIkMean) {
+      const Cx<T>* src2 = src + (ft.sb[g] - ft.sa[g]) * a.in_fstride;
+#pragma unroll
+      for (int s = 0; s < A; ++s) {
+        const int i = row_of(a.in_map, j + B * s, a.in_rows);
+        v[s] = (T)0.5 * (v[s] + ((ok && i >= 0) ? src2[(long long)i * a.in_rstride] : zero));
       }
     }
     small_dft<T, A, INV>(v);

@@ -768,13 +768,20 @@ int run_mhd_tmodel(psb_ctx* c, StepIO<T> io, const psb_params* p) {
 // ---------------------------------------------------------------------------
 // myFilter(uhat, kL) (src/Classes.py:1271-1279) on load, then the strain of PreStrain
 template <typename T>
-struct PreStrainFiltered {
-  static constexpr int F_SRC = 3, F_DST = 9;
+struct PreStrainFiltered : PreStrain<T> {
   const double *g1, *g2, *g3;
+  PreStrainFiltered(const double* a, const double* b, const double* c) : g1(a), g2(b), g3(c) {}
+  __host__ FieldTab<T> fields() const {
+    FieldTab<T> t = PreStrain<T>::fields();
+    t.m1 = g1;
+    t.m2 = g2;
+    t.m3 = g3;
+    return t;
+  }
   __device__ void operator()(int i, int o, int cc, const AxisArgs<T>& a, const Cx<T>* s, Cx<T>* d) const {
     const T g = (T)(g1[i] * g2[o] * g3[cc]);
     const Cx<T> f[3] = {g * s[0], g * s[1], g * s[2]};
-    PreStrain<T>{}(i, o, cc, a, f, d);
+    PreStrain<T>::operator()(i, o, cc, a, f, d);
   }
 };
 
@@ -1718,7 +1725,7 @@ int dsmag_rhs(psb_ctx* c, StepIO<T> io, const psb_params* p, const psb_tuned* ts
   EpiStore<T, 12> sa{A, fs, N2, N3h}, sb{B, fs, N2, N3h};
   const PhysSmag<T> ss{(T)-0.5};  // -2 (-1/2) |S| S_ij = |S| S_ij
   PSB_TRY(run_ns32<T>(c, Qin, PreStrain<T>{}, ss, sa, ts));
-  PSB_TRY(run_ns32<T>(c, Qin, PreStrainFiltered<T>{g, g + N1, g + N1 + N2}, ss, sb, ts));
+  PSB_TRY(run_ns32<T>(c, Qin, PreStrainFiltered<T>(g, g + N1, g + N1 + N2), ss, sb, ts));
   if (!Qin) return PSB_OK;  // allocation only
   const double d2 = -2.0 * c->Delta * c->Delta;
   {
@@ -1932,7 +1939,6 @@ bool plan_is_wide(const FFTPlan& p) {
 // Fy / Gy: lines per column and outer groups of the y-inverse pass
 struct TuneDims {
   int Fi, Fb, Fz, Fo, maxppc, defppc, Fy = 1, Gy;
-  bool regx = true, regy = true;  // the x- / y-inverse pass has a register form
   size_t zextra = 0;
   int Ls[5], Fs[5];
   int zP = 0;  // the register z pass's pencils per CTA and plan (0: none at this length)
@@ -1947,8 +1953,10 @@ TuneDims tune_dims(psb_ctx* c, int closure, int act, int hidden) {
     t.Fz = PhysProducts<T>::F_IN;
     t.defppc = phys_default_ppc<PhysProducts<T>>::value;
   } else if (closure == PSB_SMAG) {
-    t.Fi = t.Fb = t.Gy = 9, t.Fo = 12, t.maxppc = phys_max_ppc<PhysSmag<T>>::value;
-    t.regx = psb::pre_has_fields<PreStrain<T>>::value;
+    t.Fi = PreStrain<T>::F_DST, t.Fb = pre_b_fields<PreStrain<T>>::value, t.Fo = 12;
+    t.Fy = PreYStrain<T>::F_DST;
+    t.Gy = pre_ypass<T, PreStrain<T>>::groups;
+    t.maxppc = phys_max_ppc<PhysSmag<T>>::value;
     t.Fz = PhysSmag<T>::F_IN;
     t.defppc = phys_default_ppc<PhysSmag<T>>::value;
   } else {
@@ -1999,7 +2007,7 @@ void default_pass_shape(psb_ctx* c, const TuneDims& t, int k, psb_pass_shape& sh
     return;
   }
   const int nouter = k == 0 ? c->N2 : (k == 1 ? t.Gy * t.Ls[0] : t.Fo * t.Ls[0]);
-  const bool reg = k == 0 ? t.regx : (k == 1 ? t.regy : k == 3);
+  const bool reg = k != 2 && k != 4;
   default_axis_shape<T>(c, t.Ls[k], c->N3 / 2, t.Fs[k], nouter, reg, sh.tile, sh.plan);
   sh.reg = reg && has_reg_axis(t.Ls[k]);
 }
@@ -2121,7 +2129,7 @@ int set_shape(psb_ctx* c, int closure, int k, int tile, const int* radices, int 
   q.npass = nrad;
   // the register pass's own radices name it (its tile is fixed)
   FFTPlan rp = q;
-  bool reg_shape = (k == 0 ? td.regx : (k == 1 ? td.regy : k == 3)) && nrad == 2 && reg_axis_plan(L, rp) &&
+  bool reg_shape = (k != 2 && k != 4) && nrad == 2 && reg_axis_plan(L, rp) &&
                    radices[0] == rp.radix[0] && radices[1] == rp.radix[1];
   if (k == 4)
     reg_shape = reg_x_plan(L, rp) && nrad == rp.npass && std::equal(radices, radices + nrad, rp.radix);

@@ -142,6 +142,7 @@ __device__ __forceinline__ Cx<T> had_sub(Cx<T> a, Cx<T> b, Cx<T> c) { return mk<
 // own factor when the results are stored.
 //   SLOTS        slots of the buffer
 //   HEAVY        how many more than four fields' points a thread holds (0, 1, 2)
+//   DERIV        1: some inputs are z derivatives (ZArgs::dz), 2: or means (ZArgs::in2)
 //   JOBS         independent sets of fields, each a tile of its own: job k takes
 //                fields [in0(k), in0(k+1)) to results [out0(k), out0(k+1))
 //   in(f), out(g) slot of an input / output field
@@ -153,7 +154,7 @@ struct Mid {
 // one job of every field
 template <class Phys>
 struct MidOneJob {
-  static constexpr int JOBS = 1;
+  static constexpr int JOBS = 1, DERIV = 0;
   __host__ __device__ static constexpr int in0(int k) { return k == 0 ? 0 : Phys::F_IN; }
   __host__ __device__ static constexpr int out0(int k) { return k == 0 ? 0 : Phys::F_OUT; }
 };
@@ -221,7 +222,7 @@ struct Mid<PhysProducts<T>> : MidOneJob<PhysProducts<T>> {
 template <typename T>
 struct Mid<PhysSmag<T>> {
   static constexpr bool value = true;
-  static constexpr int SLOTS = 6, JOBS = 2, HEAVY = 0;
+  static constexpr int SLOTS = 6, JOBS = 2, HEAVY = 0, DERIV = 2;
   __host__ __device__ static constexpr int in0(int k) { return k == 0 ? 0 : (k == 1 ? 3 : 9); }
   __host__ __device__ static constexpr int out0(int k) { return 6 * k; }
   __host__ __device__ static constexpr int in(int f) { return f < 3 ? f : f - 3; }
@@ -427,7 +428,7 @@ struct Mid<PhysMHDLin<T>> : MidOneJob<PhysMHDLin<T>> {
 template <typename T, int ACT, int HID>
 struct Mid<PhysLearned<T, ACT, HID>> : MidOneJob<PhysLearned<T, ACT, HID>> {
   static constexpr bool value = true;
-  static constexpr int SLOTS = 12, HEAVY = 0;
+  static constexpr int SLOTS = 12, HEAVY = 0, DERIV = 1;
   __host__ __device__ static constexpr int in(int f) { return f; }
   __host__ __device__ static constexpr int out(int g) { return 6 + g; }
 };
@@ -546,14 +547,25 @@ __device__ __forceinline__ void z_reg_tile(const ZArgs<T>& a, const Phys& phys, 
 #pragma unroll
     for (int s = 0; s < A; ++s) x[s] = (P32 ? s < NZ : B * s < kz) ? src[B * s] : zero;
     if (!P32 && col0 && kz > H) xh = src[H];
-    if (a.dz[f]) {
-      // the derivative along z of the stored field
+    if constexpr (Md::DERIV > 0) {
+      if (a.dz[f]) {
+        // the derivative along z of the stored field
 #pragma unroll
-      for (int s = 0; s < NZ; ++s) {
-        const T k = P32 || B * s < kz ? (T)a.k3[j + B * s] : (T)0;
-        x[s] = mk<T>(-k * x[s].y, k * x[s].x);
+        for (int s = 0; s < NZ; ++s) {
+          const T k = P32 || B * s < kz ? (T)a.k3[j + B * s] : (T)0;
+          x[s] = mk<T>(-k * x[s].y, k * x[s].x);
+        }
+        if (!P32 && col0 && kz > H) xh.x = -(T)a.k3[H] * xh.y;
       }
-      if (!P32 && col0 && kz > H) xh.x = -(T)a.k3[H] * xh.y;
+    }
+    if constexpr (Md::DERIV > 1) {
+      if (a.in2[f]) {
+        const Cx<T>* s2 = a.in2[f] + pen * a.in_pstride[f] + j;
+#pragma unroll
+        for (int s = 0; s < NZ; ++s)
+          if (P32 || B * s < kz) x[s] = (T)0.5 * (x[s] + s2[B * s]);
+        if (!P32 && col0 && kz > H) xh.x = (T)0.5 * (xh.x + s2[H].x);
+      }
     }
     // k = 0 and H enter with their real parts (c2r convention)
     if (col0) x[0].y = (T)0;
