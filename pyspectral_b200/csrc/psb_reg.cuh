@@ -138,16 +138,25 @@ __device__ __forceinline__ void axis_reg_body(const AxisArgs<T>& a, const FieldT
     for (int row = zlo + q; row < zhi; row += A) dst[(long long)row * a.out_rstride] = zero;
 }
 
+// CTAs per SM the registers are bounded for: the A elements of a load item and
+// about 36 (FP64: 56) more.
+template <typename T, int A>
+constexpr int axis_reg_minb() {
+  constexpr int regs = A * (int)sizeof(Cx<T>) / 4 + (sizeof(T) == 4 ? 36 : 56);
+  constexpr int b = 65536 / (regs * A * reg_cols<T>());
+  return b < 1 ? 1 : (b > 16 ? 16 : b);
+}
+
 // grid = (ceil(ncols / C), nouter, fields); block = A C threads
 template <typename T, int A, int B, bool INV>
-__global__ void __launch_bounds__(A* reg_cols<T>(), 1) axis_reg_kernel(const __grid_constant__ AxisArgs<T> a,
+__global__ void __launch_bounds__(A* reg_cols<T>(), axis_reg_minb<T, A>()) axis_reg_kernel(const __grid_constant__ AxisArgs<T> a,
                                                                     const __grid_constant__ FieldTab<T> ft) {
   axis_reg_body<T, A, B, INV>(a, ft, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 
 // Batched: grid.x = column tiles * runs (run-major); run r reads its arguments from args[r].
 template <typename T, int A, int B, bool INV>
-__global__ void __launch_bounds__(A* reg_cols<T>(), 1) axis_reg_batch(const AxisArgs<T>* __restrict__ args,
+__global__ void __launch_bounds__(A* reg_cols<T>(), axis_reg_minb<T, A>()) axis_reg_batch(const AxisArgs<T>* __restrict__ args,
                                                                    const __grid_constant__ FieldTab<T> ft) {
   const int nt = (args[0].ncols + reg_cols<T>() - 1) / reg_cols<T>();
   const int run = blockIdx.x / nt;
