@@ -664,12 +664,27 @@ struct PhysPLQL {
   }
 };
 
+// The six symmetric products u_i q_j + u_j q_i (11, 22, 33, 12, 13, 23; 2 u_i q_i
+// on the diagonal), q = PL_q: the nine products enter PLQL and its pressure term
+// in these sums only (PySpectral/src/RHSfunctions.py:338-352).
+template <typename T>
+struct PhysPLQS {
+  static constexpr int F_IN = 6, F_OUT = 6;
+  __device__ __forceinline__ void operator()(long long, int, const T* in, T* out) const {
+#pragma unroll
+    for (int i = 0; i < 3; ++i) out[i] = (T)2 * in[i] * in[3 + i];
+    out[3] = in[0] * in[4] + in[1] * in[3];
+    out[4] = in[0] * in[5] + in[2] * in[3];
+    out[5] = in[1] * in[5] + in[2] * in[4];
+  }
+};
+
 // PLQL on the N grid and the memory-closure RHS = unpad_2x(PL) + coef*PLQL
 // (PySpectral/src/RHSfunctions.py:338-358).  With coef_ptr set the PLQL field
 // is stored and the RHS is formed later (dynamic tau-model).
 template <typename T>
 struct EpiPLQL {
-  static constexpr int F_IN = 9, NACC = 3;
+  static constexpr int F_IN = 6, NACC = 3;
   __host__ double io_bytes(long long npts) const {
     if (plql_out) return (double)sizeof(Cx<T>) * npts * 3;
     return io.bytes(npts, 3) + (double)sizeof(Cx<T>) * npts * 3;  // + PL_p read
@@ -682,13 +697,10 @@ struct EpiPLQL {
   T Om1, Om2, Om3;
   int ny1, ny2, ny3;
   Cx<T>* plql_out;  // if non-null: store PLQL and stop
-  // products u_j (PL_q)_i, 3 j + i: k_j (u_j q_i + u_i q_j) in sum i
   __device__ __forceinline__ KTabs<T> ktabs() const { return k; }
   template <int R>
   __device__ __forceinline__ void acc(int f, const T* k1, T k2, T k3, const Cx<T>* v, Cx<T> (*D)[R]) const {
-    const int j = f / 3, i = f - 3 * j;
-    if (i == j) acc_sym<R>(i, k1, k2, k3, v, D);
-    acc_sym<R>(i == j ? i : i + j + 2, k1, k2, k3, v, D);
+    acc_sym<R>(f, k1, k2, k3, v, D);
   }
   __device__ void operator()(int i1, int i2, int i3, const Cx<T>* P) const { epi_point<T>(*this, i1, i2, i3, P); }
   struct In {

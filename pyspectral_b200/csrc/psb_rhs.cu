@@ -458,11 +458,12 @@ int run_pl(psb_ctx* c, const Cx<T>* Qin, const psb_params* p, const MemCfg& m, C
   return launch_epi<T>(c, e, epi, "2x x-forward+PL");
 }
 
-// Stage B: PLQL from u (B2) and PL_q (E) -> 9 products -> N-grid epilogue.
+// Stage B: PLQL from u (B2) and PL_q (E) -> products -> N-grid epilogue.
 // FULL: the products stay on the whole 2x grid (every k3 of the 2x grid, 2N2
 // rows, 2N1 rows) and the epilogue runs there (EpiPLQLFull); otherwise they
-// are truncated to the N grid (unpad_2x) on the way out.  Any epilogue of 9
-// product spectra fits (EpiPLQL, EpiStore<T, 9>, EpiPLQLFull).
+// are truncated to the N grid (unpad_2x) on the way out.  An epilogue of six
+// spectra gets the symmetric products (EpiPLQL), one of nine every product
+// (EpiStore<T, 9>, EpiPLQLFull).
 template <typename T, class Epi = EpiPLQL<T>, bool FULL = false>
 int run_plql(psb_ctx* c, const MemCfg& m, Cx<T>* B2, Cx<T>* E, Epi epi) {
   const int N1 = c->N1, N2 = c->N2, N3 = c->N3, N3h = c->N3h;
@@ -472,8 +473,12 @@ int run_plql(psb_ctx* c, const MemCfg& m, Cx<T>* B2, Cx<T>* E, Epi epi) {
   int st = PSB_OK;
   Cx<T>* A3 = scratch<T>(c, "mem.A3", (size_t)3 * F1 * F2 * F3h, &st);
   Cx<T>* B3 = scratch<T>(c, "mem.B3", (size_t)3 * F1 * F2 * F3h, &st);
-  Cx<T>* C3 = scratch<T>(c, FULL ? "mem.C3f" : "mem.C3", (size_t)9 * F1 * F2 * KO, &st);
-  Cx<T>* D3 = scratch<T>(c, FULL ? "mem.D3f" : "mem.D3", (size_t)9 * F1 * RY * KO, &st);
+  // nine products u_j q_i, or the six symmetric sums of them
+  using Phys = std::conditional_t<Epi::F_IN == 6, PhysPLQS<T>, PhysPLQL<T>>;
+  constexpr int FO = Phys::F_OUT;
+  static_assert(Epi::F_IN == FO, "phys/epi mismatch");
+  Cx<T>* C3 = scratch<T>(c, FULL ? "mem.C3f" : (FO == 6 ? "mem.C3s" : "mem.C3"), (size_t)FO * F1 * F2 * KO, &st);
+  Cx<T>* D3 = scratch<T>(c, FULL ? "mem.D3f" : (FO == 6 ? "mem.D3s" : "mem.D3"), (size_t)FO * F1 * RY * KO, &st);
   if (st != PSB_OK) return st;
   if (!B2) return PSB_OK;
   const long long fsC = (long long)F1 * F2 * F3h;
@@ -518,7 +523,7 @@ int run_plql(psb_ctx* c, const MemCfg& m, Cx<T>* B2, Cx<T>* E, Epi epi) {
     z.in_kz[3 + f] = F3h;
   }
   const long long fsO = (long long)F1 * F2 * KO;
-  for (int g = 0; g < 9; ++g) {
+  for (int g = 0; g < FO; ++g) {
     z.out[g] = C3 + g * fsO;
     z.out_pstride[g] = KO;
   }
@@ -528,7 +533,7 @@ int run_plql(psb_ctx* c, const MemCfg& m, Cx<T>* B2, Cx<T>* E, Epi epi) {
   z.fac = (T)(s2 / ((double)F1 * F2 * F3));
   z.plan = *plan_for(c, F3);
   z.tw = twiddles<T>(c);
-  PSB_TRY(launch_z<T>(c, z, PhysPLQL<T>{}, "PLQL z-products"));
+  PSB_TRY(launch_z<T>(c, z, Phys{}, "PLQL z-products"));
   AxisArgs<T> d = axis_common<T>(c, F2);
   d.in = C3;
   d.out = D3;
@@ -536,7 +541,7 @@ int run_plql(psb_ctx* c, const MemCfg& m, Cx<T>* B2, Cx<T>* E, Epi epi) {
   d.in_rstride = KO;
   d.out_ostride = (long long)RY * KO;
   d.out_rstride = KO;
-  d.nouter = 9 * F1;
+  d.nouter = FO * F1;
   d.ncols = KO;
   d.in_rows = F2;
   d.out_rows = RY;

@@ -4,4 +4,5 @@
 namespace psbh {
 using namespace psb;
 PSB_REG_Z(float, PhysPLQL<float>)
+PSB_REG_Z(float, PhysPLQS<float>)
 }  // namespace psbh

@@ -4,4 +4,5 @@
 namespace psbh {
 using namespace psb;
 PSB_REG_Z(double, PhysPLQL<double>)
+PSB_REG_Z(double, PhysPLQS<double>)
 }  // namespace psbh

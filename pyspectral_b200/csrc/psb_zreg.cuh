@@ -360,6 +360,49 @@ struct Mid<PhysPLQL<T>> : MidOneJob<PhysPLQL<T>> {
   }
 };
 
+// symmetric products of u and q: two of the three components of (u, q) in
+// registers at a time; component 0 is read again for its product with 2
+template <typename T>
+struct Mid<PhysPLQS<T>> : MidOneJob<PhysPLQS<T>> {
+  static constexpr bool value = true;
+  static constexpr int SLOTS = 7, HEAVY = 1;
+  __host__ __device__ static constexpr int in(int f) { return f; }
+  // out 11, 22, 33, 12, 13, 23 -> slots 1, 6, 2, 4, 0, 5
+  __host__ __device__ static constexpr int out(int g) {
+    return g == 0 ? 1 : (g == 1 ? 6 : (g == 2 ? 2 : (g == 3 ? 4 : (g == 4 ? 0 : 5))));
+  }
+  template <int A, int B>
+  __device__ static __forceinline__ void run(const PhysPLQS<T>&, const MidIO<T, A, B>& io, int) {
+    Cx<T> u[B], q[B], v[B], w[B], p[B];
+    io.load(0, u);
+    io.load(3, q);
+    io.load(1, v);
+    io.load(4, w);
+#pragma unroll
+    for (int r = 0; r < B; ++r) p[r] = (T)2 * had(u[r], q[r]);
+    io.store(1, p);
+#pragma unroll
+    for (int r = 0; r < B; ++r) p[r] = had_add(u[r], w[r], had(v[r], q[r]));
+    io.store(4, p);
+#pragma unroll
+    for (int r = 0; r < B; ++r) p[r] = (T)2 * had(v[r], w[r]);
+    io.store(6, p);
+    io.load(2, u);
+    io.load(5, q);
+#pragma unroll
+    for (int r = 0; r < B; ++r) p[r] = had_add(u[r], w[r], had(v[r], q[r]));
+    io.store(5, p);
+    io.load(0, v);
+    io.load(3, w);
+#pragma unroll
+    for (int r = 0; r < B; ++r) p[r] = (T)2 * had(u[r], q[r]);
+    io.store(2, p);
+#pragma unroll
+    for (int r = 0; r < B; ++r) p[r] = had_add(u[r], w[r], had(v[r], q[r]));
+    io.store(0, p);
+  }
+};
+
 // linearised MHD products: two components of (u, B, q, r) in registers at a
 // time; component 0 is read again for its products with 2
 template <typename T>
