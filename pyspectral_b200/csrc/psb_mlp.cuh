@@ -403,6 +403,81 @@ __device__ __forceinline__ void mlp_forward_fast(const MlpFwdSmem<H>& s, const u
   }
 }
 
+// A lane's weight fragments, held over many point tiles (28 registers at width 32).
+template <int H>
+struct MlpFrags {
+  uint2 f1[H / 8], f2[(H / 16) * (H / 8)], f3[H / 16];
+  __device__ __forceinline__ void load(const MlpFwdSmem<H>& s) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int j = 0; j < H / 8; ++j) f1[j] = s.f1[j * 32 + lane];
+#pragma unroll
+    for (int j = 0; j < (H / 16) * (H / 8); ++j) f2[j] = s.f2[j * 32 + lane];
+#pragma unroll
+    for (int j = 0; j < H / 16; ++j) f3[j] = s.f3[j * 32 + lane];
+  }
+};
+// mlp_forward_fast with the fragments in registers.
+template <int ACT, int H>
+__device__ __forceinline__ void mlp_forward_held(const MlpFwdSmem<H>& s, const MlpFrags<H>& w, const uint32_t* xa, float* y) {
+  constexpr int NJ = H / 8, NK = H / 16;
+  const int t = threadIdx.x & 3;
+  float h[NJ][4];
+#pragma unroll
+  for (int j = 0; j < NJ; ++j) {
+    const float b0 = s.b1[8 * j + 2 * t], b1 = s.b1[8 * j + 2 * t + 1];
+    h[j][0] = b0;
+    h[j][1] = b1;
+    h[j][2] = b0;
+    h[j][3] = b1;
+    const uint2 bb = w.f1[j];
+    const uint32_t b[2] = {bb.x, bb.y};
+    mma16816(h[j], xa, b);
+  }
+  uint32_t a[NK][4];
+#pragma unroll
+  for (int kk = 0; kk < NK; ++kk) {
+    a[kk][0] = act_pack<ACT>(h[2 * kk][0], h[2 * kk][1]);
+    a[kk][1] = act_pack<ACT>(h[2 * kk][2], h[2 * kk][3]);
+    a[kk][2] = act_pack<ACT>(h[2 * kk + 1][0], h[2 * kk + 1][1]);
+    a[kk][3] = act_pack<ACT>(h[2 * kk + 1][2], h[2 * kk + 1][3]);
+  }
+#pragma unroll
+  for (int j = 0; j < NJ; ++j) {
+    const float b0 = s.b2[8 * j + 2 * t], b1 = s.b2[8 * j + 2 * t + 1];
+    h[j][0] = b0;
+    h[j][1] = b1;
+    h[j][2] = b0;
+    h[j][3] = b1;
+  }
+#pragma unroll
+  for (int kk = 0; kk < NK; ++kk)
+#pragma unroll
+    for (int j = 0; j < NJ; ++j) {
+      const uint2 bb = w.f2[kk * NJ + j];
+      const uint32_t b[2] = {bb.x, bb.y};
+      mma16816(h[j], a[kk], b);
+    }
+#pragma unroll
+  for (int kk = 0; kk < NK; ++kk) {
+    a[kk][0] = act_pack<ACT>(h[2 * kk][0], h[2 * kk][1]);
+    a[kk][1] = act_pack<ACT>(h[2 * kk][2], h[2 * kk][3]);
+    a[kk][2] = act_pack<ACT>(h[2 * kk + 1][0], h[2 * kk + 1][1]);
+    a[kk][3] = act_pack<ACT>(h[2 * kk + 1][2], h[2 * kk + 1][3]);
+  }
+  const float c0 = s.b3[2 * t], c1 = s.b3[2 * t + 1];
+  y[0] = c0;
+  y[1] = c1;
+  y[2] = c0;
+  y[3] = c1;
+#pragma unroll
+  for (int kk = 0; kk < NK; ++kk) {
+    const uint2 bb = w.f3[kk];
+    const uint32_t b[2] = {bb.x, bb.y};
+    mma16816(y, a[kk], b);
+  }
+}
+
 // A fragment of normalised features for 16 points; feat(r, f) returns the raw
 // feature f (< 10) of row r (< 16) of this warp's tile.
 template <class S, class F>

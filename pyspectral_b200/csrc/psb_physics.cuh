@@ -1224,6 +1224,9 @@ struct PhysLearned {
       ym[e2] = c < kMlpOut ? s.ymean[c] : 0.f;
     }
     const int npts = P * A * 2 * B;
+    // a warp runs eight or so tiles here: the width-32 network's weights stay in registers
+    MlpFrags<H == 32 ? 32 : 16> w;
+    if constexpr (H == 32) w.load(s);
     for (int pt0 = warp * 16; pt0 < npts; pt0 += nw * 16) {
       int b[2];
       bool ok[2];
@@ -1249,7 +1252,10 @@ struct PhysLearned {
       xa[2] = pack_bf16(v[2], v[3]);
       xa[3] = pack_bf16(v[6], v[7]);
       float y[4];
-      mlp_forward_fast<ACT, H>(s, xa, y);
+      if constexpr (H == 32)
+        mlp_forward_held<ACT, H>(s, w, xa, y);
+      else
+        mlp_forward_fast<ACT, H>(s, xa, y);
       if (t < 3) {
 #pragma unroll
         for (int e = 0; e < 4; ++e) {

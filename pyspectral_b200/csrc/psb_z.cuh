@@ -5,14 +5,49 @@
 
 namespace psbh {
 
-// Pencils per CTA: enough for one middle item per thread, within the shared
-// memory of the kernel's CTAs per SM, and two CTAs per SM over the whole launch.
+// Pencils per CTA: the fewest instructions per pencil by the rounds of the three
+// stages (an outer round is NT/32 * (32/B) lines, a middle round NT/A items, an
+// incomplete one costs as much as a full one), against the CTAs that the shared
+// memory leaves on an SM.  Five pencils where a round holds 32 lines and a job
+// six fields, for instance: 30 lines each way, where four or six leave a
+// quarter of the lanes idle.
+template <typename T, class Phys, int A, int B>
+int z_reg_best_pencils() {
+  using Pl = psb::ZPlan<T, A, B>;
+  using Md = psb::Mid<Phys>;
+  constexpr int LW = Pl::NT / 32 * Pl::GW, QS = Pl::NT / A, MB = Pl::minb(Md::HEAVY);
+  auto up = [](int a, int b) { return (a + b - 1) / b; };
+  int best = 1;
+  double bc = 1e30;
+  for (int P = 1; P <= 32; ++P) {
+    const size_t smem = psb::z_reg_smem<Phys, T, A, B>(P);
+    if (smem > 200 * 1024) break;
+    const int ctas = std::min<int>(MB, (int)(228 * 1024 / (smem + 1024)));
+    double work = 0;
+    for (int k = 0; k < Md::JOBS; ++k) {
+      const int fi = Md::in0(k + 1) - Md::in0(k), fo = Md::out0(k + 1) - Md::out0(k);
+      work += 30.0 * A * (up(fi * P, LW) + up(fo * P, LW));
+      if (psb::phys_is_block<Phys>::value)
+        work += 20.0 * B * (up(fi * P, QS) + up(fo * P, QS)) + 130.0 * up(up(P * Pl::M, 16), Pl::NT / 32);
+      else
+        work += 20.0 * B * (fi + fo) * up(P, QS);
+    }
+    // fewer resident CTAs hide less of each other's latency
+    static const double hide[9] = {8, 4, 2.1, 1.25, 1.08, 1, 1, 1, 1};
+    const double cost = work / P * hide[std::min(ctas, 8)];
+    if (cost < bc) {
+      bc = cost;
+      best = P;
+    }
+  }
+  return best;
+}
+// ... and two CTAs per SM over the whole launch.
 template <typename T, class Phys, int A, int B>
 int z_reg_pencils(long long total) {
-  using Pl = psb::ZPlan<T, A, B>;
   constexpr int NJ = psb::Mid<Phys>::JOBS;
-  int P = std::max(1, Pl::NT / A);
-  while (P > 1 && psb::z_reg_smem<Phys, T, A, B>(P) > (size_t)(228 * 1024 / Pl::minb(psb::Mid<Phys>::HEAVY) - 1024)) --P;
+  static const int best = z_reg_best_pencils<T, Phys, A, B>();
+  int P = best;
   while (P > 1 && (total + P - 1) / P * NJ < 2 * 148) P = (P + 1) / 2;
   return P;
 }
