@@ -130,16 +130,14 @@ int psb_ctx_create(const psb_grid* grid, int precision, int device, psb_ctx** ou
 int psb_ctx_destroy(psb_ctx* ctx);
 /* Stream (cudaStream_t) on which the context queues its work; NULL = legacy default. */
 int psb_ctx_set_stream(psb_ctx* ctx, void* stream);
-/* Stage the inputs of the passes that read their rows unchanged (forward y
- * pass, the x pass of the spectral epilogue, plain inverse y passes) with
+/* At lengths without a register pass, stage the inputs of the passes that read
+ * their rows unchanged (forward y pass, the x pass of the spectral epilogue, plain inverse y passes) with
  * bulk tensor copies (1, the default) or with per-element loads (0).  Same
  * results either way; no counterpart in the reference (a launch choice). */
 int psb_ctx_set_tma(psb_ctx* ctx, int enable);
-/* Run the z pass of the 3/2-padded Navier-Stokes closures (DNS products,
- * Smagorinsky, learned; FP32) with its spectra loaded into and stored from
- * registers around the transforms when its schedule is a compiled two-pass
- * one ending in radix 16 (1, the default), or through shared memory (0).
- * Same results either way; no counterpart in the reference (a launch choice). */
+/* Run the z pass with its transforms in registers where its length has such a
+ * form (1, the default), or through shared memory (0).  Same results to
+ * rounding; no counterpart in the reference (a launch choice). */
 int psb_ctx_set_zrr(psb_ctx* ctx, int enable);
 /* Device status of the context's kernels since the last call, then cleared:
  * 0; 1 when a bounded wait inside a kernel gave up; 2 when a kernel found a
@@ -364,7 +362,8 @@ int psb_ensemble_destroy(psb_ensemble* e);
  * (PSB_DNS, PSB_SMAG or PSB_LEARNED) on `state` (not modified) with params p,
  * and keep the fastest in ctx: later psb_rhs / psb_step_rk4 calls of that
  * closure use them.  Results differ from the untuned ones only by rounding
- * (other radix orders). */
+ * (other radix orders).  A pass whose padded length has a register form runs
+ * that form whatever its shape, and is not timed. */
 int psb_autotune(psb_ctx* ctx, int closure, void* state, const psb_params* p);
 /* The tuned shape of pass 0..4 of closure (tile 0 when not tuned). */
 int psb_tuned_shape(const psb_ctx* ctx, int closure, int pass, int* tile, int* radices, int maxr);

@@ -345,8 +345,7 @@ class Context:
         self.check(self.lib.psb_ctx_set_tma(self.h, 1 if on else 0), "psb_ctx_set_tma")
 
     def set_zrr(self, on: bool):
-        """Register-direct z pass for two-pass (R1, 16) schedules (default) or the
-        shared-memory z pass."""
+        """Register z pass where its length has one (default) or the shared-memory z pass."""
         self.check(self.lib.psb_ctx_set_zrr(self.h, 1 if on else 0), "psb_ctx_set_zrr")
 
     def device_status(self):

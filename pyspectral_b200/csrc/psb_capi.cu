@@ -35,7 +35,7 @@ bool smooth23(int L) {
   return L == 1;
 }
 
-// Default radix schedule: radix 8 first, then 4, 2, 3 (the fastest default
+// Default radix schedule of the staged passes: radix 8 first, then 4, 2, 3 (the fastest default
 // measured on B200 at these lengths: larger radices raise register pressure
 // more than they save passes).  The batch autotuner also tries the
 // fewest-pass schedules over {16, 12, 8, 6, 4, 3, 2} and every radix order.

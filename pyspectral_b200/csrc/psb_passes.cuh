@@ -21,6 +21,10 @@
 //                     epilogue (`Epi`): pressure projection, viscous term,
 //                     closure divergence, Coriolis, RK stage update.
 //
+// These staged forms take any length of factors 2 and 3.  The lengths in use
+// have register forms (psb_reg.cuh, psb_zreg.cuh, psb_xreg.cuh), which run in
+// their place; the rest, and the persistent ensemble, run here.
+//
 // The padding maps reproduce PySpectral/src/padding.py:2-49 (pad/unpad drop
 // index N/2 of x and y and the k3=N/2 plane; pad_2x/unpad_2x keep the -N/2
 // mode).

@@ -1,5 +1,5 @@
 // Register passes: the strided-axis passes of the padded transforms for the
-// lengths L = A B of kRegAxis, with global memory on both sides and one
+// lengths L = A B of PSB_REG_AXIS, with global memory on both sides and one
 // shared-memory exchange between the two radices.
 //
 // Thread (j, c) loads the A elements j + B s of column c straight from the
@@ -16,7 +16,13 @@
 // share an SM and their loads cover each other's barrier; the passes it
 // replaces kept a tile of every field of a column in one CTA (up to 100 KB of
 // shared memory, two CTAs per SM) and made five to seven shared-memory round
-// trips per element.
+// trips per element.  Measured per launch on a B200, before -> after:
+//   t-model 128^3 FP64, 256 points  x-inverse 167 -> 44 us, y-inverse 318 -> 74,
+//                                   y-forward 439 -> 306
+//   DNS 256^3 FP32, 384 points      x-inverse 529 -> 149, y-inverse 894 -> 207
+//   learned 128^3 FP32, 192 points  y-inverse 177 -> 88
+// FP64 runs at up to 5 TB/s of the measured 6.5; FP32 at 2.3 to 3.6, its accesses
+// being 8 bytes a thread.
 #pragma once
 #include "psb_passes.cuh"
 

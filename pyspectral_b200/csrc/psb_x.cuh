@@ -27,7 +27,8 @@ int launch_reg_x(psb_ctx* c, psb::XEpiArgs<T> e, const Epi& epi, const char* wha
   constexpr int C = psb::xreg_cols<T>();
   e.main_blocks = (e.kz + C - 1) / C * e.n2;
   // three groups of threads a tile while every CTA of the launch is resident at once
-  // (a grid of 32^3 FP64: 11.8 -> 7 us); beyond that they only halve the CTAs per SM
+  // (DNS 32^3 FP64, timed with its launch: 14.9 us with one group, 12.8 with two or
+  // three); beyond that they only take CTAs from an SM that has more to run
   if constexpr (Epi::NACC > 0 && A * B * R <= 192) {
     constexpr int wave = 148 * (psb::xreg_minb<T, Epi, A, B, R>() / 3);
     if (e.main_blocks <= wave) return launch_reg_xs<T, Epi, A, B, R, 3>(c, e, epi, what, bytes);

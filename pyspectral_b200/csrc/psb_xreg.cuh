@@ -1,5 +1,5 @@
 // Register x pass: the last forward transform of the product spectra, fused
-// with the spectral epilogue, for the lengths L = A B R of kRegX.
+// with the spectral epilogue, for the lengths L = A B R of PSB_REG_X.
 //
 // A CTA owns C columns (64 bytes of k3) of one k2 and takes the F_IN fields one
 // after another: radix A from global memory, one shared-memory exchange (two
@@ -13,8 +13,13 @@
 // fused pass it replaces staged every field of a column in shared memory (12
 // fields: 100 KB, one or two CTAs per SM, six shared-memory accesses per
 // element); this one holds two buffers of one field, and the sums instead of
-// the products, so four to eight CTAs run per SM.  R is small because NACC R
-// accumulators live through the whole loop.
+// the products, so more CTAs run per SM.  R is small because NACC R accumulators
+// live through the whole loop: with R = 8 an FP64 thread of the t-model needs 228
+// registers, two CTAs per SM.  Measured per launch on a B200, before -> after:
+//   t-model 128^3 FP64, PLQL   373 -> 150 us     DNS 256^3 FP32   1063 -> 560
+//   Smagorinsky 64^3 FP64 1.0-1.6 -> 2.0 TB/s    DNS 32^3 FP64    10.5 -> 12.8
+// (the smallest grid pays for its six fields in series; the pass it replaces
+// staged them at once).
 #pragma once
 #include "psb_physics.cuh"
 

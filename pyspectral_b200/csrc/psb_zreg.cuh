@@ -1,6 +1,6 @@
 // Register z pass: c2r of the F_IN spectral pencils, the physical-space
 // products, r2c of the F_OUT results, for the real lengths M = 2 A B of
-// kRegZ, with the transforms and the products in registers.
+// PSB_REG_Z_F32 / _F64, with the transforms and the products in registers.
 //
 // A real pencil of M points is one complex transform of H = M/2 = A B points
 // of z[n] = x[2n] + i x[2n+1]; with X[k], k <= H, its spectrum and W = e^{2 pi i/M},
@@ -25,6 +25,13 @@
 // What bounds it: shared-memory bandwidth and the issue rate in the small
 // grids, HBM beyond L2.  The line stride and the stride of i are chosen at
 // compile time for the fewest bank conflicts of the two access patterns.
+// Measured per launch on a B200, staged form -> this one:
+//   Smagorinsky FP64   64^3 77 -> 50 us, 128^3 650 -> 380
+//   t-model 128^3 FP64 (256 points)   products 1304 -> 370, PLQL 1767 -> 527
+//   MHD t-model 128^3 FP32            815 -> 316 and 1294 -> 489
+//   DNS 256^3 FP32 (384 points)       2320 -> 464
+//   Smagorinsky FP32, 162 points      121 -> 50
+//   learned FP32       64^3 50 -> 48, 128^3 352 -> 308 (the network's MMAs remain)
 //
 // Fields sit in `slots` of the buffer (slot, pencil, i, j); Mid<Phys> says
 // which slot an input or output field uses: an output may reuse the slot of an
