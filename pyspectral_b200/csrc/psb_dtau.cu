@@ -161,9 +161,10 @@ int dtau_rhs(psb_ctx* c, StepIO<T> io, const psb_params* p, double* tau_out) {
   Cx<T>* Lf = scratch<T>(c, "dtau.Lf", 3 * nb, &st);
   // test filter masks (N grid): |k| < kf per axis (PySpectral/src/Classes.py:131-146)
   double* filt = reinterpret_cast<double*>(scratch<double>(c, "dtau.filt", (size_t)(N1 + N2 + N3h), &st));
-  double* sums = reinterpret_cast<double*>(scratch<double>(c, "dtau.sums", 4, &st));
-  double* part = reinterpret_cast<double*>(scratch<double>(c, "dtau.part", 3 * kDtauSumBlocks, &st));
+  // the sums and tau (8), then the blocks' partial sums
+  double* sums = reinterpret_cast<double*>(scratch<double>(c, "dtau.sums", 4 + 3 * kDtauSumBlocks, &st));
   if (st != PSB_OK) return st;
+  double* part = sums + 8;
   if (c->dtau_kf != kf) {
     std::vector<double> h(N1 + N2 + N3h);
     std::vector<double> k1(N1), k2(N2), k3(N3h);
