@@ -154,6 +154,7 @@ template <typename T>
 struct FieldTab {
   int nf = 0;
   unsigned char kind[12] = {}, sa[12] = {}, sb[12] = {};
+  int mfrom = 0;  // the first field that takes the factor m
   // optional separable factors (m1[row] m2[outer] m3[col]), applied in this order
   const double *m1 = nullptr, *m2 = nullptr, *m3 = nullptr;
   const double *f1 = nullptr, *f2 = nullptr, *f3 = nullptr;

@@ -81,7 +81,7 @@ __device__ __forceinline__ void axis_reg_body(const AxisArgs<T>& a, const FieldT
       const int i = row_of(a.in_map, j + B * s, a.in_rows);
       v[s] = (ok && i >= 0) ? src[(long long)i * a.in_rstride] : zero;
     }
-    if (ft.m1) {
+    if (ft.m1 && g >= ft.mfrom) {
       const double mc = ok ? ft.m2[o] : 0.0, m3 = ok ? ft.m3[col] : 0.0;
 #pragma unroll
       for (int s = 0; s < A; ++s) {
