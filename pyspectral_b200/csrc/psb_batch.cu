@@ -80,6 +80,7 @@ struct Batch {
   static constexpr int Fi = Pre::F_DST, Fb = pre_b_fields<Pre>::value, Fo = Phys::F_OUT;
   using YP = pre_ypass<T, Pre>;
   using YPre = typename YP::type;
+  static_assert(pre_has_zsrc2<Pre>::value == phys_in2<Phys>::value, "means of two spectra: pre/phys mismatch");
   psb_batch* b;
   psb_ctx* c;
   Dims d;

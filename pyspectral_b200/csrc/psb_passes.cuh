@@ -123,6 +123,16 @@ struct phys_default_ppc<P, decltype((void)P::DEFAULT_PPC, void())> {
   static constexpr int value = P::DEFAULT_PPC;
 };
 
+// Whether some inputs of the z pass are means of two stored spectra (Phys::IN2).
+template <class P, class = void>
+struct phys_in2 {
+  static constexpr bool value = false;
+};
+template <class P>
+struct phys_in2<P, decltype((void)P::IN2, void())> {
+  static constexpr bool value = P::IN2;
+};
+
 template <typename T>
 struct AxisArgs {
   const Cx<T>* in;
@@ -533,6 +543,7 @@ __device__ __forceinline__ void zpass_tile(const ZArgs<T>& a, const Phys& phys, 
   const int M = a.plan.L;
   const int P = a.ppc;
   constexpr int FMAX = FI > FO ? FI : FO;
+  constexpr bool IN2 = phys_in2<Phys>::value;
   const int nl = (FMAX * P + 1) / 2;
   const int LS = zline(M);
   Cx<T>* X = tw + M;
@@ -556,7 +567,8 @@ __device__ __forceinline__ void zpass_tile(const ZArgs<T>& a, const Phys& phys, 
       constexpr int U = 4;
       const int hp = P >> 1, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
       for (int cb = threadIdx.x >> 5; cb < nin; cb += U * nw) {
-        const Cx<T>*src[U], *src2[U];
+        const Cx<T>* src[U];
+        const Cx<T>* src2[IN2 ? U : 1];
         long long ps[U];
         int kz[U];
         bool oka[U], okb[U], dz[U];
@@ -572,7 +584,7 @@ __device__ __forceinline__ void zpass_tile(const ZArgs<T>& a, const Phys& phys, 
           okb[u] = pa + 1 < a.npencils;
           ps[u] = a.in_pstride[f];
           src[u] = a.in[f] + (oka[u] ? pa * ps[u] : 0);
-          src2[u] = a.in2[f] ? a.in2[f] + (oka[u] ? pa * ps[u] : 0) : nullptr;
+          if constexpr (IN2) src2[u] = a.in2[f] ? a.in2[f] + (oka[u] ? pa * ps[u] : 0) : nullptr;
           dz[u] = c < nin && a.dz[f] != 0;
           anydz |= dz[u];
           kzmax = max(kzmax, kz[u]);
@@ -595,9 +607,11 @@ __device__ __forceinline__ void zpass_tile(const ZArgs<T>& a, const Phys& phys, 
               va = mk<T>(-kk * va.y, kk * va.x);
               vb = mk<T>(-kk * vb.y, kk * vb.x);
             }
-            if (src2[u]) {
-              va = (T)0.5 * (va + (oka[u] ? src2[u][k] : zero));
-              vb = (T)0.5 * (vb + (okb[u] ? src2[u][ps[u] + k] : zero));
+            if constexpr (IN2) {
+              if (src2[u]) {
+                va = (T)0.5 * (va + (oka[u] ? src2[u][k] : zero));
+                vb = (T)0.5 * (vb + (okb[u] ? src2[u][ps[u] + k] : zero));
+              }
             }
             Cx<T>* Z = X + (size_t)(cb + u * nw) * LS;
             if (k == 0 || k == half) {
@@ -633,7 +647,8 @@ __device__ __forceinline__ void zpass_tile(const ZArgs<T>& a, const Phys& phys, 
           const T kk = (T)a.k3[k];
           v = mk<T>(-kk * v.y, kk * v.x);
         }
-        if (a.in2[f]) v = (T)0.5 * (v + a.in2[f][pen * a.in_pstride[f] + k]);
+        if constexpr (IN2)
+          if (a.in2[f]) v = (T)0.5 * (v + a.in2[f][pen * a.in_pstride[f] + k]);
         if (part == 0) A = v; else B = v;
       }
       Cx<T>* Z = X + (size_t)c * LS;
@@ -701,11 +716,21 @@ __device__ __forceinline__ void zpass_body(const ZArgs<T>& a, const Phys& phys, 
   zpass_tile<T, Phys, WIDE>(a, phys, bx);
 }
 
+// CTAs per SM the registers are bounded for.  FP64: two, as the tile's share of
+// the shared memory leaves room for (128 registers; the transforms need about
+// 122).  With 140 registers and one CTA per SM the DNS pass of 64 x 64 x 288
+// (432 points) takes 529 us against 332, and psb_fft_c2r of 128^3 258 against
+// 209.  The radices of the wide form and the network's tiles need more.
+template <typename T, class Phys, bool WIDE>
+constexpr int zpass_minb() {
+  return sizeof(T) == 4 ? 3 : (WIDE || phys_is_block<Phys>::value ? 1 : 2);
+}
+
 // Tiles bx = blockIdx.x, + gridDim.x, ... < ceil(npencils/ppc): any grid
 // size covers every tile; a grid of (resident CTAs per SM) x SMs stages the
 // twiddles and the Phys extra once per CTA instead of once per tile.
 template <typename T, class Phys, bool WIDE = false>
-__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 1) zpass_kernel(ZArgs<T> a, Phys phys) {
+__global__ void __launch_bounds__(256, zpass_minb<T, Phys, WIDE>()) zpass_kernel(ZArgs<T> a, Phys phys) {
   pdl_trigger();
   zpass_setup<T, Phys>(a, phys);
   pdl_wait();
@@ -742,7 +767,7 @@ __device__ __forceinline__ void zpass_batch_body(const ZArgs<T>* __restrict__ A,
 }
 
 template <typename T, class Phys, bool WIDE>
-__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 1)
+__global__ void __launch_bounds__(256, zpass_minb<T, Phys, WIDE>())
     zpass_batch(const ZArgs<T>* __restrict__ A, const Phys* __restrict__ phys, int runs) {
   zpass_batch_body<T, Phys, WIDE>(A, phys, runs);
 }

@@ -213,6 +213,7 @@ struct PhysProducts {
 template <typename T>
 struct PhysSmag {
   static constexpr int F_IN = 9, F_OUT = 12;
+  static constexpr bool IN2 = true;  // S13 and S23 (PreStrain::zsrc2)
   T csd2;  // 0.16*Delta*0.16*Delta
   __device__ __forceinline__ void operator()(long long, int, const T* in, T* out) const {
     const T u = in[0], v = in[1], w = in[2];

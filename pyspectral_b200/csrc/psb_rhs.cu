@@ -49,6 +49,7 @@ int run_ns32(psb_ctx* c, const Cx<T>* Qin, Pre pre, Phys phys, Epi epi, const ps
   constexpr int Fi = Pre::F_DST, Fb = pre_b_fields<Pre>::value, Fo = Phys::F_OUT;
   static_assert(Phys::F_IN == Fb + pre_z_derived<Pre>::value, "pre/phys mismatch");
   static_assert(Epi::F_IN == Phys::F_OUT, "phys/epi mismatch");
+  static_assert(pre_has_zsrc2<Pre>::value == phys_in2<Phys>::value, "means of two spectra: pre/phys mismatch");
   int st = PSB_OK;
   Cx<T>* A = scratch<T>(c, "ns.A", (size_t)Fi * M1 * N2 * Kz, &st);
   Cx<T>* B = scratch<T>(c, "ns.B", (size_t)Fb * M1 * M2 * Kz, &st);
