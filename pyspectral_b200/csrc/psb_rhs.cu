@@ -830,9 +830,12 @@ __device__ __forceinline__ void dsmag_lm(const Cx<T>* __restrict__ A, const Cx<T
   }
 }
 
-// per-block partial sums of <L:M> and <M:M> (src/RHSfunctions.py:1838-1842)
+// per-block partial sums of <L:M> and <M:M> (src/RHSfunctions.py:1838-1842).
+// kLmBlocks is two CTAs per SM, so the registers are bounded for two: left to
+// the compiler the kernel took 172 to 188, one CTA per SM and two waves
+// (128^3 FP64 113 us against 82, FP32 70 against 50).
 template <typename T>
-__global__ void __launch_bounds__(256) dsmag_lm_kernel(const Cx<T>* __restrict__ A, const Cx<T>* __restrict__ B,
+__global__ void __launch_bounds__(256, 2) dsmag_lm_kernel(const Cx<T>* __restrict__ A, const Cx<T>* __restrict__ B,
                                                        const double* __restrict__ g, int N1, int N2, int N3,
                                                        int n3h, double d2, double* __restrict__ part) {
   const long long fs = (long long)N1 * N2 * n3h;
