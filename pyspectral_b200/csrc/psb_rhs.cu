@@ -37,6 +37,17 @@ AxisArgs<T> axis_common(psb_ctx* c, int L) {
 // ---------------------------------------------------------------------------
 // 3/2-padded Navier-Stokes (DNS, Smagorinsky, SGS of filtered DNS)
 // ---------------------------------------------------------------------------
+// Physics that are the products (PhysProducts) of input fields 0-2 and, apart
+// from them, of fields 3-5 (Phys::TWO_PRODUCTS).
+template <class P, class = void>
+struct two_products {
+  static constexpr bool value = false;
+};
+template <class P>
+struct two_products<P, decltype((void)P::TWO_PRODUCTS, void())> {
+  static constexpr bool value = P::TWO_PRODUCTS;
+};
+
 // ts: autotuned launch shapes of the five passes (psb_autotune), or null
 template <typename T, class Pre, class Phys, class Epi>
 int run_ns32(psb_ctx* c, const Cx<T>* Qin, Pre pre, Phys phys, Epi epi, const psb_tuned* ts = nullptr) {
@@ -111,18 +122,27 @@ int run_ns32(psb_ctx* c, const Cx<T>* Qin, Pre pre, Phys phys, Epi epi, const ps
   z.fac = (T)(s32 / ((double)M1 * M2 * M3));
   z.plan = *plan_for(c, M3);
   z.tw = twiddles<T>(c);
-  // the products of u and of the filtered u: the products pass once for each, in
-  // registers (64^3 FP64 in one staged pass 133 us, 86 with a compiled schedule)
-  if constexpr (Phys::F_IN == 6 && Phys::F_OUT == 12) {
-    for (int h = 0; h < 2; ++h) {
+  // two products passes in the registers against one staged pass of both sets
+  // (64^3 FP64 42 us against 133); where the length has no register pass the one
+  // staged launch is the faster (12^3, 18 points, FP64 16.7 us against 29.6)
+  bool split = false;
+  if constexpr (two_products<Phys>::value) {
+    split = c->use_zrr && has_reg_z<T, PhysProducts<T>>(M3);
+    for (int h = 0; split && h < 2; ++h) {
       ZArgs<T> y = z;
-      for (int f = 0; f < 3; ++f) y.in[f] = z.in[3 * h + f], y.in_pstride[f] = z.in_pstride[3 * h + f], y.in_kz[f] = z.in_kz[3 * h + f];
-      for (int g = 0; g < 6; ++g) y.out[g] = z.out[6 * h + g], y.out_pstride[g] = z.out_pstride[6 * h + g];
+      for (int f = 0; f < 3; ++f) {
+        y.in[f] = z.in[3 * h + f];
+        y.in_pstride[f] = z.in_pstride[3 * h + f];
+        y.in_kz[f] = z.in_kz[3 * h + f];
+      }
+      for (int g = 0; g < 6; ++g) {
+        y.out[g] = z.out[6 * h + g];
+        y.out_pstride[g] = z.out_pstride[6 * h + g];
+      }
       PSB_TRY((launch_z<T, PhysProducts<T>, true>(c, y, PhysProducts<T>{}, "z-fused")));
     }
-  } else {
-    PSB_TRY((launch_z<T, Phys, true>(c, z, phys, "z-fused", 0.0, sh[2])));
   }
+  if (!split) PSB_TRY((launch_z<T, Phys, true>(c, z, phys, "z-fused", 0.0, sh[2])));
   // y forward with truncation
   AxisArgs<T> d = axis_common<T>(c, M2);
   d.in = C;
@@ -194,6 +214,7 @@ struct PreMask3 {
 template <typename T>
 struct PhysSGSDNS {
   static constexpr int F_IN = 6, F_OUT = 12;
+  static constexpr bool TWO_PRODUCTS = true;
   __device__ __forceinline__ void operator()(long long, int, const T* in, T* out) const {
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
