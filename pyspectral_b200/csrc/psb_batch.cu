@@ -80,6 +80,8 @@ struct Batch {
   static constexpr int Fi = Pre::F_DST, Fb = pre_b_fields<Pre>::value, Fo = Phys::F_OUT;
   using YP = pre_ypass<T, Pre>;
   using YPre = typename YP::type;
+  // the staged y-inverse pass: lines per column, outer groups
+  static constexpr int Fy = pre_tile_fields<YPre>(), Gy = YP::groups * pre_tile_groups<YPre>();
   static_assert(pre_has_zsrc2<Pre>::value == phys_in2<Phys>::value, "means of two spectra: pre/phys mismatch");
   psb_batch* b;
   psb_ctx* c;
@@ -172,8 +174,8 @@ struct Batch {
     tile = b->tile[pass];
     plan = b->plan[pass];
     if (!reg_pass(pass) || !is_reg_axis(plan)) return;
-    const int F = pass == 0 ? Fi : (pass == 1 ? YPre::F_DST : 1);
-    const int no = pass == 0 ? d.N2 : (pass == 1 ? YP::groups * d.M1 : Fo * d.M1);
+    const int F = pass == 0 ? Fi : (pass == 1 ? Fy : 1);
+    const int no = pass == 0 ? d.N2 : (pass == 1 ? Gy * d.M1 : Fo * d.M1);
     default_axis_shape<T>(c, plan.L, d.Kz, F, no, false, tile, plan);
   }
 
@@ -361,7 +363,7 @@ struct Batch {
       case 3: {
         const bool inv = pass == 1;
         const int ct = b->tile[pass];
-        // y-inverse: YP::groups outer groups of YPre::F_DST lines per column
+        // y-inverse, register form: YP::groups outer groups of YPre::F_DST fields
         const int G = inv ? YP::groups : Fo, F = inv ? Fb : Fo;
         const double by = (double)R * esz * F * d.M1 * d.Kz * (double)(d.N2 + d.M2);
         if (is_reg_axis(b->plan[pass])) {
@@ -371,8 +373,8 @@ struct Batch {
           if constexpr (has_fields<YPre>())
             return reg_axis_batch<T>(c, ay, YPre{}.fields(), d.M2, d.Kz, G * d.M1, R, true, "batch y-inverse", by);
         }
-        dim3 g((d.Kz + ct - 1) / ct, G * d.M1, R);
-        const size_t sm = smem_axis(d.M2, inv ? YPre::F_DST : 1, ct);
+        dim3 g((d.Kz + ct - 1) / ct, (inv ? Gy : Fo) * d.M1, R);
+        const size_t sm = smem_axis(d.M2, inv ? Fy : 1, ct);
         if (inv) {
           auto go = [&](auto k) {
             set_smem(k, sm);
@@ -466,7 +468,7 @@ struct Batch {
                Epi (*mkepi)(psb_ctx*, StepIO<T>, const psb_params&)) {
     const size_t esz = sizeof(Cx<T>);
     const int Ls[5] = {d.M1, d.M2, d.M3, d.M2, d.M1};
-    const int Fs[5] = {Fi, YPre::F_DST, 0, 1, Fo};
+    const int Fs[5] = {Fi, Fy, 0, 1, Fo};
     // RHS-mode passes read the runs' states and write only scratch; run one
     // full RHS first so that every intermediate buffer holds real data.
     for (int pass = 0; pass < 5; ++pass) PSB_TRY(launch(pass, 4));
@@ -599,7 +601,7 @@ int run_batch(psb_batch* b, int nsteps, bool tune, Pre pre0, Phys (*mkphys)(psb_
     b->arena_bytes = need;
   }
   if (b->plan[0].L == 0) {
-    default_shapes<T>(b, BT::Fi, BT::Fb, Phys::F_IN, BT::Fo, BT::YPre::F_DST, BT::YP::groups, &BT::reg_pass,
+    default_shapes<T>(b, BT::Fi, BT::Fb, Phys::F_IN, BT::Fo, BT::Fy, BT::Gy, &BT::reg_pass,
                    phys_default_ppc<Phys>::value, (size_t)phys_is_block<Phys>::extra);
     if constexpr (z_registered<Phys>::value)
       if (c->use_zrr && has_reg_z<T, Phys>(x.d.M3))
@@ -770,7 +772,7 @@ size_t ens_group(psb_batch* b, int kind, EnsGroup& g) {
   g.nx[0] = (d.Kz + t[0] - 1) / t[0];
   g.ny[0] = d.N2;
   g.nx[1] = (d.Kz + t[1] - 1) / t[1];
-  g.ny[1] = BT::YP::groups * d.M1;
+  g.ny[1] = BT::Gy * d.M1;
   g.nx[2] = (int)(((long long)d.M1 * d.M2 + t[2] - 1) / t[2]);
   g.ny[2] = 1;
   g.nx[3] = (d.Kz + t[3] - 1) / t[3];
@@ -782,7 +784,7 @@ size_t ens_group(psb_batch* b, int kind, EnsGroup& g) {
   for (int k = 0; k < 5; ++k) g.items[k] = (long long)g.nx[k] * g.ny[k] * g.R;
   size_t sm = 0;
   sm = std::max(sm, x.smem_axis(d.M1, BT::Fi, t[0]));
-  sm = std::max(sm, x.smem_axis(d.M2, BT::YPre::F_DST, t[1]));
+  sm = std::max(sm, x.smem_axis(d.M2, BT::Fy, t[1]));
   sm = std::max(sm, x.smem_z(t[2]));
   sm = std::max(sm, x.smem_axis(d.M2, 1, t[3]));
   sm = std::max(sm, x.smem_axis(d.M1, BT::Fo, t[4]));

@@ -487,7 +487,9 @@ template <typename T, bool INV, class Pre, bool TUNABLE = false>
 int launch_axis(psb_ctx* c, psb::AxisArgs<T> a, Pre pre, const char* what, const psb_pass_shape* sh = nullptr) {
   const size_t esz = sizeof(Cx<T>);
   const int L = a.plan.L;
-  a.col_tile = pick_ct(a.ncols, Pre::F_DST, L, esz, a.nouter);
+  constexpr int FT = psb::pre_tile_fields<Pre>();                   // fields of a staged tile
+  const int outer = a.nouter * psb::pre_tile_groups<Pre>();        // outer indices of the staged grid
+  a.col_tile = pick_ct(a.ncols, FT, L, esz, outer);
   if (sh && sh->tile && !sh->reg) {
     a.col_tile = sh->tile;
     a.plan = sh->plan;
@@ -499,8 +501,8 @@ int launch_axis(psb_ctx* c, psb::AxisArgs<T> a, Pre pre, const char* what, const
   if constexpr (psb::pre_has_fields<Pre>::value) {
     if (has_reg_axis(L)) return reg_axis<T>(c, a, pre.fields(), INV, what, bytes);
   }
-  const size_t smem = (size_t)(L + 2 * L * Pre::F_DST * a.col_tile) * esz;
-  dim3 grid((a.ncols + a.col_tile - 1) / a.col_tile, a.nouter);
+  const size_t smem = (size_t)(L + 2 * L * FT * a.col_tile) * esz;
+  dim3 grid((a.ncols + a.col_tile - 1) / a.col_tile, outer);
   auto go = [&](auto k) {
     set_smem(k, smem);
     LaunchScope scope(c, what, bytes);

@@ -179,6 +179,28 @@ struct pre_has_fields<P, decltype((void)sizeof(decltype(std::declval<const P&>()
   static constexpr bool value = true;
 };
 
+// Pre functors whose staged pass takes one destination field a CTA (Pre::SPLIT):
+// field g is split(kind(g), k_row, s[sa(g)], s[sb(g)]), so a CTA loads only what
+// its field needs and its tile keeps wide rows.  Outer index o of the staged grid
+// is field o / a.nouter at outer index o % a.nouter.
+template <class P, class = void>
+struct pre_split {
+  static constexpr bool value = false;
+};
+template <class P>
+struct pre_split<P, decltype((void)P::SPLIT, void())> {
+  static constexpr bool value = P::SPLIT;
+};
+// Fields of a staged CTA's tile, and CTAs (fields) an outer index.
+template <class P>
+constexpr int pre_tile_fields() {
+  return pre_split<P>::value ? 1 : P::F_DST;
+}
+template <class P>
+constexpr int pre_tile_groups() {
+  return pre_split<P>::value ? P::F_DST : 1;
+}
+
 template <typename T>
 struct PreCopy {
   static constexpr int F_SRC = 1, F_DST = 1;
@@ -264,7 +286,9 @@ __device__ __forceinline__ void axis_pass_body(const AxisArgs<T>& a, const Pre& 
   Cx<T>* tw = reinterpret_cast<Cx<T>*>(smem_raw);
   const int L = a.plan.L;
   const int ct = a.col_tile;
-  const int lines = Pre::F_DST * ct;
+  constexpr bool SP = pre_split<Pre>::value;
+  constexpr int FS = SP ? 2 : Pre::F_SRC, FD = pre_tile_fields<Pre>();
+  const int lines = FD * ct;
   Cx<T>* bufA = tw + L;
   Cx<T>* bufB = bufA + (size_t)L * lines;
   const int o = by;
@@ -282,25 +306,37 @@ __device__ __forceinline__ void axis_pass_body(const AxisArgs<T>& a, const Pre& 
   // [in_rows+shift, L) of the row map (every map used has in_rows >= hi)
   {
     const RowMap m = a.in_map;
-    const int g0 = m.lo < L ? m.lo : L, g1 = min(m.hi + m.shift, L);
+    const int z0 = m.lo < L ? m.lo : L, z1 = min(m.hi + m.shift, L);
     const int t0 = min(a.in_rows + m.shift, L);
-    for (int j = g0; j < g1; ++j)
+    for (int j = z0; j < z1; ++j)
       for (int l = threadIdx.x; l < lines; l += nt) bufA[(size_t)j * lines + l] = zero;
     for (int j = t0; j < L; ++j)
       for (int l = threadIdx.x; l < lines; l += nt) bufA[(size_t)j * lines + l] = zero;
   }
   pdl_wait();
-  const Cx<T>* inb = a.in + (long long)o * a.in_ostride;
+  const int g0 = SP ? o / a.nouter : 0;  // split: the field, and what forms it
+  FieldKind kind = kCopy;
+  long long fo[FS];
+  if constexpr (SP) {
+    kind = Pre::kind(g0);
+    fo[0] = Pre::sa(g0) * a.in_fstride;
+    fo[1] = Pre::sb(g0) * a.in_fstride;
+  } else {
+#pragma unroll
+    for (int f = 0; f < FS; ++f) fo[f] = f * a.in_fstride;
+  }
+  const Cx<T>* inb = a.in + (long long)(SP ? o - g0 * a.nouter : o) * a.in_ostride;
   // U rows per round: every load of a round is issued before the first store
-  constexpr int U = Pre::F_SRC >= 3 ? 2 : (Pre::F_SRC == 2 ? 4 : 8);
+  constexpr int U = FS >= 3 ? 2 : (FS == 2 ? 4 : 8);
   for (int i0 = r0; i0 < a.in_rows; i0 += U * dr) {
-    Cx<T> s[U][Pre::F_SRC];
+    Cx<T> s[U][FS];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const int i = i0 + u * dr;
 #pragma unroll
-      for (int f = 0; f < Pre::F_SRC; ++f)
-        s[u][f] = (colok && i < a.in_rows) ? inb[f * a.in_fstride + i * a.in_rstride + col] : zero;
+      for (int f = 0; f < FS; ++f)
+        s[u][f] = (colok && i < a.in_rows && (!SP || f == 0 || kind == kIkMean)) ? inb[fo[f] + i * a.in_rstride + col]
+                                                                                 : zero;
     }
 #pragma unroll
     for (int u = 0; u < U; ++u) {
@@ -308,19 +344,22 @@ __device__ __forceinline__ void axis_pass_body(const AxisArgs<T>& a, const Pre& 
       if (i >= a.in_rows) break;
       const int j = a.in_map(i);
       if (j < 0) continue;
-      Cx<T> d[Pre::F_DST];
+      Cx<T> d[FD];
       if (colok) {
-        pre(i, o, col, a, s[u], d);
+        if constexpr (SP)
+          d[0] = Pre::split(kind, (T)a.k_row[i], s[u][0], s[u][1]);
+        else
+          pre(i, o, col, a, s[u], d);
       } else {
 #pragma unroll
-        for (int g = 0; g < Pre::F_DST; ++g) d[g] = zero;
+        for (int g = 0; g < FD; ++g) d[g] = zero;
       }
 #pragma unroll
-      for (int g = 0; g < Pre::F_DST; ++g) bufA[(size_t)j * lines + g * ct + c] = d[g];
+      for (int g = 0; g < FD; ++g) bufA[(size_t)j * lines + g * ct + c] = d[g];
     }
   }
   __syncthreads();
-  axis_transform_store<T, INV, Pre::F_DST, WIDE>(a, bufA, bufB, tw, o, c0);
+  axis_transform_store<T, INV, FD, WIDE>(a, bufA, bufB, tw, o, c0);
 }
 
 // TMA-staged axis pass for passes that read their rows unchanged (PreCopy,
@@ -372,13 +411,13 @@ __global__ void __launch_bounds__(256) axis_pass_tma_kernel(AxisArgs<T> a, const
   axis_transform_store<T, INV, 1, false>(a, bufA, bufB, tw, o, c0);
 }
 
-// grid = (ceil(ncols/col_tile), nouter)
+// grid = (ceil(ncols/col_tile), nouter * pre_tile_groups)
 template <typename T, bool INV, class Pre, bool WIDE = false>
 __global__ void __launch_bounds__(256) axis_pass_kernel(AxisArgs<T> a, Pre pre) {
   axis_pass_body<T, INV, Pre, WIDE>(a, pre, blockIdx.x, blockIdx.y);
 }
 
-// Batched: grid = (ceil(ncols/col_tile), nouter, runs); run blockIdx.z takes
+// Batched: grid = (ceil(ncols/col_tile), nouter * pre_tile_groups, runs); run blockIdx.z takes
 // its arguments from A[z] and pre[z] (same tile shape for every run).
 template <typename T, bool INV, class Pre, bool WIDE>
 __global__ void __launch_bounds__(256) axis_pass_batch(const AxisArgs<T>* __restrict__ A, const Pre* __restrict__ pre) {

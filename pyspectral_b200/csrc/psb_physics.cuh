@@ -139,28 +139,30 @@ struct PreCopyN {
 template <typename T>
 struct PreYStrain {
   static constexpr int F_SRC = 6, F_DST = 8, GROUPS = 1, IN_FIELDS = 1, OUT_FIELDS = 1;
+  // the staged pass takes one field a CTA: with the eight in one tile its rows are
+  // one column wide (64 x 384 x 64 FP32, 576 points: PSB_MEASURE_Y)
+  static constexpr bool SPLIT = true;
+  // stored fields u, v, w, i k1 u, i k1 v, i k1 w; field g from sa(g) (and sb(g))
+  __host__ __device__ static constexpr int sa(int g) {
+    return g < 4 ? g : (g == 4 ? 1 : (g == 5 ? 0 : (g == 6 ? 5 : 2)));
+  }
+  __host__ __device__ static constexpr int sb(int) { return 4; }
+  __host__ __device__ static constexpr FieldKind kind(int g) {
+    return g < 4 || g == 6 ? kCopy : (g == 5 ? kIkMean : kIkRow);
+  }
+  __device__ __forceinline__ static Cx<T> split(FieldKind kind, T k, Cx<T> a, Cx<T> b) {
+    if (kind == kCopy) return a;
+    return kind == kIkRow ? pik(k, a) : (T)0.5 * (pik(k, a) + b);
+  }
   __host__ FieldTab<T> fields() const {
-    const unsigned char sa[8] = {0, 1, 2, 3, 1, 0, 5, 2};
-    const unsigned char kind[8] = {kCopy, kCopy, kCopy, kCopy, kIkRow, kIkMean, kCopy, kIkRow};
     FieldTab<T> t;
     t.nf = 8;
     for (int g = 0; g < 8; ++g) {
-      t.sa[g] = sa[g];
-      t.kind[g] = kind[g];
+      t.sa[g] = (unsigned char)sa(g);
+      t.sb[g] = (unsigned char)sb(g);
+      t.kind[g] = kind(g);
     }
-    t.sb[5] = 4;
     return t;
-  }
-  __device__ void operator()(int i, int, int, const AxisArgs<T>& a, const Cx<T>* s, Cx<T>* d) const {
-    const T k2 = (T)a.k_row[i];
-    d[0] = s[0];
-    d[1] = s[1];
-    d[2] = s[2];
-    d[3] = s[3];
-    d[4] = pik(k2, s[1]);
-    d[5] = (T)0.5 * (pik(k2, s[0]) + s[4]);
-    d[6] = s[5];
-    d[7] = pik(k2, s[2]);
   }
 };
 template <typename T>

@@ -2006,8 +2006,8 @@ TuneDims tune_dims(psb_ctx* c, int closure, int act, int hidden) {
     t.defppc = phys_default_ppc<PhysProducts<T>>::value;
   } else if (closure == PSB_SMAG) {
     t.Fi = PreStrain<T>::F_DST, t.Fb = pre_b_fields<PreStrain<T>>::value, t.Fo = 12;
-    t.Fy = PreYStrain<T>::F_DST;
-    t.Gy = pre_ypass<T, PreStrain<T>>::groups;
+    t.Fy = pre_tile_fields<PreYStrain<T>>();
+    t.Gy = pre_ypass<T, PreStrain<T>>::groups * pre_tile_groups<PreYStrain<T>>();
     t.maxppc = phys_max_ppc<PhysSmag<T>>::value;
     t.Fz = PhysSmag<T>::F_IN;
     t.defppc = phys_default_ppc<PhysSmag<T>>::value;
