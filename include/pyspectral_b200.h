@@ -130,10 +130,12 @@ int psb_ctx_create(const psb_grid* grid, int precision, int device, psb_ctx** ou
 int psb_ctx_destroy(psb_ctx* ctx);
 /* Stream (cudaStream_t) on which the context queues its work; NULL = legacy default. */
 int psb_ctx_set_stream(psb_ctx* ctx, void* stream);
-/* At lengths without a register pass, stage the inputs of the passes that read
- * their rows unchanged (forward y pass, the x pass of the spectral epilogue, plain inverse y passes) with
- * bulk tensor copies (1, the default) or with per-element loads (0).  Same
- * results either way; no counterpart in the reference (a launch choice). */
+/* Where a staged pass runs (a length without a register pass, or a staged shape
+ * given to psb_set_tuned_shape), stage the inputs of the passes that read their
+ * rows unchanged (forward y pass, the x pass of the spectral epilogue, plain
+ * inverse y passes) with bulk tensor copies (1, the default) or with per-element
+ * loads (0).  Same results either way; no counterpart in the reference (a launch
+ * choice). */
 int psb_ctx_set_tma(psb_ctx* ctx, int enable);
 /* Run the z pass with its transforms in registers where its length has such a
  * form (1, the default), or through shared memory (0).  Same results to
@@ -362,8 +364,8 @@ int psb_ensemble_destroy(psb_ensemble* e);
  * (PSB_DNS, PSB_SMAG or PSB_LEARNED) on `state` (not modified) with params p,
  * and keep the fastest in ctx: later psb_rhs / psb_step_rk4 calls of that
  * closure use them.  Results differ from the untuned ones only by rounding
- * (other radix orders).  A pass whose padded length has a register form runs
- * that form whatever its shape, and is not timed. */
+ * (other radix orders).  Where the padded length has a register pass it is one
+ * of the candidates; the z pass is left to psb_ctx_set_zrr there. */
 int psb_autotune(psb_ctx* ctx, int closure, void* state, const psb_params* p);
 /* The tuned shape of pass 0..4 of closure (tile 0 when not tuned). */
 int psb_tuned_shape(const psb_ctx* ctx, int closure, int pass, int* tile, int* radices, int maxr);
@@ -375,7 +377,10 @@ int psb_autotune_clear(psb_ctx* ctx, int closure);
  * (nrad radices from {2,3,4,6,8,12,16} whose product is the pass's padded
  * length).  Replays a saved psb_autotune result (the pyFFTW plans of
  * src/Classes.py:590-625 carry no such choice: this is the autotuner's cache).
- * The other passes keep their tuned or default shapes. */
+ * Where the length has a register pass, that pass's own tile and radices (as
+ * psb_tuned_shape reports them) select it and any other shape the staged pass;
+ * a staged z shape takes effect while psb_ctx_set_zrr is 0.  The other passes
+ * keep their tuned or default shapes. */
 int psb_set_tuned_shape(psb_ctx* ctx, int closure, int pass, int tile, const int* radices, int nrad);
 
 #ifdef __cplusplus

@@ -25,7 +25,7 @@ struct psb_pass_shape {
   int tile = 0;
   psb::FFTPlan plan{};
   bool wide = false;
-  bool reg = false;  // the register pass's own shape: the runtime-schedule kernels ignore it
+  bool reg = false;  // the register pass of this length, tile and radices its own
 };
 // Shapes of the five passes (x-inverse, y-inverse, z, y-forward, x-forward) of
 // a 3/2-padded closure's RHS.
@@ -354,10 +354,6 @@ inline bool has_reg_axis(int L) {
   FFTPlan p{};
   return reg_axis_plan(L, p);
 }
-inline bool is_reg_axis(const FFTPlan& p) {
-  FFTPlan q{};
-  return reg_axis_plan(p.L, q) && p.npass == 2 && p.radix[0] == q.radix[0] && p.radix[1] == q.radix[1];
-}
 // a: one launch's arguments (plan.L and plan.tw_off name the length and its
 // twiddles); the batched form reads run r's arguments from args[r] on the device
 template <typename T>
@@ -453,10 +449,6 @@ inline bool has_reg_x(int L) {
   FFTPlan p{};
   return reg_x_plan(L, p);
 }
-inline bool is_reg_x(const FFTPlan& p) {
-  FFTPlan q{};
-  return reg_x_plan(p.L, q) && p.npass == q.npass && std::equal(q.radix, q.radix + q.npass, p.radix);
-}
 template <typename T, class Epi>
 int reg_x(psb_ctx* c, const psb::XEpiArgs<T>& e, const Epi& epi, const char* what, double bytes);
 template <typename T, class Epi>
@@ -490,16 +482,16 @@ int launch_axis(psb_ctx* c, psb::AxisArgs<T> a, Pre pre, const char* what, const
   constexpr int FT = psb::pre_tile_fields<Pre>();                   // fields of a staged tile
   const int outer = a.nouter * psb::pre_tile_groups<Pre>();        // outer indices of the staged grid
   a.col_tile = pick_ct(a.ncols, FT, L, esz, outer);
-  if (sh && sh->tile && !sh->reg) {
+  const bool staged = sh && sh->tile && !sh->reg;  // a shape of the staged pass was asked for
+  if (staged) {
     a.col_tile = sh->tile;
     a.plan = sh->plan;
   }
   const double bytes = (double)esz * a.nouter * a.ncols *
                        ((double)Pre::F_SRC * count_mapped(a.in_map, a.in_rows) + (double)Pre::F_DST * a.out_rows);
-  // the register pass of this length (psb_reg.cuh), where there is one; a tuned shape's tile and
-  // radices apply to the runtime-schedule kernels of the other lengths
+  // the register pass of this length (psb_reg.cuh), where there is one
   if constexpr (psb::pre_has_fields<Pre>::value) {
-    if (has_reg_axis(L)) return reg_axis<T>(c, a, pre.fields(), INV, what, bytes);
+    if (has_reg_axis(L) && !staged) return reg_axis<T>(c, a, pre.fields(), INV, what, bytes);
   }
   const size_t smem = (size_t)(L + 2 * L * FT * a.col_tile) * esz;
   dim3 grid((a.ncols + a.col_tile - 1) / a.col_tile, outer);
@@ -518,7 +510,7 @@ int launch_axis(psb_ctx* c, psb::AxisArgs<T> a, Pre pre, const char* what, const
     // every box lands on a 128-byte boundary: the buffer's start, and box b at b*(L/nbox) rows
     const bool boxes_aligned = nbox == 1 || ((size_t)(L / nbox) * a.col_tile * esz) % 128 == 0;
     if (c->use_tma && plain_rows && nbox > 0 && boxes_aligned && (a.col_tile * esz) % 16 == 0 &&
-        !(sh && sh->wide)) {
+        !(staged && sh->wide)) {
       const long long dims[4] = {a.ncols, 1, a.in_rows, a.nouter};
       const long long strides[3] = {a.in_rstride, a.in_rstride, a.in_ostride};
       const int box[4] = {a.col_tile, 1, L / nbox, 1};
@@ -535,7 +527,7 @@ int launch_axis(psb_ctx* c, psb::AxisArgs<T> a, Pre pre, const char* what, const
     }
   }
   if constexpr (TUNABLE) {
-    if (sh && sh->wide) return go(psb::axis_pass_kernel<T, INV, Pre, true>);
+    if (staged && sh->wide) return go(psb::axis_pass_kernel<T, INV, Pre, true>);
   }
   return go(psb::axis_pass_kernel<T, INV, Pre>);
 }
@@ -553,8 +545,8 @@ int launch_z(psb_ctx* c, psb::ZArgs<T> z, Phys phys, const char* what, double ex
   // a field formed as d/dz of another input re-reads that input's line: no new bytes
   for (int f = 0; f < Phys::F_IN; ++f)
     if (!z.dz[f] || z.in2[f]) bytes += (double)esz * z.npencils * z.in_kz[f];
-  // the register z pass of this length (psb_zreg.cuh), where there is one; a tuned shape applies to
-  // the staged one
+  // the register z pass of this length (psb_zreg.cuh), where there is one and psb_ctx_set_zrr has not
+  // switched it off; a shape applies to the staged one
   if constexpr (z_registered<Phys>::value)
     if (c->use_zrr && has_reg_z<T, Phys>(M)) return reg_z<T, Phys>(c, z, phys, what, bytes);
   int P = psb::phys_default_ppc<Phys>::value;
@@ -586,17 +578,17 @@ int launch_epi(psb_ctx* c, psb::XEpiArgs<T> e, Epi epi, const char* what, const 
   const size_t esz = sizeof(Cx<T>);
   const int L = e.plan.L;
   const double bytes = epi.io_bytes((long long)e.n1 * e.n2 * e.n3h) + (double)esz * Epi::F_IN * L * e.n2 * e.kz;
-  // the register pass of this length (psb_xreg.cuh), where there is one; a tuned shape applies to
-  // the staged ones of the other lengths
+  const bool staged = sh && sh->tile && !sh->reg;  // a shape of the staged pass was asked for
+  // the register pass of this length (psb_xreg.cuh), where there is one
   if constexpr (x_registered<Epi>::value)
-    if (has_reg_x(L)) return reg_x<T, Epi>(c, e, epi, what, bytes);
+    if (has_reg_x(L) && !staged) return reg_x<T, Epi>(c, e, epi, what, bytes);
   int extra = 0;
   if (e.n3h > e.kz) {
     const long long pts = (long long)e.n1 * e.n2 * (e.n3h - e.kz);
     extra = (int)std::min<long long>((pts + 255) / 256, 1024);
   }
   e.col_tile = pick_ct(e.kz, Epi::F_IN, L, esz, e.n2);
-  if (sh && sh->tile && !sh->reg) {
+  if (staged) {
     e.col_tile = sh->tile;
     e.plan = sh->plan;
   }
@@ -614,7 +606,7 @@ int launch_epi(psb_ctx* c, psb::XEpiArgs<T> e, Epi epi, const char* what, const 
     const int nbox = tma_boxes(L);
     CUtensorMap map;
     const bool boxes_aligned = nbox == 1 || ((size_t)(L / nbox) * Epi::F_IN * e.col_tile * esz) % 128 == 0;
-    if (c->use_tma && nbox > 0 && boxes_aligned && (e.col_tile * esz) % 16 == 0 && !(sh && sh->wide)) {
+    if (c->use_tma && nbox > 0 && boxes_aligned && (e.col_tile * esz) % 16 == 0 && !(staged && sh->wide)) {
       const long long dims[4] = {e.kz, Epi::F_IN, L, e.n2};
       const long long strides[3] = {e.in_fstride, e.in_rstride, e.in_ostride};
       const int box[4] = {e.col_tile, Epi::F_IN, L / nbox, 1};
@@ -632,7 +624,7 @@ int launch_epi(psb_ctx* c, psb::XEpiArgs<T> e, Epi epi, const char* what, const 
     }
   }
   if constexpr (TUNABLE) {
-    if (sh && sh->wide) return go(psb::xfwd_epi_kernel<T, Epi, true>);
+    if (staged && sh->wide) return go(psb::xfwd_epi_kernel<T, Epi, true>);
   }
   return go(psb::xfwd_epi_kernel<T, Epi>);
 }

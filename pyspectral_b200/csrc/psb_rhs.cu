@@ -2121,8 +2121,8 @@ int tune_rhs(psb_ctx* c, int closure, const void* state, const psb_params* p) {
   for (int k = 0; k < 5 && status == PSB_OK; ++k) {
     psb_pass_shape& cur = c->tuned[closure].pass[k];
     const psb_pass_shape inc = cur;
-    // a register pass has one shape (the runtime-schedule shapes of its length are slower throughout)
-    if (inc.reg) continue;
+    // the register z pass is chosen by psb_ctx_set_zrr, not by a shape
+    if (k == 2 && inc.reg) continue;
     float base = 0.f;
     if ((status = time_pass(k, 6, &base)) != PSB_OK) break;
     std::vector<int> tiles;
@@ -2137,10 +2137,11 @@ int tune_rhs(psb_ctx* c, int closure, const void* state, const psb_params* p) {
     psb_pass_shape best = inc;
     float bms = 0.97f * base;
     for (int tl : tiles) {
-      for (const FFTPlan& q2 : radix_orders(inc.plan)) {
+      for (const FFTPlan& q2 : radix_orders(*plan_for(c, Ls[k]))) {
         cur.tile = tl;
         cur.plan = q2;
         cur.wide = plan_is_wide(q2);
+        cur.reg = false;
         float ms = 0.f;
         if ((status = time_pass(k, 6, &ms)) != PSB_OK) break;
         if (ms < bms) {
@@ -2152,7 +2153,7 @@ int tune_rhs(psb_ctx* c, int closure, const void* state, const psb_params* p) {
     }
     if (status != PSB_OK) break;
     cur = best;
-    if (best.tile != inc.tile || best.plan.npass != inc.plan.npass ||
+    if (best.reg != inc.reg || best.tile != inc.tile || best.plan.npass != inc.plan.npass ||
         !std::equal(best.plan.radix, best.plan.radix + best.plan.npass, inc.plan.radix)) {
       float again = 0.f, def = 0.f;
       if ((status = time_pass(k, 10, &again)) != PSB_OK) break;
@@ -2170,6 +2171,8 @@ int tune_rhs(psb_ctx* c, int closure, const void* state, const psb_params* p) {
 // A caller-given launch shape for pass k of `closure` (a saved autotuner
 // result, or a shape a test wants to exercise): checked against the pass's
 // transform length, the radices the kernels have and the shared-memory budget.
+bool staged_radix(int r) { return r == 2 || r == 3 || r == 4 || r == 6 || r == 8 || r == 12 || r == 16; }
+
 template <typename T>
 int set_shape(psb_ctx* c, int closure, int k, int tile, const int* radices, int nrad) {
   const TuneDims td = tune_dims<T>(c, closure, PSB_ACT_RELU, 32);
@@ -2179,15 +2182,17 @@ int set_shape(psb_ctx* c, int closure, int k, int tile, const int* radices, int 
   bool wide = false;
   FFTPlan q = *plan_for(c, L);
   q.npass = nrad;
-  // the register pass's own radices name it (its tile is fixed)
+  // the register pass is named by its radices and its tile, or by its radices alone
+  // where the staged passes do not have them
   FFTPlan rp = q;
-  bool reg_shape = (k != 2 && k != 4) && nrad == 2 && reg_axis_plan(L, rp) &&
-                   radices[0] == rp.radix[0] && radices[1] == rp.radix[1];
-  if (k == 4)
-    reg_shape = reg_x_plan(L, rp) && nrad == rp.npass && std::equal(radices, radices + nrad, rp.radix);
-  if (k == 2)
+  bool reg_shape = false;
+  if (k == 2) {
     reg_shape = td.zP > 0 && nrad == 3 && std::equal(radices, radices + 3, td.zplan.radix) && tile >= 1 &&
                 tile <= 128;
+  } else if (k == 4 ? reg_x_plan(L, rp) : reg_axis_plan(L, rp)) {
+    reg_shape = nrad == rp.npass && std::equal(radices, radices + nrad, rp.radix) &&
+                (tile == (k == 4 ? xreg_cols<T>() : reg_cols<T>()) || !std::all_of(radices, radices + nrad, staged_radix));
+  }
   for (int s = 0; s < nrad; ++s) {
     const int r = radices[s];
     if (reg_shape) {
@@ -2195,7 +2200,7 @@ int set_shape(psb_ctx* c, int closure, int k, int tile, const int* radices, int 
       prod *= r;
       continue;
     }
-    if (r != 2 && r != 3 && r != 4 && r != 6 && r != 8 && r != 12 && r != 16)
+    if (!staged_radix(r))
       return fail(c, PSB_ERR_ARG, "psb_set_tuned_shape: radices must be 2, 3, 4, 6, 8, 12 or 16");
     wide = wide || r > 8 || r == 6;
     prod *= r;
@@ -2220,7 +2225,7 @@ int set_shape(psb_ctx* c, int closure, int k, int tile, const int* radices, int 
     for (int j : {0, 1, 3, 4}) default_pass_shape<T>(c, td, j, t.pass[j]);
     t.pass[2].tile = td.zP ? td.zP : P;
     t.pass[2].plan = td.zplan;
-  t.pass[2].reg = td.zP > 0;
+    t.pass[2].reg = td.zP > 0;
     it = c->tuned.emplace(closure, t).first;
   }
   psb_pass_shape& sh = it->second.pass[k];
