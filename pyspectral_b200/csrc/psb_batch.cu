@@ -6,8 +6,9 @@
 //
 // Launch shapes are chosen by an autotuner: for every pass it times the
 // candidate column tiles (x/y passes), pencils per CTA (z-pass) and radix
-// orders of the transform length on the batch's own data, and keeps the
-// fastest.  Timing reads the runs' states and writes only scratch (the last
+// orders of the staged pass on the batch's own data and keeps the fastest, then
+// times the register pass of the length, where there is one, against it.  The
+// persistent ensemble runs the staged shapes.  Timing reads the runs' states and writes only scratch (the last
 // pass runs a middle-stage update on scratch copies), so tuning leaves the
 // runs' states untouched.
 #include <algorithm>
@@ -32,10 +33,15 @@ struct psb_batch {
   void* dargs = nullptr;  // device argument blocks
   size_t dargs_bytes = 0;
   bool dirty = true;
-  // launch shape per pass: 0 x-inverse, 1 y-inverse, 2 z, 3 y-forward, 4 x-forward
+  // shape of the staged pass: 0 x-inverse, 1 y-inverse, 2 z, 3 y-forward, 4 x-forward
+  // (the batched launches where a pass runs staged, and the persistent ensemble)
   std::array<int, 5> tile{{0, 0, 0, 0, 0}};
   std::array<FFTPlan, 5> plan{};
-  bool tuned = false;
+  // shape of the register pass (plan.L 0: the length has none)
+  std::array<int, 5> rtile{{0, 0, 0, 0, 0}};
+  std::array<FFTPlan, 5> rplan{};
+  std::array<bool, 5> staged{};  // the staged pass is the one chosen for the batched launches
+  bool runs_reg(int pass) const { return rplan[pass].L != 0 && !staged[pass] && (pass != 2 || c->use_zrr); }
   std::vector<char> host;  // staging of the argument blocks
 };
 
@@ -139,46 +145,21 @@ struct Batch {
   static constexpr bool reg_pass(int pass) {
     return pass == 0 ? has_fields<Pre>() : (pass == 1 ? has_fields<YPre>() : pass == 3);
   }
-  // The z pass runs as a register pass (its plan is the register pass's {A, B, 2}).
-  bool reg_z_pass() const {
-    FFTPlan q{};
-    if constexpr (z_registered<Phys>::value) {
-      if (!has_reg_z<T, Phys>(d.M3)) return false;
-      reg_z_shape<T, Phys>(d.M3, (long long)d.M1 * d.M2 * R, q);
-      return b->plan[2].npass == q.npass && std::equal(q.radix, q.radix + q.npass, b->plan[2].radix);
+  // The register passes' shapes (psb_batch::rtile, rplan).
+  void register_shapes() const {
+    const int Ls[5] = {d.M1, d.M2, d.M3, d.M2, d.M1};
+    for (int k : {0, 1, 3, 4}) {
+      FFTPlan p = *plan_for(c, Ls[k]);
+      b->rplan[k] = FFTPlan{};
+      if (k == 4 ? !reg_x_plan(Ls[k], p) : !(reg_pass(k) && reg_axis_plan(Ls[k], p))) continue;
+      b->rplan[k] = p;
+      b->rtile[k] = k == 4 ? xreg_cols<T>() : reg_cols<T>();
     }
-    return false;
+    b->rplan[2] = FFTPlan{};
+    if constexpr (z_registered<Phys>::value)
+      if (has_reg_z<T, Phys>(d.M3))
+        b->rtile[2] = reg_z_shape<T, Phys>(d.M3, (long long)d.M1 * d.M2 * R, b->rplan[2]);
   }
-  // The same for the x-forward pass.
-  void generic_x(int& tile, FFTPlan& plan) const {
-    tile = b->tile[4];
-    plan = b->plan[4];
-    if (is_reg_x(plan)) default_x_shape<T>(c, plan.L, d.Kz, Fo, d.N2, false, tile, plan);
-  }
-  // Pencils per CTA and plan of the staged z pass: the pass's own shape, or the default
-  // where the register pass runs (the persistent ensemble runs the staged one).
-  void generic_z(int& P, FFTPlan& plan) const {
-    P = b->tile[2];
-    plan = b->plan[2];
-    if (!reg_z_pass()) return;
-    plan = *plan_for(c, d.M3);
-    P = phys_default_ppc<Phys>::value;
-    while (P > 1 && smem_z(P) > kSmemBudget) P /= 2;
-    const long long np = (long long)d.M1 * d.M2;
-    while (P > 1 && (np + P - 1) / P * R < 2 * 148) P /= 2;
-  }
-  // Column tile and plan in the argument blocks of axis pass `pass`: the pass's own shape, or,
-  // where the pass runs as a register pass (which takes neither), the default of the
-  // runtime-schedule bodies that the persistent ensemble runs on the same blocks.
-  void generic_shape(int pass, int& tile, FFTPlan& plan) const {
-    tile = b->tile[pass];
-    plan = b->plan[pass];
-    if (!reg_pass(pass) || !is_reg_axis(plan)) return;
-    const int F = pass == 0 ? Fi : (pass == 1 ? Fy : 1);
-    const int no = pass == 0 ? d.N2 : (pass == 1 ? Gy * d.M1 : Fo * d.M1);
-    default_axis_shape<T>(c, plan.L, d.Kz, F, no, false, tile, plan);
-  }
-
   // Argument blocks of every run (host copy, then one upload).
   int build(const Pre& pre0, Phys (*mkphys)(psb_ctx*, const psb_params&),
             Epi (*mkepi)(psb_ctx*, StepIO<T>, const psb_params&)) {
@@ -192,7 +173,8 @@ struct Batch {
       const Cx<T>* Q = reinterpret_cast<const Cx<T>*>(b->state[r]);
       Cx<T>*A = run_buf(r, 0), *B = run_buf(r, 1), *C = run_buf(r, 2), *D = run_buf(r, 3);
       AxisArgs<T> a{};
-      generic_shape(0, a.col_tile, a.plan);
+      a.col_tile = b->tile[0];
+      a.plan = b->plan[0];
       a.tw = twiddles<T>(c);
       a.scale = (T)1;
       a.in = Q;
@@ -214,7 +196,8 @@ struct Batch {
       a.k_col = c->kz;
       ax[r] = a;
       AxisArgs<T> y{};
-      generic_shape(1, y.col_tile, y.plan);
+      y.col_tile = b->tile[1];
+      y.plan = b->plan[1];
       y.tw = twiddles<T>(c);
       y.scale = (T)1;
       y.in = A;
@@ -242,12 +225,14 @@ struct Batch {
       }
       z.out_kz = d.Kz;
       z.npencils = (long long)d.M1 * d.M2;
-      generic_z(z.ppc, z.plan);
+      z.ppc = b->tile[2];
+      z.plan = b->plan[2];
       z.fac = (T)(s32 / ((double)d.M1 * d.M2 * d.M3));
       z.tw = twiddles<T>(c);
       az[r] = z;
       AxisArgs<T> yf{};
-      generic_shape(3, yf.col_tile, yf.plan);
+      yf.col_tile = b->tile[3];
+      yf.plan = b->plan[3];
       yf.tw = twiddles<T>(c);
       yf.scale = (T)1;
       yf.in = C;
@@ -272,7 +257,8 @@ struct Batch {
       e.n2 = d.N2;
       e.n3h = d.N3h;
       e.kz = d.Kz;
-      generic_x(e.col_tile, e.plan);
+      e.col_tile = b->tile[4];
+      e.plan = b->plan[4];
       e.out_map = map_pad32(d.N1);
       e.main_blocks = ((d.Kz + e.col_tile - 1) / e.col_tile) * d.N2;
       e.tw = twiddles<T>(c);
@@ -339,14 +325,15 @@ struct Batch {
       if (p.radix[s] > 8 || p.radix[s] == 6) return true;
     return false;
   }
+  // reg: the register pass, else the staged one
   template <bool W>
-  int launch_w(int pass, int stage) {
+  int launch_w(int pass, int stage, bool reg) {
     const size_t esz = sizeof(Cx<T>);
     switch (pass) {
       case 0: {
         const double by = (double)R * esz * d.N2 * d.Kz * (3.0 * d.N1 + (double)Fi * d.M1);
         if constexpr (has_fields<Pre>())
-          if (is_reg_axis(b->plan[0]))
+          if (reg)
             return reg_axis_batch<T>(c, ax, Pre{}.fields(), d.M1, d.Kz, d.N2, R, true, "batch x-inverse", by);
         const int ct = b->tile[0];
         dim3 g((d.Kz + ct - 1) / ct, d.N2, R);
@@ -366,7 +353,7 @@ struct Batch {
         // y-inverse, register form: YP::groups outer groups of YPre::F_DST fields
         const int G = inv ? YP::groups : Fo, F = inv ? Fb : Fo;
         const double by = (double)R * esz * F * d.M1 * d.Kz * (double)(d.N2 + d.M2);
-        if (is_reg_axis(b->plan[pass])) {
+        if (reg) {
           if (!inv)
             return reg_axis_batch<T>(c, ayf, PreCopy<T>{}.fields(), d.M2, d.Kz, G * d.M1, R, false, "batch y-forward",
                                      by);
@@ -396,7 +383,7 @@ struct Batch {
         const int P = b->tile[2];
         const long long np = (long long)d.M1 * d.M2;
         if constexpr (z_registered<Phys>::value)
-          if (reg_z_pass())
+          if (reg)
             return reg_z_batch<T, Phys>(c, az, phys, d.M3, np, R, "batch z-fused",
                                         (double)R * esz * np * d.Kz * (Fb + Fo));
         const long long items = (np + P - 1) / P * R;
@@ -416,7 +403,7 @@ struct Batch {
         const int extra = (int)std::min<long long>((pts + 255) / 256, 1024);
         const double by = (double)R * (esz * Fo * d.M1 * d.N2 * d.Kz + esz * 3.0 * d.N1 * d.N2 * d.N3h *
                                                                            3.0);
-        if (is_reg_x(b->plan[4]))
+        if (reg)
           return reg_x_batch<T, Epi>(c, ae, epi + (size_t)stage * R, d.M1, d.Kz, d.N1, d.N2, d.N3h, R,
                                      "batch x-forward+epilogue", by);
         const int ct = b->tile[4];
@@ -435,7 +422,10 @@ struct Batch {
     }
   }
 
-  int launch(int pass, int stage) { return wide(pass) ? launch_w<true>(pass, stage) : launch_w<false>(pass, stage); }
+  int launch(int pass, int stage, bool reg) {
+    return wide(pass) ? launch_w<true>(pass, stage, reg) : launch_w<false>(pass, stage, reg);
+  }
+  int launch(int pass, int stage) { return launch(pass, stage, b->runs_reg(pass)); }
 
   int step(int nsteps) {
     for (int s = 0; s < nsteps; ++s)
@@ -446,14 +436,14 @@ struct Batch {
 
   // ---- autotuning -----------------------------------------------------------
   // Mean time of `reps` launches of one pass (RHS-mode epilogue), ms.
-  int time_pass(int pass, int reps, float* ms) {
+  int time_pass(int pass, int reps, float* ms, bool reg = false) {
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
-    int st = launch(pass, 4);  // warm-up (and shape check)
+    int st = launch(pass, 4, reg);  // warm-up (and shape check)
     if (st == PSB_OK) {
       cudaEventRecord(e0, c->stream);
-      for (int k = 0; k < reps && st == PSB_OK; ++k) st = launch(pass, 4);
+      for (int k = 0; k < reps && st == PSB_OK; ++k) st = launch(pass, 4, reg);
       cudaEventRecord(e1, c->stream);
       cudaEventSynchronize(e1);
       cudaEventElapsedTime(ms, e0, e1);
@@ -472,11 +462,8 @@ struct Batch {
     // RHS-mode passes read the runs' states and write only scratch; run one
     // full RHS first so that every intermediate buffer holds real data.
     for (int pass = 0; pass < 5; ++pass) PSB_TRY(launch(pass, 4));
+    // the staged shapes first, then the register pass against the staged one kept
     for (int pass = 0; pass < 5; ++pass) {
-      // a register pass has one shape (the runtime-schedule shapes of its length are slower throughout)
-      if (pass == 2 ? reg_z_pass()
-                    : (pass == 4 ? is_reg_x(b->plan[4]) : reg_pass(pass) && is_reg_axis(b->plan[pass])))
-        continue;
       std::vector<int> tiles;
       if (pass == 2) {
         for (int P : {1, 2, 4, 8})
@@ -524,9 +511,14 @@ struct Batch {
           PSB_TRY(build(pre0, mkphys, mkepi));
         }
       }
+      if (b->rplan[pass].L != 0) {
+        float reg = 0, stg = 0;
+        PSB_TRY(time_pass(pass, 10, &reg, true));
+        PSB_TRY(time_pass(pass, 10, &stg));
+        b->staged[pass] = stg < 0.97f * reg;
+      }
     }
     (void)esz;
-    b->tuned = true;
     return PSB_OK;
   }
 };
@@ -557,20 +549,17 @@ EpiSmagStep<T> mk_epi_smag(psb_ctx* c, StepIO<T> io, const psb_params& p) {
   return EpiSmagStep<T>{io, ktab<T>(c->kx, c->ky, c->kz), (T)p.nu, p.rotate, (T)p.Om1, (T)p.Om2, (T)p.Om3};
 }
 
-// Default launch shapes: the single-run rules of the library.
+// Default staged shapes: the single-run rules of the library.
 // Fz: z-pass inputs (with the fields it derives itself); Fy / Gy: lines per
-// column and outer groups of the y-inverse pass; reg: which passes have a
-// register form
-template <typename T>
-void default_shapes(psb_batch* b, int Fi, int Fb, int Fz, int Fo, int Fy, int Gy, bool (*reg)(int), int ppc,
+// column and outer groups of the y-inverse pass
+void default_shapes(psb_batch* b, int Fi, int Fb, int Fz, int Fo, int Fy, int Gy, size_t esz, int ppc,
                     size_t zextra) {
   psb_ctx* c = b->c;
-  const size_t esz = sizeof(Cx<T>);
   const Dims d = dims(c, Fi, Fb, Fo);
-  default_axis_shape<T>(c, d.M1, d.Kz, Fi, d.N2, reg(0), b->tile[0], b->plan[0]);
-  default_axis_shape<T>(c, d.M2, d.Kz, Fy, Gy * d.M1, reg(1), b->tile[1], b->plan[1]);
-  default_axis_shape<T>(c, d.M2, d.Kz, 1, Fo * d.M1, reg(3), b->tile[3], b->plan[3]);
-  default_x_shape<T>(c, d.M1, d.Kz, Fo, d.N2, true, b->tile[4], b->plan[4]);
+  b->tile[0] = pick_ct(d.Kz, Fi, d.M1, esz, d.N2);
+  b->tile[1] = pick_ct(d.Kz, Fy, d.M2, esz, Gy * d.M1);
+  b->tile[3] = pick_ct(d.Kz, 1, d.M2, esz, Fo * d.M1);
+  b->tile[4] = pick_ct(d.Kz, Fo, d.M1, esz, d.N2);
   const int FMAX = std::max(Fz, Fo);
   int P = ppc;
   auto sm = [&](int P) { return (size_t)(d.M3 + 2 * (size_t)((FMAX * P + 1) / 2) * d.M3) * esz + zextra; };
@@ -579,7 +568,11 @@ void default_shapes(psb_batch* b, int Fi, int Fb, int Fz, int Fo, int Fy, int Gy
   const long long np = (long long)d.M1 * d.M2;
   while (P > 1 && (np + P - 1) / P * b->nruns < 2 * 148) P /= 2;
   b->tile[2] = P;
+  b->plan[0] = *plan_for(c, d.M1);
+  b->plan[1] = *plan_for(c, d.M2);
   b->plan[2] = *plan_for(c, d.M3);
+  b->plan[3] = *plan_for(c, d.M2);
+  b->plan[4] = *plan_for(c, d.M1);
 }
 
 template <typename T, class Pre, class Phys, class Epi>
@@ -601,11 +594,9 @@ int run_batch(psb_batch* b, int nsteps, bool tune, Pre pre0, Phys (*mkphys)(psb_
     b->arena_bytes = need;
   }
   if (b->plan[0].L == 0) {
-    default_shapes<T>(b, BT::Fi, BT::Fb, Phys::F_IN, BT::Fo, BT::Fy, BT::Gy, &BT::reg_pass,
+    default_shapes(b, BT::Fi, BT::Fb, Phys::F_IN, BT::Fo, BT::Fy, BT::Gy, sizeof(Cx<T>),
                    phys_default_ppc<Phys>::value, (size_t)phys_is_block<Phys>::extra);
-    if constexpr (z_registered<Phys>::value)
-      if (c->use_zrr && has_reg_z<T, Phys>(x.d.M3))
-        b->tile[2] = reg_z_shape<T, Phys>(x.d.M3, (long long)x.d.M1 * x.d.M2 * x.R, b->plan[2]);
+    x.register_shapes();
   }
   if (b->dirty) {
     PSB_TRY(x.build(pre0, mkphys, mkepi));
@@ -758,17 +749,7 @@ size_t ens_group(psb_batch* b, int kind, EnsGroup& g) {
   g.cpy = x.cpy;
   g.phys = x.phys;
   g.epi = x.epi;
-  // the tiles in the argument blocks (the runtime-schedule bodies run here)
-  std::array<int, 5> t = b->tile;
-  for (int k : {0, 1, 3}) {
-    FFTPlan plan;
-    x.generic_shape(k, t[k], plan);
-  }
-  {
-    FFTPlan plan;
-    x.generic_z(t[2], plan);
-    x.generic_x(t[4], plan);
-  }
+  const int* t = b->tile.data();
   g.nx[0] = (d.Kz + t[0] - 1) / t[0];
   g.ny[0] = d.N2;
   g.nx[1] = (d.Kz + t[1] - 1) / t[1];
@@ -854,8 +835,8 @@ int psb_batch_step_rk4(psb_batch* b, int nsteps) {
 
 int psb_batch_shape(const psb_batch* b, int pass, int* tile, int* radices, int maxr) {
   if (!b || pass < 0 || pass > 4 || !tile) return PSB_ERR_ARG;
-  *tile = b->tile[pass];
-  const FFTPlan& p = b->plan[pass];
+  *tile = b->runs_reg(pass) ? b->rtile[pass] : b->tile[pass];
+  const FFTPlan& p = b->runs_reg(pass) ? b->rplan[pass] : b->plan[pass];
   for (int s = 0; s < maxr; ++s) radices[s] = s < p.npass ? p.radix[s] : 0;
   return PSB_OK;
 }
