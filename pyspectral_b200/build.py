@@ -23,11 +23,6 @@ LIB = os.path.join(HERE, "libpyspectral_b200.so")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 FLAGS = ARCH + ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr",
                 "-Xcompiler", "-Wno-deprecated-declarations"]
-# The files that instantiate the register passes hold hundreds of kernels each: ptxas works on
-# them in four threads.  The others keep the one-thread allocation, which gives large kernels
-# fewer spills (persistent ensemble FP32 216 bytes against 312) and the small ones the register
-# counts that their grids are sized for.
-SPLIT = ["-split-compile=4"]
 
 
 def nvcc() -> str:
@@ -63,8 +58,7 @@ def build(force: bool = False, extra_flags=None, verbose: bool = False) -> str:
         obj = os.path.join(BUILD, os.path.basename(src)[:-3] + ".o")
         objs.append(obj)
         if force or _stale(obj, [src] + deps):
-            split = SPLIT if os.path.basename(src).startswith(("psb_x_", "psb_z_", "psb_axis_")) else []
-            jobs.append([nv] + flags + split + ["-c", src, "-o", obj])
+            jobs.append([nv] + flags + ["-c", src, "-o", obj])
 
     def run(cmd):
         r = subprocess.run(cmd, capture_output=True, text=True)
