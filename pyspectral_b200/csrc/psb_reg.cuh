@@ -149,7 +149,8 @@ __device__ __forceinline__ void axis_reg_body(const AxisArgs<T>& a, const FieldT
 template <typename T, int A>
 constexpr int axis_reg_minb() {
   constexpr int regs = A * (int)sizeof(Cx<T>) / 4 + (sizeof(T) == 4 ? 36 : 56);
-  constexpr int b = 65536 / (regs * A * reg_cols<T>());
+  constexpr int nt = (A * reg_cols<T>() + 31) / 32 * 32;
+  constexpr int b = 65536 / (regs * nt);
   return b < 1 ? 1 : (b > 16 ? 16 : b);
 }
 
