@@ -155,6 +155,7 @@ struct Batch {
       b->rplan[k] = p;
       b->rtile[k] = k == 4 ? xreg_cols<T>() : reg_cols<T>();
     }
+    b->staged[4] = !x_pass_in_registers<T, Epi>(d.M1, d.Kz, d.N2, R);
     b->rplan[2] = FFTPlan{};
     if constexpr (z_registered<Phys>::value)
       if (has_reg_z<T, Phys>(d.M3))

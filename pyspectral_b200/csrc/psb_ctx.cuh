@@ -449,6 +449,43 @@ inline bool has_reg_x(int L) {
   FFTPlan p{};
   return reg_x_plan(L, p);
 }
+// Warps of a block of the register x pass of length L.
+template <typename T>
+inline int x_reg_warps(int L) {
+#define PSB_CASE(LEN, A, B, R) \
+  case LEN:                    \
+    return psb::xreg_threads<T, A, B>() / 32;
+  switch (L) {
+    PSB_REG_X(PSB_CASE)
+    default:
+      return 0;
+  }
+#undef PSB_CASE
+}
+// Whether the x pass of a length with a register form runs it.  A block takes its
+// fields one after another, so a launch that gives an SM few warps is a chain of
+// latencies, where the staged pass has every field's loads in flight at once.  The
+// line, in warps an SM gets from the launch, lies where the two meet: 6 in FP64, 2
+// in FP32 (its small launches share a tile's fields between three groups of
+// threads), 16 and 64 for the MHD epilogue, which reads up to 21 spectra a mode.
+// Staged against register, us: FP64 DNS 48^3 (5.8 warps) 12.6 / 14.4, 64^3 (10)
+// 19.0 / 18.7; Smagorinsky 32^3 (1.7) 10.7 / 16.7, 64^3 33.1 / 24.9; MHD 64^3 (7.8)
+// 24.8 / 37.1, 72^3 (15) 37.2 / 39.0, 96^3 (25) 98 / 90; FP32 MHD 64^3 (8.6)
+// 18.9 / 26.8, 96^3 (27) 45.4 / 49.3; Smagorinsky 24^3 (1) 10.4 / 12.6.
+template <class Epi, class = void>
+struct x_min_warps {
+  static constexpr int f64 = 6, f32 = 2;
+};
+template <class Epi>
+struct x_min_warps<Epi, decltype((void)Epi::X_WARPS64, void())> {
+  static constexpr int f64 = Epi::X_WARPS64, f32 = Epi::X_WARPS32;
+};
+template <typename T, class Epi>
+inline bool x_pass_in_registers(int L, int kz, int n2, int runs = 1) {
+  if (!x_registered<Epi>::value || !has_reg_x(L)) return false;
+  const long long blocks = (long long)((kz + psb::xreg_cols<T>() - 1) / psb::xreg_cols<T>()) * n2 * runs;
+  return blocks * x_reg_warps<T>(L) >= 148LL * (sizeof(T) == 8 ? x_min_warps<Epi>::f64 : x_min_warps<Epi>::f32);
+}
 template <typename T, class Epi>
 int reg_x(psb_ctx* c, const psb::XEpiArgs<T>& e, const Epi& epi, const char* what, double bytes);
 template <typename T, class Epi>
@@ -581,7 +618,7 @@ int launch_epi(psb_ctx* c, psb::XEpiArgs<T> e, Epi epi, const char* what, const 
   const bool staged = sh && sh->tile && !sh->reg;  // a shape of the staged pass was asked for
   // the register pass of this length (psb_xreg.cuh), where there is one
   if constexpr (x_registered<Epi>::value)
-    if (has_reg_x(L) && !staged) return reg_x<T, Epi>(c, e, epi, what, bytes);
+    if (sh && sh->tile ? sh->reg : x_pass_in_registers<T, Epi>(L, e.kz, e.n2)) return reg_x<T, Epi>(c, e, epi, what, bytes);
   int extra = 0;
   if (e.n3h > e.kz) {
     const long long pts = (long long)e.n1 * e.n2 * (e.n3h - e.kz);

@@ -489,6 +489,7 @@ __device__ __forceinline__ void acc_mhd(int f, const T* k1, T k2, T k3, const Cx
 template <typename T>
 struct EpiMHD {
   static constexpr int F_IN = 9, NACC = 6;
+  static constexpr int X_WARPS64 = 16, X_WARPS32 = 64;  // x_pass_in_registers
   __host__ double io_bytes(long long npts) const {
     return io.bytes(npts, 6) + (force ? (double)sizeof(Cx<T>) * npts * 3 : 0.0);
   }
@@ -935,6 +936,7 @@ struct EpiMHDT {
 template <typename T, int F>
 struct EpiStore {
   static constexpr int F_IN = F, NACC = 0;  // no sums: put() stores each field's modes as they come
+  static constexpr int X_WARPS64 = 2, X_WARPS32 = 2;  // x_pass_in_registers
   Cx<T>* out;
   long long fstride;
   int n2, n3h;

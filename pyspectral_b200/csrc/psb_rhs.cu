@@ -2054,8 +2054,9 @@ size_t pass_smem(const TuneDims& t, int k, int tile) {
 template <typename T>
 void default_pass_shape(psb_ctx* c, const TuneDims& t, int k, psb_pass_shape& sh) {
   if (k == 4) {
-    default_x_shape<T>(c, t.Ls[4], c->N3 / 2, t.Fs[4], c->N2, true, sh.tile, sh.plan);
-    sh.reg = has_reg_x(t.Ls[4]);
+    // every tunable closure's epilogue has the same line (x_min_warps)
+    sh.reg = x_pass_in_registers<T, EpiNS<T, false>>(t.Ls[4], c->N3 / 2, c->N2);
+    default_x_shape<T>(c, t.Ls[4], c->N3 / 2, t.Fs[4], c->N2, sh.reg, sh.tile, sh.plan);
     return;
   }
   const int nouter = k == 0 ? c->N2 : (k == 1 ? t.Gy * t.Ls[0] : t.Fo * t.Ls[0]);
@@ -2136,6 +2137,16 @@ int tune_rhs(psb_ctx* c, int closure, const void* state, const psb_params* p) {
     }
     psb_pass_shape best = inc;
     float bms = 0.97f * base;
+    if (k == 4 && !inc.reg && has_reg_x(Ls[4])) {  // the register pass where the default is the staged one
+      default_x_shape<T>(c, Ls[4], Kz, Fs[4], N2, true, cur.tile, cur.plan);
+      cur.reg = true;
+      float ms = 0.f;
+      if ((status = time_pass(k, 6, &ms)) != PSB_OK) break;
+      if (ms < bms) {
+        bms = ms;
+        best = cur;
+      }
+    }
     for (int tl : tiles) {
       for (const FFTPlan& q2 : radix_orders(*plan_for(c, Ls[k]))) {
         cur.tile = tl;

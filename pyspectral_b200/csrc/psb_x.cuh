@@ -11,6 +11,17 @@ inline int x_extra_blocks(int n1, int n2, int ncz, int nt) {
   return (int)std::min<long long>((pts + nt - 1) / nt, 4096);
 }
 
+// Blocks up to which a launch takes three groups of threads a tile: every CTA is
+// resident at once (FP32 Smagorinsky 48^3 14.6 us against 22.8 with one group,
+// learned 36^3 10.2 against 12.3); beyond that the groups only take CTAs from an SM
+// that has more to run.  0: never.  FP64 launches this small run the staged pass
+// (x_pass_in_registers), and a block of three groups has at most 1024 threads.
+template <typename T, class Epi, int A, int B, int R>
+constexpr int x_group_wave() {
+  if (sizeof(T) == 8 || Epi::NACC == 0 || 3 * psb::xreg_threads<T, A, B>() > 1024) return 0;
+  return 148 * (psb::xreg_minb<T, Epi, A, B, R>() / 3);
+}
+
 template <typename T, class Epi, int A, int B, int R, int S>
 int launch_reg_xs(psb_ctx* c, const psb::XEpiArgs<T>& e, const Epi& epi, const char* what, double bytes) {
   const int extra = x_extra_blocks(e.n1, e.n2, e.n3h - e.kz, S * psb::xreg_threads<T, A, B>());
@@ -26,13 +37,8 @@ template <typename T, class Epi, int A, int B, int R>
 int launch_reg_x(psb_ctx* c, psb::XEpiArgs<T> e, const Epi& epi, const char* what, double bytes) {
   constexpr int C = psb::xreg_cols<T>();
   e.main_blocks = (e.kz + C - 1) / C * e.n2;
-  // three groups of threads a tile while every CTA of the launch is resident at once
-  // (DNS 32^3 FP64, timed with its launch: 14.9 us with one group, 12.8 with two or
-  // three); beyond that they only take CTAs from an SM that has more to run
-  if constexpr (Epi::NACC > 0 && A * B * R <= 192) {
-    constexpr int wave = 148 * (psb::xreg_minb<T, Epi, A, B, R>() / 3);
-    if (e.main_blocks <= wave) return launch_reg_xs<T, Epi, A, B, R, 3>(c, e, epi, what, bytes);
-  }
+  if constexpr (x_group_wave<T, Epi, A, B, R>() > 0)
+    if (e.main_blocks <= x_group_wave<T, Epi, A, B, R>()) return launch_reg_xs<T, Epi, A, B, R, 3>(c, e, epi, what, bytes);
   return launch_reg_xs<T, Epi, A, B, R, 1>(c, e, epi, what, bytes);
 }
 

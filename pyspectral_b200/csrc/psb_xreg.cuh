@@ -62,7 +62,7 @@ constexpr int xreg_threads() {
 
 // S: groups of threads that share a tile's fields (group g takes fields g, g + S,
 // ...); the partial sums are exchanged at the end and each group finishes 1/S of
-// the rows.  A launch of less than one wave takes S = 3: a third of the serial chain.
+// the rows.  S = 3 is a third of the serial chain (x_groups).
 template <typename T, class Epi, int A, int B, int R, int S>
 __device__ __forceinline__ void xreg_body(const XEpiArgs<T>& a, const Epi& epi, int bx, int gx) {
   constexpr int L = A * B * R, AB = A * B, C = xreg_cols<T>(), NT = xreg_threads<T, A, B>(), F = Epi::F_IN;
@@ -224,17 +224,29 @@ __device__ __forceinline__ void xreg_body(const XEpiArgs<T>& a, const Epi& epi, 
   }
 }
 
-// CTAs per SM the registers are bounded for: 128 (168 from four FP64 sums on) or,
-// in FP32, 104 (128 from four sums on) registers a thread.
+// CTAs per SM the registers are bounded for: 128 registers a thread (168 from four
+// FP64 sums on), in FP32 104 (128 from four sums on).  One CTA more where it is the
+// second and leaves 72 registers (FP64 with four sums: 128), or in FP32 the third of
+// seven or more warps and leaves 96; up to four sums.  The blocks are large, one CTA is
+// a third to a half of an SM.  Measured, one CTA per SM -> two
+// (or two -> three at 108 points): FP32 DNS 192 points 80 -> 60 us (128^3), 216
+// points 111 -> 86 (144^3), 108 points 23 -> 17 (72^3); Smagorinsky 144 points
+// 76 -> 47 (96^3), 192 points 138 -> 107 (128^3).  With six sums the epilogues
+// spill instead, as do blocks of six warps in threes (18 warps are five on a
+// scheduler, 96 registers): two there, DNS 64^3 FP32 38.4 -> 36.2 us a right-hand side.
 template <typename T, class Epi, int A, int B, int R>
 constexpr int xreg_minb() {
+  constexpr int nt = xreg_threads<T, A, B>();
   constexpr int regs = sizeof(T) == 8 ? (Epi::NACC > 3 ? 168 : 128) : (Epi::NACC > 3 ? 128 : 104);
-  constexpr int b = 65536 / (regs * xreg_threads<T, A, B>());
-  return b < 1 ? 1 : (b > 16 ? 16 : b);
+  constexpr int b = 65536 / (regs * nt), left = 65536 / ((b + 1) * nt);
+  constexpr bool more = sizeof(T) == 8 ? Epi::NACC == 4 && b == 1 && left >= 128
+                                       : Epi::NACC <= 4 && ((b == 1 && left >= 72) || (b == 2 && nt >= 224 && left >= 96));
+  if (sizeof(T) == 4 && nt == 192 && b == 3) return 2;
+  return more ? (b < 16 ? b + 1 : 16) : (b < 1 ? 1 : (b > 16 ? 16 : b));
 }
 
-// Shared memory: two buffers a group (and room for the exchanged sums, which
-// are no larger), the middle radix's twiddles.
+// Shared memory: two buffers a group, or the sums that the groups exchange where
+// those are larger (NACC / 2 times the buffers), and the middle radix's twiddles.
 template <typename T, class Epi, int A, int B, int R, int S>
 constexpr size_t xreg_smem() {
   const int bufs = S * 2 * A * B * R * xreg_cols<T>(), sums = S > 1 ? S * Epi::NACC * R * A * B * xreg_cols<T>() : 0;
