@@ -13,8 +13,9 @@ int launch_reg_axis(psb_ctx* c, const psb::AxisArgs<T>& a, const psb::FieldTab<T
   constexpr size_t smem = (size_t)A * B * C * sizeof(Cx<T>);
   set_smem(psb::axis_reg_kernel<T, A, B, INV>, smem);
   LaunchScope scope(c, what, bytes);
-  launch_pdl_if(!std::exchange(c->serial_next, false), psb::axis_reg_kernel<T, A, B, INV>, dim3((a.ncols + C - 1) / C, a.nouter, ft.nf), A * C, smem, c->stream,
-             a, ft);
+  const dim3 grid((a.ncols + C - 1) / C, a.nouter, ft.nf);
+  const bool serial = serial_after_z(scope.after_z, (long long)grid.x * grid.y * grid.z, 148LL * psb::axis_reg_minb<T, A>());
+  launch_pdl_if(!serial, psb::axis_reg_kernel<T, A, B, INV>, grid, A * C, smem, c->stream, a, ft);
   return launch_ok(c, what);
 }
 
@@ -40,8 +41,9 @@ int launch_reg_axis_batch(psb_ctx* c, const psb::AxisArgs<T>* args, const psb::F
   constexpr size_t smem = (size_t)A * B * C * sizeof(Cx<T>);
   set_smem(psb::axis_reg_batch<T, A, B, INV>, smem);
   LaunchScope scope(c, what, bytes);
-  launch_pdl_if(!std::exchange(c->serial_next, false), psb::axis_reg_batch<T, A, B, INV>, dim3((ncols + C - 1) / C * runs, nouter, ft.nf), A * C, smem,
-             c->stream, args, ft);
+  const dim3 grid((ncols + C - 1) / C * runs, nouter, ft.nf);
+  const bool serial = serial_after_z(scope.after_z, (long long)grid.x * grid.y * grid.z, 148LL * psb::axis_reg_minb<T, A>());
+  launch_pdl_if(!serial, psb::axis_reg_batch<T, A, B, INV>, grid, A * C, smem, c->stream, args, ft);
   return launch_ok(c, what);
 }
 

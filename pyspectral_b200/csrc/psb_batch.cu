@@ -394,6 +394,7 @@ struct Batch {
           set_smem(k, sm);
           const long long g = persistent_grid(k, sm, items);
           LaunchScope s(c, "batch z-fused", (double)R * esz * np * d.Kz * (Fb + Fo));
+          c->after_z = kAfterStagedZ;
           launch_pdl(k, dim3((unsigned)g), 256, sm, c->stream, (const ZArgs<T>*)az, (const Phys*)phys, R);
           return launch_ok(c, "batch z-fused");
         };

@@ -68,7 +68,7 @@ struct psb_ctx {
   unsigned long long launches = 0;
   int timing = 0;
   int use_tma = 1;          // stage eligible pass inputs with bulk tensor copies
-  bool serial_next = false; // the next launch follows a z pass that ran alone (launch_after_z)
+  int after_z = 0;          // what the last launch was, to the next one (kAfterNone, ...)
   int use_zrr = 1;          // register z pass where the length has one (0: the staged one)
   int* dstatus = nullptr;   // device status word (a bounded wait gave up), owned
   struct Rec {
@@ -144,11 +144,16 @@ inline cudaEvent_t take_event(psb_ctx* c) {
 }
 
 // Bracket one kernel launch: count it and, when timing is on, record events.
+// psb_ctx::after_z: the launch before was no z pass, a register z pass that ran
+// alone (kPdlBytes), a staged z pass.  Every launch reads it once and clears it.
+enum AfterZ : int { kAfterNone = 0, kAfterLargeZ, kAfterStagedZ };
 struct LaunchScope {
   psb_ctx* c;
   psb_ctx::Rec rec;
   bool on;
-  LaunchScope(psb_ctx* ctx, const char* name, double bytes) : c(ctx), on(ctx->timing != 0) {
+  int after_z;
+  LaunchScope(psb_ctx* ctx, const char* name, double bytes)
+      : c(ctx), on(ctx->timing != 0), after_z(std::exchange(ctx->after_z, (int)kAfterNone)) {
     ++c->launches;
     if (on) {
       rec.name = name;
@@ -305,6 +310,15 @@ inline long long persistent_grid(K kernel, size_t smem, long long ntiles, int bl
 // 256^3 FP32 10.2 against 9.2.  Passes whose data stay in L2 are short and gain from
 // it (32^3 FP64 159 -> 135 us a step, 64^3 Smagorinsky FP64 582 -> 565).
 constexpr double kPdlBytes = 126e6;
+// The same for a register axis pass behind a staged z pass (psb_fft_r2c, psb_fft_c2r):
+// it waits for the z pass to end when its CTAs are one wave, all of which would
+// start under the z pass's carveout.  64^3 FP64, 320 CTAs: r2c of three fields 51.7
+// us with the overlap, 43.2 without, c2r 59.5 and 49.3; 128^3, several waves:
+// 167 and 173, 173 and 178.  Less than a CTA per SM gains from the overlap (32^3).
+// blocks: CTAs of the launch, resident: CTAs the device holds.
+inline bool serial_after_z(int after, long long blocks, long long resident) {
+  return after == kAfterLargeZ || (after == kAfterStagedZ && blocks > 148 && blocks <= resident);
+}
 
 inline int pow2_floor(int x) {
   int p = 1;
@@ -600,6 +614,7 @@ int launch_z(psb_ctx* c, psb::ZArgs<T> z, Phys phys, const char* what, double ex
     set_smem(k, smem);
     const long long g = persistent_grid(k, smem, grid);
     LaunchScope scope(c, what, bytes);
+    c->after_z = kAfterStagedZ;
     launch_pdl(k, dim3((unsigned)g), 256, smem, c->stream, z, phys);
     return launch_ok(c, what);
   };

@@ -61,8 +61,9 @@ int launch_reg_zp(psb_ctx* c, const psb::ZArgs<T>& z, const Phys& phys, const ch
   const long long g = persistent_grid(k, smem, (z.npencils + P - 1) / P * psb::Mid<Phys>::JOBS,
                                       psb::ZPlan<T, A, B>::NT);
   LaunchScope scope(c, what, bytes);
-  c->serial_next = bytes > kPdlBytes;
-  launch_pdl_if(!c->serial_next, k, dim3((unsigned)g), psb::ZPlan<T, A, B>::NT, smem, c->stream, z, phys, P);
+  const bool alone = bytes > kPdlBytes;
+  c->after_z = alone ? kAfterLargeZ : kAfterNone;
+  launch_pdl_if(!alone, k, dim3((unsigned)g), psb::ZPlan<T, A, B>::NT, smem, c->stream, z, phys, P);
   return launch_ok(c, what);
 }
 
@@ -89,8 +90,9 @@ int launch_reg_z_batch(psb_ctx* c, const psb::ZArgs<T>* args, const Phys* phys, 
   const long long g = persistent_grid(k, smem, (npencils + P - 1) / P * psb::Mid<Phys>::JOBS * runs,
                                       psb::ZPlan<T, A, B>::NT);
   LaunchScope scope(c, what, bytes);
-  c->serial_next = bytes > kPdlBytes;
-  launch_pdl_if(!c->serial_next, k, dim3((unsigned)g), psb::ZPlan<T, A, B>::NT, smem, c->stream, args, phys, runs, P);
+  const bool alone = bytes > kPdlBytes;
+  c->after_z = alone ? kAfterLargeZ : kAfterNone;
+  launch_pdl_if(!alone, k, dim3((unsigned)g), psb::ZPlan<T, A, B>::NT, smem, c->stream, args, phys, runs, P);
   return launch_ok(c, what);
 }
 
