@@ -169,6 +169,7 @@ struct Batch {
     views(b->host.data());
     const long long fsN = (long long)d.N1 * d.N2 * d.N3h;
     const double s32 = std::sqrt(std::pow(1.5, 3) * std::sqrt((double)d.N1 * d.N2 * d.N3));
+    const double fac = s32 / ((double)d.M1 * d.M2 * d.M3), fsc = field_scale(fac);
     const double rk[4] = {1. / 4, 1. / 3, 1. / 2, 1.};
     for (int r = 0; r < R; ++r) {
       const Cx<T>* Q = reinterpret_cast<const Cx<T>*>(b->state[r]);
@@ -200,7 +201,7 @@ struct Batch {
       y.col_tile = b->tile[1];
       y.plan = b->plan[1];
       y.tw = twiddles<T>(c);
-      y.scale = (T)1;
+      y.scale = (T)fsc;
       y.in = A;
       y.out = B;
       y.in_ostride = (long long)d.N2 * d.Kz;
@@ -228,7 +229,7 @@ struct Batch {
       z.npencils = (long long)d.M1 * d.M2;
       z.ppc = b->tile[2];
       z.plan = b->plan[2];
-      z.fac = (T)(s32 / ((double)d.M1 * d.M2 * d.M3));
+      z.fac = (T)(fac / fsc);
       z.tw = twiddles<T>(c);
       az[r] = z;
       AxisArgs<T> yf{};

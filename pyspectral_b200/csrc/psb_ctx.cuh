@@ -346,6 +346,13 @@ inline bool plan_is_wide_h(const psb::FFTPlan& p) {
   return false;
 }
 
+// Power of two next to fac.  The y-inverse pass multiplies by it on store and the z
+// pass by what is left of fac, so that the fields the register z pass multiplies
+// (it keeps fac until the products' spectra) are within a factor of two of their
+// physical values: products of unnormalised FP32 fields left the range at values
+// 1/fac below those the results can hold.  Powers of two change no bit of a result.
+inline double field_scale(double fac) { return std::ldexp(1.0, (int)std::lround(std::log2(fac))); }
+
 // ---- register passes (psb_reg.cuh; launched by psb_axis_f32.cu / psb_axis_f64.cu) ----
 // The register axis pass's radices of a length; false when it has none.
 inline bool reg_axis_plan(int L, FFTPlan& p) {

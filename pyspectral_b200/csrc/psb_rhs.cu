@@ -107,6 +107,9 @@ int run_ns32(psb_ctx* c, const Cx<T>* Qin, Pre pre, Phys phys, Epi epi, const ps
   b.in_map = map_pad32(N2);
   b.out_map = map_id(M2);
   b.k_row = c->ky;
+  const double s32 = std::sqrt(std::pow(1.5, 3) * std::sqrt((double)N1 * N2 * N3));
+  const double fac = s32 / ((double)M1 * M2 * M3), fsc = field_scale(fac);
+  b.scale = (T)fsc;
   PSB_TRY((launch_axis<T, true, typename YP::type, true>(c, b, typename YP::type{}, "y-inverse", sh[1])));
   // fused z
   ZArgs<T> z{};
@@ -118,8 +121,7 @@ int run_ns32(psb_ctx* c, const Cx<T>* Qin, Pre pre, Phys phys, Epi epi, const ps
   }
   z.out_kz = Kz;
   z.npencils = (long long)M1 * M2;
-  const double s32 = std::sqrt(std::pow(1.5, 3) * std::sqrt((double)N1 * N2 * N3));
-  z.fac = (T)(s32 / ((double)M1 * M2 * M3));
+  z.fac = (T)(fac / fsc);
   z.plan = *plan_for(c, M3);
   z.tw = twiddles<T>(c);
   // two products passes in the registers against one staged pass of both sets
@@ -312,6 +314,8 @@ int run_n23(psb_ctx* c, const Cx<T>* Qin, Pre pre, Phys phys, Epi epi) {
   b.out_rows = N2;
   b.in_map = map_id(N2);
   b.out_map = map_id(N2);
+  const double fac = 1.0 / ((double)N1 * N2 * N3), fsc = field_scale(fac);
+  b.scale = (T)fsc;
   PSB_TRY((launch_axis<T, true>(c, b, PreCopy<T>{}, "mhd y-inverse")));
   ZArgs<T> z{};
   for (int f = 0; f < Fi; ++f) {
@@ -325,7 +329,7 @@ int run_n23(psb_ctx* c, const Cx<T>* Qin, Pre pre, Phys phys, Epi epi) {
   }
   z.out_kz = Kz;
   z.npencils = (long long)N1 * N2;
-  z.fac = (T)(1.0 / ((double)N1 * N2 * N3));
+  z.fac = (T)(fac / fsc);
   z.plan = *plan_for(c, N3);
   z.tw = twiddles<T>(c);
   PSB_TRY(launch_z<T>(c, z, phys, "mhd z-fused"));
@@ -431,6 +435,9 @@ int run_pl(psb_ctx* c, const Cx<T>* Qin, const psb_params* p, const MemCfg& m, C
   b.out_rows = F2;
   b.in_map = map_pad2x_nyq0(N2);
   b.out_map = map_id(F2);
+  const double s2 = std::sqrt(8.0 * std::sqrt((double)N1 * N2 * N3));
+  const double fac = s2 / ((double)F1 * F2 * F3), fsc = field_scale(fac);
+  b.scale = (T)fsc;
   PSB_TRY((launch_axis<T, true>(c, b, PreCopy<T>{}, "2x y-inverse")));
   ZArgs<T> z{};
   const long long fsB = (long long)F1 * F2 * Kz, fsC = (long long)F1 * F2 * F3h;
@@ -445,8 +452,7 @@ int run_pl(psb_ctx* c, const Cx<T>* Qin, const psb_params* p, const MemCfg& m, C
   }
   z.out_kz = F3h;
   z.npencils = (long long)F1 * F2;
-  const double s2 = std::sqrt(8.0 * std::sqrt((double)N1 * N2 * N3));
-  z.fac = (T)(s2 / ((double)F1 * F2 * F3));
+  z.fac = (T)(fac / fsc);
   z.plan = *plan_for(c, F3);
   z.tw = twiddles<T>(c);
   PSB_TRY(launch_z<T>(c, z, PhysProducts<T>{}, "2x z-products"));
@@ -555,6 +561,10 @@ int run_plql(psb_ctx* c, const MemCfg& m, Cx<T>* B2, Cx<T>* E, Epi epi) {
   b.out_rows = F2;
   b.in_map = map_id(F2);
   b.out_map = map_id(F2);
+  // u in B2 carries the same power of two (run_pl)
+  const double s2 = std::sqrt(8.0 * std::sqrt((double)N1 * N2 * N3));
+  const double fac = s2 / ((double)F1 * F2 * F3), fsc = field_scale(fac);
+  b.scale = (T)fsc;
   PSB_TRY((launch_axis<T, true>(c, b, PreCopy<T>{}, "PLq y-inverse")));
   ZArgs<T> z{};
   const long long fsB = (long long)F1 * F2 * Kz;
@@ -573,8 +583,7 @@ int run_plql(psb_ctx* c, const MemCfg& m, Cx<T>* B2, Cx<T>* E, Epi epi) {
   }
   z.out_kz = KO;
   z.npencils = (long long)F1 * F2;
-  const double s2 = std::sqrt(8.0 * std::sqrt((double)N1 * N2 * N3));
-  z.fac = (T)(s2 / ((double)F1 * F2 * F3));
+  z.fac = (T)(fac / fsc);
   z.plan = *plan_for(c, F3);
   z.tw = twiddles<T>(c);
   PSB_TRY(launch_z<T>(c, z, Phys{}, "PLQL z-products"));
@@ -640,7 +649,7 @@ int run_mhd_tmodel(psb_ctx* c, StepIO<T> io, const psb_params* p) {
                   eta};
   PSB_TRY(run_mhd<T>(c, Qin, plain));
   if (!Qin) return PSB_OK;
-  const double fac = 1.0 / ((double)N1 * N2 * N3);
+  const double fac = 1.0 / ((double)N1 * N2 * N3), fsc = field_scale(fac);
   const double down = (double)N1 * N2 * N3 / ((double)F1 * F2 * F3);
   // stage A: masked (u, B) onto the 2x grid
   AxisArgs<T> a = axis_common<T>(c, F1);
@@ -672,6 +681,7 @@ int run_mhd_tmodel(psb_ctx* c, StepIO<T> io, const psb_params* p) {
   b.out_rows = F2;
   b.in_map = map_pad2x(N2);
   b.out_map = map_id(F2);
+  b.scale = (T)fsc;
   PSB_TRY((launch_axis<T, true>(c, b, PreCopy<T>{}, "mhd-t 2x y-inverse")));
   ZArgs<T> z{};
   const long long fsB = (long long)F1 * F2 * Kz;
@@ -686,7 +696,7 @@ int run_mhd_tmodel(psb_ctx* c, StepIO<T> io, const psb_params* p) {
   }
   z.out_kz = F3h;
   z.npencils = (long long)F1 * F2;
-  z.fac = (T)fac;
+  z.fac = (T)(fac / fsc);
   z.plan = *plan_for(c, F3);
   z.tw = twiddles<T>(c);
   PSB_TRY(launch_z<T>(c, z, PhysMHD<T>{}, "mhd-t 2x z-products"));
@@ -750,6 +760,7 @@ int run_mhd_tmodel(psb_ctx* c, StepIO<T> io, const psb_params* p) {
   b3.out_rows = F2;
   b3.in_map = map_id(F2);
   b3.out_map = map_id(F2);
+  b3.scale = (T)fsc;
   PSB_TRY((launch_axis<T, true>(c, b3, PreCopy<T>{}, "mhd-t QL y-inverse")));
   Cx<T>* C3 = E;
   Cx<T>* D3 = C2;
@@ -768,7 +779,7 @@ int run_mhd_tmodel(psb_ctx* c, StepIO<T> io, const psb_params* p) {
   }
   z3.out_kz = Kz;
   z3.npencils = (long long)F1 * F2;
-  z3.fac = (T)fac;
+  z3.fac = (T)(fac / fsc);
   z3.plan = *plan_for(c, F3);
   z3.tw = twiddles<T>(c);
   PSB_TRY(launch_z<T>(c, z3, PhysMHDLin<T>{}, "mhd-t PLQL z-products"));
@@ -1197,6 +1208,9 @@ int run_fm2_3n(psb_ctx* c, const Cx<T>* PL, const Cx<T>* PLq, Cx<T>* out9) {
   b.out_rows = M2;
   b.in_map = to3n2;
   b.out_map = map_id(M2);
+  const double s3 = std::sqrt(27.0 * std::sqrt((double)N1 * N2 * N3));
+  const double fac = s3 / ((double)M1 * M2 * M3), fsc = field_scale(fac);
+  b.scale = (T)fsc;
   PSB_TRY((launch_axis<T, true>(c, b, PreCopy<T>{}, "3n y-inverse")));
   ZArgs<T> z{};
   const long long fsB = (long long)M1 * M2 * Kz, fsO = (long long)M1 * M2 * Ko;
@@ -1211,8 +1225,7 @@ int run_fm2_3n(psb_ctx* c, const Cx<T>* PL, const Cx<T>* PLq, Cx<T>* out9) {
   }
   z.out_kz = Ko;
   z.npencils = (long long)M1 * M2;
-  const double s3 = std::sqrt(27.0 * std::sqrt((double)N1 * N2 * N3));
-  z.fac = (T)(s3 / ((double)M1 * M2 * M3));
+  z.fac = (T)(fac / fsc);
   z.plan = *plan_for(c, M3);
   z.tw = twiddles<T>(c);
   PSB_TRY(launch_z<T>(c, z, PhysPLQL<T>{}, "3n z-products"));

@@ -143,10 +143,11 @@ __device__ __forceinline__ Cx<T> had_add(Cx<T> a, Cx<T> b, Cx<T> c) { return mk<
 template <typename T>
 __device__ __forceinline__ Cx<T> had_sub(Cx<T> a, Cx<T> b, Cx<T> c) { return mk<T>(c.x - a.x * b.x, c.y - a.y * b.y); }
 
-// Mid<Phys>: the middle stage of a physics functor.  The physical fields are
-// unnormalised (1/fac times the physics' arguments): every result is quadratic
-// in them (|S| S_ij included), so fac^2 is applied with the forward transform's
-// own factor when the results are stored.
+// Mid<Phys>: the middle stage of a physics functor.  The physical fields are 1/fac
+// times the physics' arguments: every result is quadratic in them (|S| S_ij
+// included), so fac^2 is applied with the forward transform's own factor when the
+// results are stored.  fac is between 0.7 and 1.5, the power of two next to the whole
+// normalisation being in the stored fields already (field_scale).
 //   SLOTS        slots of the buffer
 //   HEAVY        how many more than four fields' points a thread holds (0, 1, 2)
 //   DERIV        1: some inputs are z derivatives (ZArgs::dz), 2: or means (ZArgs::in2)
