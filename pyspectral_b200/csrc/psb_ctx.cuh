@@ -415,18 +415,23 @@ struct z_registered<psb::PhysLearned<T, psb::kActGelu, HID>> {
 template <typename T, class Phys>
 inline bool has_reg_z(int M) {
   if constexpr (z_registered<Phys>::value) {
-    switch (M) {
 #define PSB_CASE(H, A, B) \
   case 2 * H:             \
     return z_plan_of<Phys>(H);
-      PSB_REG_Z_F64(PSB_CASE)
-      case 432:
-      case 512:
-        return sizeof(T) == 4 && z_plan_of<Phys>(M / 2);
-      default:
-        return false;
-#undef PSB_CASE
+    if constexpr (sizeof(T) == 4) {
+      switch (M) {
+        PSB_REG_Z_F32(PSB_CASE)
+        default:
+          return false;
+      }
+    } else {
+      switch (M) {
+        PSB_REG_Z_F64(PSB_CASE)
+        default:
+          return false;
+      }
     }
+#undef PSB_CASE
   }
   return false;
 }

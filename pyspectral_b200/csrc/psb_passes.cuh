@@ -23,7 +23,8 @@
 //
 // These staged forms take any length of factors 2 and 3.  The lengths in use
 // have register forms (psb_reg.cuh, psb_zreg.cuh, psb_xreg.cuh), which run in
-// their place; the rest, and the persistent ensemble, run here.
+// their place; the rest, the x pass of small launches (x_pass_in_registers),
+// shapes given by hand or kept by the tuner, and the persistent ensemble run here.
 //
 // The padding maps reproduce PySpectral/src/padding.py:2-49 (pad/unpad drop
 // index N/2 of x and y and the k3=N/2 plane; pad_2x/unpad_2x keep the -N/2
@@ -746,20 +747,11 @@ __device__ __forceinline__ void zpass_tile(const ZArgs<T>& a, const Phys& phys, 
   }
 }
 
-// One CTA, one tile (the batched kernel's unit).
-template <typename T, class Phys, bool WIDE = false>
-__device__ __forceinline__ void zpass_body(const ZArgs<T>& a, const Phys& phys, int bx) {
-  pdl_trigger();
-  zpass_setup<T, Phys>(a, phys);
-  pdl_wait();
-  zpass_tile<T, Phys, WIDE>(a, phys, bx);
-}
-
 // CTAs per SM the registers are bounded for.  FP64: two, as the tile's share of
 // the shared memory leaves room for (128 registers; the transforms need about
 // 122).  With 140 registers and one CTA per SM the DNS pass of 64 x 64 x 288
-// (432 points) takes 529 us against 332, and psb_fft_c2r of 128^3 258 against
-// 209.  The radices of the wide form and the network's tiles need more.
+// (432 points) takes 529 us against 332, and psb_fft_c2r of three 128^3 fields
+// 258 against 173.  The radices of the wide form and the network's tiles need more.
 template <typename T, class Phys, bool WIDE>
 constexpr int zpass_minb() {
   return sizeof(T) == 4 ? 3 : (WIDE || phys_is_block<Phys>::value ? 1 : 2);

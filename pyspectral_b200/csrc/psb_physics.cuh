@@ -139,8 +139,9 @@ struct PreCopyN {
 template <typename T>
 struct PreYStrain {
   static constexpr int F_SRC = 6, F_DST = 8, GROUPS = 1, IN_FIELDS = 1, OUT_FIELDS = 1;
-  // the staged pass takes one field a CTA: with the eight in one tile its rows are
-  // one column wide (64 x 384 x 64 FP32, 576 points: PSB_MEASURE_Y)
+  // the staged pass takes one field a CTA; with the eight in one tile its rows were one
+  // column wide (324 x 324 x 64, 486 points: FP64 2.24 ms against 3.17, FP32 1.28
+  // against 1.41; 768 points FP64, 48 x 512 x 48, is the exception, 637 us against 549)
   static constexpr bool SPLIT = true;
   // stored fields u, v, w, i k1 u, i k1 v, i k1 w; field g from sa(g) (and sb(g))
   __host__ __device__ static constexpr int sa(int g) {

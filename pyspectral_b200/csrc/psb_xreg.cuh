@@ -16,10 +16,10 @@
 // the products, so more CTAs run per SM.  R is small because NACC R accumulators
 // live through the whole loop: with R = 8 an FP64 thread of the t-model needs 228
 // registers, two CTAs per SM.  Measured per launch on a B200, before -> after:
-//   t-model 128^3 FP64, PLQL   373 -> 150 us     DNS 256^3 FP32   1063 -> 560
-//   Smagorinsky 64^3 FP64 1.0-1.6 -> 2.0 TB/s    DNS 32^3 FP64    10.5 -> 12.8
-// (the smallest grid pays for its six fields in series; the pass it replaces
-// staged them at once).
+//   t-model 128^3 FP64   PLQL 373 -> 127 us, PL (256 points) 547 -> 490
+//   DNS 256^3 FP32 (384 points)  1063 -> 482     Smagorinsky 128^3 FP64  267 -> 152
+// Launches that leave the SMs few warps pay for the series of fields and run the
+// staged pass (x_pass_in_registers): DNS 32^3 FP64 10.5 us.
 #pragma once
 #include "psb_physics.cuh"
 
