@@ -19,14 +19,14 @@ inline int x_extra_blocks(int n1, int n2, int ncz, int nt) {
 template <typename T, class Epi, int A, int B, int R>
 constexpr int x_group_wave() {
   if (sizeof(T) == 8 || Epi::NACC == 0 || 3 * psb::xreg_threads<T, A, B>() > 1024) return 0;
-  return 148 * (psb::xreg_minb<T, Epi, A, B, R>() / 3);
+  return 148 * (psb::xreg_minb<T, Epi, A, B, R, true>() / 3);
 }
 
-template <typename T, class Epi, int A, int B, int R, int S>
+template <typename T, class Epi, int A, int B, int R, int S, bool MANY>
 int launch_reg_xs(psb_ctx* c, const psb::XEpiArgs<T>& e, const Epi& epi, const char* what, double bytes) {
   const int extra = x_extra_blocks(e.n1, e.n2, e.n3h - e.kz, S * psb::xreg_threads<T, A, B>());
   constexpr size_t smem = psb::xreg_smem<T, Epi, A, B, R, S>();
-  auto k = psb::xreg_kernel<T, Epi, A, B, R, S>;
+  auto k = psb::xreg_kernel<T, Epi, A, B, R, S, MANY>;
   set_smem(k, smem);
   LaunchScope scope(c, what, bytes);
   launch_pdl(k, dim3((unsigned)(e.main_blocks + extra)), S * psb::xreg_threads<T, A, B>(), smem, c->stream, e, epi);
@@ -38,8 +38,11 @@ int launch_reg_x(psb_ctx* c, psb::XEpiArgs<T> e, const Epi& epi, const char* wha
   constexpr int C = psb::xreg_cols<T>();
   e.main_blocks = (e.kz + C - 1) / C * e.n2;
   if constexpr (x_group_wave<T, Epi, A, B, R>() > 0)
-    if (e.main_blocks <= x_group_wave<T, Epi, A, B, R>()) return launch_reg_xs<T, Epi, A, B, R, 3>(c, e, epi, what, bytes);
-  return launch_reg_xs<T, Epi, A, B, R, 1>(c, e, epi, what, bytes);
+    if (e.main_blocks <= x_group_wave<T, Epi, A, B, R>()) return launch_reg_xs<T, Epi, A, B, R, 3, true>(c, e, epi, what, bytes);
+  constexpr int few = psb::xreg_minb<T, Epi, A, B, R, false>();
+  if constexpr (few != psb::xreg_minb<T, Epi, A, B, R, true>())
+    if (e.main_blocks <= 148 * few) return launch_reg_xs<T, Epi, A, B, R, 1, false>(c, e, epi, what, bytes);
+  return launch_reg_xs<T, Epi, A, B, R, 1, true>(c, e, epi, what, bytes);
 }
 
 template <typename T, class Epi, int A, int B, int R>

@@ -233,16 +233,17 @@ __device__ __forceinline__ void xreg_body(const XEpiArgs<T>& a, const Epi& epi, 
 // points 111 -> 86 (144^3), 108 points 23 -> 17 (72^3); Smagorinsky 144 points
 // 76 -> 47 (96^3), 192 points 138 -> 107 (128^3).  With six sums the epilogues
 // spill instead, as do blocks of six warps in threes (18 warps are five on a
-// scheduler, 96 registers): two there in single runs, whose 64^3 grids have no more
-// blocks (DNS 64^3 FP32 38.4 -> 36.2 us a right-hand side), three in batches.
-template <typename T, class Epi, int A, int B, int R, bool BATCH = false>
+// scheduler, 96 registers): two there in launches of no more blocks (MANY false; DNS
+// 64^3 FP32 38.4 -> 36.2 us a right-hand side), three in larger ones (64 x 288 x 64
+// 147 -> 136) and in batches.
+template <typename T, class Epi, int A, int B, int R, bool MANY>
 constexpr int xreg_minb() {
   constexpr int nt = xreg_threads<T, A, B>();
   constexpr int regs = sizeof(T) == 8 ? (Epi::NACC > 3 ? 168 : 128) : (Epi::NACC > 3 ? 128 : 104);
   constexpr int b = 65536 / (regs * nt), left = 65536 / ((b + 1) * nt);
   constexpr bool more = sizeof(T) == 8 ? Epi::NACC == 4 && b == 1 && left >= 128
                                        : Epi::NACC <= 4 && ((b == 1 && left >= 72) || (b == 2 && nt >= 224 && left >= 96));
-  if (!BATCH && sizeof(T) == 4 && nt == 192 && b == 3) return 2;
+  if (!MANY && sizeof(T) == 4 && nt == 192 && b == 3) return 2;
   return more ? (b < 16 ? b + 1 : 16) : (b < 1 ? 1 : (b > 16 ? 16 : b));
 }
 
@@ -255,9 +256,9 @@ constexpr size_t xreg_smem() {
 }
 
 // grid = main_blocks + extra (main block b: column tile b % ntile, outer b / ntile)
-template <typename T, class Epi, int A, int B, int R, int S>
-__global__ void __launch_bounds__(S* xreg_threads<T, A, B>(), xreg_minb<T, Epi, A, B, R>() / S > 0
-                                                                   ? xreg_minb<T, Epi, A, B, R>() / S
+template <typename T, class Epi, int A, int B, int R, int S, bool MANY>
+__global__ void __launch_bounds__(S* xreg_threads<T, A, B>(), xreg_minb<T, Epi, A, B, R, MANY>() / S > 0
+                                                                   ? xreg_minb<T, Epi, A, B, R, MANY>() / S
                                                                    : 1)
     xreg_kernel(const __grid_constant__ XEpiArgs<T> a, const __grid_constant__ Epi epi) {
   xreg_body<T, Epi, A, B, R, S>(a, epi, blockIdx.x, gridDim.x);
