@@ -44,7 +44,7 @@ __device__ __forceinline__ void dtau_fold(double (*red)[THREADS], const double* 
 // The three energy sums over the modes below the test filter, part[6][gridDim.x].
 // Bound by the latency of its strided reads (15 of them a mode), so the modes are
 // spread over the chip.  Test filter 21 on 64^3 FP64 (35,301 modes): a right-hand
-// side takes 722 us; with one block of 256 threads for all modes it took 1018.
+// side takes 713 us; with one block of 256 threads for all modes about 300 more.
 template <typename T>
 __global__ void __launch_bounds__(kDtauSumThreads) dtau_sums_kernel(
     const Cx<T>* __restrict__ Q, const Cx<T>* __restrict__ Lu, const Cx<T>* __restrict__ Lf,

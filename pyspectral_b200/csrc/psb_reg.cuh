@@ -17,11 +17,11 @@
 // replaces kept a tile of every field of a column in one CTA (up to 100 KB of
 // shared memory, two CTAs per SM) and made five to seven shared-memory round
 // trips per element.  Measured per launch on a B200, before -> after:
-//   t-model 128^3 FP64, 256 points  x-inverse 167 -> 44 us, y-inverse 318 -> 74,
-//                                   y-forward 439 -> 306
-//   DNS 256^3 FP32, 384 points      x-inverse 529 -> 149, y-inverse 894 -> 207
-//   learned 128^3 FP32, 192 points  y-inverse 177 -> 88
-// FP64 runs at up to 5 TB/s of the measured 6.5; FP32 at 2.3 to 3.6, its accesses
+//   t-model 128^3 FP64, 256 points  x-inverse 167 -> 42 us, y-inverse 318 -> 68,
+//                                   y-forward 439 -> 284
+//   DNS 256^3 FP32, 384 points      x-inverse 529 -> 149, y-inverse 894 -> 208
+//   learned 128^3 FP32, 192 points  y-inverse 177 -> 87
+// FP64 runs at up to 5.7 TB/s of the measured 6.5; FP32 at 2.3 to 4.5, its accesses
 // being 8 bytes a thread.
 #pragma once
 #include "psb_passes.cuh"

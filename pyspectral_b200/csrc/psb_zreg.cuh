@@ -26,12 +26,12 @@
 // grids, HBM beyond L2.  The line stride and the stride of i are chosen at
 // compile time for the fewest bank conflicts of the two access patterns.
 // Measured per launch on a B200, staged form -> this one:
-//   Smagorinsky FP64   64^3 77 -> 50 us, 128^3 650 -> 380
-//   t-model 128^3 FP64 (256 points)   products 1304 -> 370, PLQL 1767 -> 527
-//   MHD t-model 128^3 FP32            815 -> 316 and 1294 -> 489
-//   DNS 256^3 FP32 (384 points)       2320 -> 464
+//   Smagorinsky FP64   64^3 77 -> 50 us, 128^3 650 -> 400
+//   t-model 128^3 FP64 (256 points)   products 1304 -> 371, PLQL 1767 -> 511
+//   MHD t-model 128^3 FP32            815 -> 312 and 1294 -> 493
+//   DNS 256^3 FP32 (384 points)       2320 -> 462
 //   Smagorinsky FP32, 162 points      121 -> 50
-//   learned FP32       64^3 50 -> 48, 128^3 352 -> 308 (the network's MMAs remain)
+//   learned FP32       64^3 50 -> 48, 128^3 352 -> 292 (the network's MMAs remain)
 //
 // Fields sit in `slots` of the buffer (slot, pencil, i, j); Mid<Phys> says
 // which slot an input or output field uses: an output may reuse the slot of an
