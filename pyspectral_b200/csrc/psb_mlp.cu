@@ -50,9 +50,11 @@ __device__ __forceinline__ void bfrag_kn(uint32_t* b, const __nv_bfloat16* W, in
   b[1] = pack_raw(W[(k + 8) * ld + n0 + g], W[(k + 9) * ld + n0 + g]);
 }
 
-// grad[NPARAMS] += dL/dparams over B points; loss_acc += sum of squared errors / (6B)
+// grad[NPARAMS] += dL/dparams over B points; loss_acc += sum of squared errors / (6B).
+// Bounded to two CTAs per SM: left to the compiler the width-64 ReLU form takes 154
+// registers and one CTA (four minibatches of 65,536: 900 us against 712).
 template <int ACT, int H>
-__global__ void __launch_bounds__(256) mlp_train_kernel(const float* __restrict__ P, const float* __restrict__ nrm,
+__global__ void __launch_bounds__(256, 2) mlp_train_kernel(const float* __restrict__ P, const float* __restrict__ nrm,
                                                         const float* __restrict__ X, const float* __restrict__ T,
                                                         const int* __restrict__ idx, int B, float* __restrict__ grad,
                                                         double* __restrict__ loss_acc) {
